@@ -1,0 +1,228 @@
+// Pair products on the symmetry-folded spectrum.
+//
+// The image set of a mode (x, y, z) is {x, L-x} x {y, L-y} x {z, L-z} (and
+// the same shifted by multiples of L at a larger bandwidth), so a
+// window that is even in every component and symmetric in x and y (every
+// isotropic window, and the cylindrical ones with the line of sight on z)
+// has the same FFT kernel on the up to eight columns (+-x, +-y), (+-y, +-x).
+// pp_fold_kernel adds the pair products T = w_z Re(F_i conj F_j) of those
+// columns into one, for x >= y in [0, L/2]: the passes over bins then walk
+// (L/2+1)(L/2+2)/2 columns instead of L^2.
+//
+// An isotropic window is a function of n2 = |k L|^2 alone, so at bandwidth 1
+// its pair product is a sum over n2:
+//   sum_k T(k) K_b(k) = sum_n2 W_b(n2) Hist(n2),
+//   Hist(n2) = sum over modes and images with |image|^2 = n2 of P P P T.
+// Hist does not depend on the bin: pp_hist_kernel builds it once (8 adds per
+// folded mode, which is what bounds it: scattered 64-bit atomics on an array
+// that stays in L2) and pp_radial_bins_kernel evaluates each bin's window
+// once per n2, 3 L^2 + 1 values, instead of 8 times per mode.  The histogram
+// is in 64-bit fixed point (exponent from the largest |T|), so its sums are
+// exact and do not depend on the order of the atomics.
+#pragma once
+
+#include "pair_products.cuh"
+
+namespace hermes {
+
+constexpr int kHistThreads = 256;
+constexpr int kHistBits = 42;       // max |T| < 2^42 quanta: 2^20 additions cannot overflow
+constexpr int kRadialPerBlock = 4096;
+constexpr int kRadialBins = 4;      // bins per block of pp_radial_bins_kernel
+
+__host__ __device__ __forceinline__ long long fold_columns(int L) {
+  const long long H = L / 2 + 1;
+  return H * (H + 1) / 2;
+}
+
+// (x, y), x >= y, of folded column c = x (x + 1) / 2 + y.
+__device__ __forceinline__ void fold_xy(int c, int& x, int& y) {
+  x = (int)((sqrtf(8.f * (float)c + 1.f) - 1.f) * 0.5f);
+  while (x * (x + 1) / 2 > c) --x;
+  while ((x + 1) * (x + 2) / 2 <= c) ++x;
+  y = c - x * (x + 1) / 2;
+}
+
+// T[p][column][z] of the folded columns, one warp per column; the largest
+// |T| of each pair (as float bits; a NaN has the largest) in maxbits.
+template <int NP>
+__global__ void __launch_bounds__(kHistThreads)
+pp_fold_kernel(PPArgs a, float* __restrict__ T, unsigned* __restrict__ maxbits) {
+  const int L = a.L, H = L / 2 + 1, Lm = L - 1;
+  const int ncol = (int)fold_columns(L);
+  const int lane = threadIdx.x & 31;
+  const int nw = gridDim.x * (kHistThreads / 32);
+  unsigned mx[NP];
+#pragma unroll
+  for (int p = 0; p < NP; ++p) mx[p] = 0u;
+  for (int c = blockIdx.x * (kHistThreads / 32) + (threadIdx.x >> 5); c < ncol; c += nw) {
+    int x, y;
+    fold_xy(c, x, y);
+    const bool rx = x != 0 && 2 * x != L, ry = y != 0 && 2 * y != L, sw = x != y;
+    // rows (x, y), (-x, y), (x, -y), (-x, -y), then the same with x and y exchanged
+    const int xs[2] = {x, (L - x) & Lm}, ys[2] = {y, (L - y) & Lm};
+    for (int z = lane; z < H; z += 32) {
+      float t[NP];
+#pragma unroll
+      for (int p = 0; p < NP; ++p) t[p] = 0.f;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const int i = r & 1, j = (r >> 1) & 1, s = r >> 2;
+        if ((i && !rx) || (j && !ry) || (s && !sw)) continue;
+        const long long row = s ? (long long)ys[j] * L + xs[i] : (long long)xs[i] * L + ys[j];
+        const long long m = row * H + z;
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          const float2 u = a.si[p][m];
+          const float2 v = a.sj[p] == a.si[p] ? u : a.sj[p][m];
+          t[p] += u.x * v.x + u.y * v.y;
+        }
+      }
+      const float wgt = (z == 0 || 2 * z == L) ? 1.f : 2.f;
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const float v = (a.exclude_k0 && c == 0 && z == 0) ? 0.f : wgt * t[p];
+        T[((size_t)p * ncol + c) * H + z] = v;
+        mx[p] = max(mx[p], __float_as_uint(fabsf(v)));
+      }
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    const unsigned m = __reduce_max_sync(0xffffffffu, mx[p]);
+    if (lane == 0 && m) atomicMax(&maxbits[p], m);
+  }
+}
+
+// Exponent shift of the fixed point: quanta = v * 2^shift, |v| <= the largest |T|.
+__device__ __forceinline__ int hist_shift(unsigned maxbits) { return kHistBits + 126 - (int)(maxbits >> 23); }
+
+// v * 2^shift rounded to the nearest integer (ties away from zero), with
+// integer operations only; |v| 2^shift < 2^62.
+__device__ __forceinline__ long long f32_shifted_ll(float v, int shift) {
+  const int b = __float_as_int(v);
+  const int e = (b >> 23) & 0xFF;
+  if (e == 0) return 0;  // zero or subnormal
+  const long long m = (long long)((b & 0x7FFFFF) | 0x800000);
+  const int up = e + shift - 150;
+  long long q;
+  if (up >= 0) {
+    q = m << up;
+  } else {
+    q = up <= -25 ? 0 : ((m + (1LL << (-up - 1))) >> -up);
+  }
+  return b < 0 ? -q : q;
+}
+
+// hist[p][n2] += P(a) P(b) P(c) T[p][column][z] over the images (a, b, c) of
+// every folded mode; one warp per column, lanes along z.
+template <int NP>
+__global__ void __launch_bounds__(kHistThreads)
+pp_hist_kernel(const float* __restrict__ T, int L, const double* __restrict__ pd, const unsigned* __restrict__ maxbits,
+               unsigned long long* __restrict__ hist, int nh) {
+  extern __shared__ float P[];
+  for (int i = threadIdx.x; i <= L; i += kHistThreads) P[i] = (float)pd[i];
+  __syncthreads();
+  const int H = L / 2 + 1, ncol = (int)fold_columns(L);
+  const int lane = threadIdx.x & 31;
+  const int nw = gridDim.x * (kHistThreads / 32);
+  int shift[NP];
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    const unsigned mb = maxbits[p];
+    if (mb >= 0x7F800000u) return;  // not finite: the bins report NaN
+    shift[p] = hist_shift(mb);
+  }
+  for (int c = blockIdx.x * (kHistThreads / 32) + (threadIdx.x >> 5); c < ncol; c += nw) {
+    int x, y;
+    fold_xy(c, x, y);
+    float w[4];
+    int s[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int pa = (i & 1) ? L - x : x, pb = (i & 2) ? L - y : y;
+      w[i] = P[pa] * P[pb];
+      s[i] = pa * pa + pb * pb;
+    }
+    for (int z = lane; z < H; z += 32) {
+      const int z2 = z * z, m2 = (L - z) * (L - z);
+      const float p1 = P[z], p2 = P[L - z];
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const float t = T[((size_t)p * ncol + c) * H + z];
+        unsigned long long* h = hist + (size_t)p * nh;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const long long q1 = f32_shifted_ll(w[i] * p1 * t, shift[p]), q2 = f32_shifted_ll(w[i] * p2 * t, shift[p]);
+          if (q1) atomicAdd(h + s[i] + z2, (unsigned long long)q1);
+          if (q2) atomicAdd(h + s[i] + m2, (unsigned long long)q2);
+        }
+      }
+    }
+  }
+}
+
+// partial[block][bin][pair] = sum over the block's n2 of W_bin(n2) hist(n2)
+// (window values in float32, products and sums in float64).
+template <int NP>
+__global__ void __launch_bounds__(kHistThreads)
+pp_radial_bins_kernel(const WinDev* __restrict__ wins, int n_bins, int L, const double* __restrict__ pd,
+                      const unsigned* __restrict__ maxbits, const unsigned long long* __restrict__ hist, int nh,
+                      double* __restrict__ partial, double* __restrict__ k0) {
+  extern __shared__ float P[];
+  __shared__ double red[kHistThreads / 32][kRadialBins * NP];
+  const int b0 = blockIdx.y * kRadialBins, nb = min(kRadialBins, n_bins - b0);
+  if (blockIdx.x == 0) {
+    for (int i = threadIdx.x; i <= L; i += kHistThreads) P[i] = (float)pd[i];
+    __syncthreads();
+    if (threadIdx.x < nb)
+      k0[b0 + threadIdx.x] = (double)kernel_value(wins[b0 + threadIdx.x], 0, 0, 0, L, P, 1).x;
+  }
+  double acc[kRadialBins][NP];
+#pragma unroll
+  for (int b = 0; b < kRadialBins; ++b)
+#pragma unroll
+    for (int p = 0; p < NP; ++p) acc[b][p] = 0.0;
+  const int end = min(nh, (int)(blockIdx.x + 1) * kRadialPerBlock);
+  for (int n2 = blockIdx.x * kRadialPerBlock + threadIdx.x; n2 < end; n2 += kHistThreads) {
+    double h[NP];
+    bool any = false;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const long long q = (long long)hist[(size_t)p * nh + n2];
+      any = any || q != 0;
+      h[p] = (double)q;
+    }
+    if (!any) continue;
+#pragma unroll
+    for (int b = 0; b < kRadialBins; ++b) {
+      if (b < nb) {
+        bool ok;
+        const double w = (double)window_iso_n2(wins[b0 + b], n2, &ok).x;
+#pragma unroll
+        for (int p = 0; p < NP; ++p) acc[b][p] = fma(w, h[p], acc[b][p]);
+      }
+    }
+  }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int b = 0; b < kRadialBins; ++b)
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      double v = acc[b][p];
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) red[wid][b * NP + p] = v;
+    }
+  __syncthreads();
+  if (threadIdx.x < nb * NP) {
+    const int b = threadIdx.x / NP, p = threadIdx.x % NP;
+    double s = 0.0;
+    for (int w = 0; w < kHistThreads / 32; ++w) s += red[w][b * NP + p];
+    const unsigned mb = maxbits[p];
+    s = mb >= 0x7F800000u ? __longlong_as_double(0x7ff8000000000000LL)
+                          : ldexp(s * (double)wins[b0 + b].scale, -hist_shift(mb));
+    partial[((long long)blockIdx.x * n_bins + b0 + b) * NP + p] = s;
+  }
+}
+
+}  // namespace hermes

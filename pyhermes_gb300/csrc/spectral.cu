@@ -10,6 +10,7 @@
 // the half spectra:  sum_x (f1 * K)(x) f2(x) / L^3 = sum_k F1 K conj(F2) / L^6.
 #include <cufft.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -17,6 +18,7 @@
 
 #include "hermes_common.cuh"
 #include "window_eval.cuh"
+#include "pair_fold.cuh"
 #include "pair_products.cuh"
 
 namespace hermes {
@@ -374,22 +376,18 @@ extern "C" int hermes_spectrum_multiply(void* spec, const float* k_real, const v
 //   A = sum over the (x, y) images of P P f(k_perp R),  B = sum over the z
 //   images of P g(k_par H)   (cyl_image_sum).
 // So sum_k T(k) K_b(k) = sum_(x,y) A_b(x, y) * [sum_z T(x, y, z) B_b(z)]: per
-// column a [columns x z] by [z x bins] product, then a weighted sum.
-//
-// A depends on (x, y) only through the image set {x, L-x} x {y, L-y} and
-// p^2 + q^2, so A(x, y) = A(min(x, L-x), min(y, L-y)) = A(y, x).
-// cyl_perp_table_kernel evaluates it once per (x, y) in the triangle
-// 0 <= y <= x <= L/2 and bin (1/8 of the plane), into a table that the
-// column kernel reads.
+// column a [columns x z] by [z x bins] product, then a weighted sum.  A
+// depends on (x, y) only through the image set {x, L-x} x {y, L-y} and
+// p^2 + q^2 (at any bandwidth), so the columns are the folded ones of
+// pp_fold_kernel (1/8 of the plane); cyl_perp_table_kernel evaluates A once
+// per folded column and bin.
 //
 // Column kernel: a block takes kCylBins bins (two per lane); B is tabulated
 // for them in shared memory as [z][bin].  A warp takes CW consecutive
-// columns (their modes are contiguous), stages the weighted products
-// T = w_z Re(u conj v) in chunks of kCylZ z-planes as [z][pair][column], and
-// per z reads CW columns' T (broadcast, 128-bit) and its two bins' B (64-bit)
-// for 2 x CW FMAs per pair: a register tile instead of one shared-memory load
-// per FMA.  The spectra are read once per bin group; the groups run side by
-// side, so the second and later reads mostly hit L2.
+// columns (contiguous in the folded T), stages them in chunks of kCylZ
+// z-planes as [z][pair][column], and per z reads CW columns' T (broadcast,
+// 128-bit) and its two bins' B (64-bit) for 2 x CW FMAs per pair: a register
+// tile instead of one shared-memory load per FMA.
 constexpr int kCylBins = 64;
 constexpr int kCylZ = 64;
 
@@ -398,41 +396,36 @@ struct CylCols {
   static constexpr int value = NP == 1 ? 8 : 4;  // columns per warp task
 };
 
+// A of every folded column and bin: atab[column][nbp].
 __global__ void cyl_perp_table_kernel(const WinDev* __restrict__ wins, int n_bins, int nbp,
                                       const double* __restrict__ pd, int np, int L, int bw,
                                       float* __restrict__ atab) {
   extern __shared__ float Pt[];
   for (int i = threadIdx.x; i < np; i += blockDim.x) Pt[i] = (float)pd[i];
   __syncthreads();
-  const int H = L / 2 + 1;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)H * H * nbp) return;
+  if (i >= fold_columns(L) * nbp) return;
   const int b = (int)(i % nbp);
-  const long long cell = i / nbp;
-  const int x = (int)(cell / H), y = (int)(cell - (long long)x * H);
-  if (y > x) return;
+  int x, y;
+  fold_xy((int)(i / nbp), x, y);
   float av = 0.f;
   if (b < n_bins) {
     const WinDev& w = wins[b];
-    const int sgn = w.mode == HERMES_KMODE_OCTANT ? 1 : -1;
     const int n_img = 4 * bw * bw;
     for (int t = 0; t < n_img; ++t) {
-      const int pair = t >> 2, sp = t & 1, sq = (t >> 1) & 1;
-      const int ii = pair / bw, jj = pair - ii * bw;
-      const int pu = sp ? ii * L + (L - x) : ii * L + x;
-      const int qu = sq ? jj * L + (L - y) : jj * L + y;
-      av = fmaf(Pt[pu] * Pt[qu], cyl_perp(w, sp ? sgn * pu : pu, sq ? sgn * qu : qu), av);
+      const int pair = t >> 2, ii = pair / bw, jj = pair - ii * bw;
+      const int pu = ii * L + ((t & 1) ? L - x : x), qu = jj * L + ((t & 2) ? L - y : y);
+      av = fmaf(Pt[pu] * Pt[qu], cyl_perp(w, pu, qu), av);
     }
   }
-  atab[((size_t)x * H + y) * nbp + b] = av;
-  atab[((size_t)y * H + x) * nbp + b] = av;
+  atab[i] = av;
 }
 
 template <int NP>
 __global__ void __launch_bounds__(kPPThreads, 2)
-pair_products_cylz_kernel(PPArgs a, const WinDev* __restrict__ wins, const double* __restrict__ pd,
-                          const float* __restrict__ atab, int nbp, double* __restrict__ partial,
-                          double* __restrict__ k0) {
+pair_products_cylz_kernel(PPArgs a, const float* __restrict__ fold, const WinDev* __restrict__ wins,
+                          const double* __restrict__ pd, const float* __restrict__ atab, int nbp,
+                          double* __restrict__ partial, double* __restrict__ k0) {
   constexpr int kWarps = kPPThreads / 32;
   constexpr int CW = CylCols<NP>::value;
   constexpr int TZ = CW * NP;  // floats per z-plane of a warp's staged chunk
@@ -474,7 +467,7 @@ pair_products_cylz_kernel(PPArgs a, const WinDev* __restrict__ wins, const doubl
 #pragma unroll
     for (int p = 0; p < NP; ++p) acc[j][p] = 0.0;
   }
-  const long long ncol = (long long)L * L;  // a multiple of CW
+  const long long ncol = fold_columns(L);
   for (long long col0 = ((long long)blockIdx.x * kWarps + wid) * CW; col0 < ncol;
        col0 += (long long)gridDim.x * kWarps * CW) {
     // (bin 2 lane, bin 2 lane + 1) sums of each column, updated by paired FMAs
@@ -488,24 +481,18 @@ pair_products_cylz_kernel(PPArgs a, const WinDev* __restrict__ wins, const doubl
       const int zn = min(kCylZ, H - zc);
       __syncwarp();
       // lane i stages z-plane zc + i of all CW columns: per column the lanes
-      // read consecutive modes (coalesced), the CW loads are in flight
-      // together, and the plane's products are written as 128-bit rows
+      // read consecutive values (coalesced), the CW loads are in flight
+      // together, and the plane's values are written as 128-bit rows
 #pragma unroll
       for (int ii = 0; ii < kCylZ / 32; ++ii) {
         const int i = lane + 32 * ii;
         if (i < zn) {
-          const int z = zc + i;
-          const float wgt = (z == 0 || z == L / 2) ? 1.f : 2.f;
           float tv[NP][CW];
 #pragma unroll
-          for (int c = 0; c < CW; ++c) {
-            const long long m = (col0 + c) * H + z;
+          for (int c = 0; c < CW; ++c)
 #pragma unroll
-            for (int p = 0; p < NP; ++p) {
-              const float2 u = a.si[p][m], v = a.sj[p][m];
-              tv[p][c] = (a.exclude_k0 && m == 0) ? 0.f : wgt * (u.x * v.x + u.y * v.y);
-            }
-          }
+            for (int p = 0; p < NP; ++p)
+              tv[p][c] = col0 + c < ncol ? fold[(p * ncol + col0 + c) * H + zc + i] : 0.f;
 #pragma unroll
           for (int p = 0; p < NP; ++p)
 #pragma unroll
@@ -549,9 +536,8 @@ pair_products_cylz_kernel(PPArgs a, const WinDev* __restrict__ wins, const doubl
 #pragma unroll
     for (int c = 0; c < CW; ++c) {
       const long long col = col0 + c;
-      const int x = (int)(col / L), y = (int)(col - (long long)x * L);
-      const int xq = min(x, L - x), yq = min(y, L - y);
-      const float2 av = *reinterpret_cast<const float2*>(atab + ((size_t)xq * H + yq) * nbp + b0 + 2 * lane);
+      if (col >= ncol) break;
+      const float2 av = *reinterpret_cast<const float2*>(atab + (size_t)col * nbp + b0 + 2 * lane);
       const float aj[2] = {av.x, av.y};
 #pragma unroll
       for (int j = 0; j < 2; ++j)
@@ -592,6 +578,17 @@ static size_t cylz_smem(int np, int L, int n_pairs) {
 // Bins padded to whole groups of kCylBins (the A table's row stride).
 static int cylz_nbp(int n_bins) { return (n_bins + kCylBins - 1) / kCylBins * kCylBins; }
 
+// True when every bin is an isotropic window (a function of |k|^2 alone)
+// whose kernel keeps its k = 0 value, or the k = 0 mode is left out.
+static bool all_radial(const std::vector<WinDev>& hw, bool exclude_k0) {
+  for (const WinDev& w : hw) {
+    const bool iso = w.type == HERMES_WIN_SPHERE || w.type == HERMES_WIN_GAUSSIAN || w.type == HERMES_WIN_SHELL ||
+                     w.type == HERMES_WIN_THICK_SHELL || w.type == HERMES_WIN_GAUSSIAN_SHELL;
+    if (!iso || (w.zero_k0 && !exclude_k0)) return false;
+  }
+  return !hw.empty();
+}
+
 // True when every bin is a cylindrical window with the line of sight on z
 // and all bins use the same image mode (the column kernel's precondition).
 static bool all_cyl_z(const std::vector<WinDev>& hw) {
@@ -610,19 +607,101 @@ static long long pp_mode_blocks(int J) {
   return (total + per - 1) / per;
 }
 
+namespace {
+struct PPWs {
+  WinDev* wins;
+  double* partial;           // [blocks][n_bins][n_pairs]
+  double* dout;              // [n_bins][n_pairs]
+  double* k0;                // [n_bins]
+  float* fold;               // [n_pairs][folded columns][H]
+  unsigned* maxbits;         // [n_pairs]
+  union {                    // one of the two folded passes runs
+    float* atab;             // A table of cylindrical bins [folded columns][nbp]
+    unsigned long long* hist;  // histogram over n2 [n_pairs][3 L^2 + 1]
+  };
+  size_t used;
+};
+
+// The one workspace layout of hermes_pair_products.
+PPWs pp_carve(void* ws, size_t cap, int J, int n_bins, int n_pairs) {
+  const int L = 1 << J;
+  const size_t ncol = (size_t)fold_columns(L), H = (size_t)L / 2 + 1;
+  Carver c(ws, cap);
+  PPWs w;
+  w.wins = c.take<WinDev>(n_bins);
+  w.partial = c.take<double>((size_t)pp_mode_blocks(J) * n_bins * n_pairs);
+  w.dout = c.take<double>((size_t)n_bins * n_pairs);
+  w.k0 = c.take<double>((size_t)n_bins);
+  w.maxbits = c.take<unsigned>((size_t)n_pairs);
+  w.fold = c.take<float>(n_pairs * ncol * H);
+  const size_t shared = std::max(ncol * (size_t)cylz_nbp(n_bins) * sizeof(float),
+                                 n_pairs * (3 * (size_t)L * L + 1) * sizeof(unsigned long long));
+  w.hist = reinterpret_cast<unsigned long long*>(c.take<char>(shared));
+  w.used = c.used;
+  return w;
+}
+
+// Folded passes of NP pairs: the fold, then the cylindrical columns or the
+// histogram over n2; writes partial sums and returns their block count.
+template <int NP>
+int pp_folded(const PPArgs& a, const PPWs& w, const double* phi_power, bool radial, long long max_blocks, int* nblk,
+              cudaStream_t s) {
+  const int L = a.L, H = L / 2 + 1;
+  int dev = 0, nsm = 148;
+  HERMES_CUDA_TRY(cudaGetDevice(&dev));
+  HERMES_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const long long ncol = fold_columns(L);
+  const int fold_grid = (int)std::min<long long>((ncol + 7) / 8, (long long)nsm * 8);
+  HERMES_CUDA_TRY(cudaMemsetAsync(w.maxbits, 0, sizeof(unsigned) * NP, s));
+  pp_fold_kernel<NP><<<fold_grid, kHistThreads, 0, s>>>(a, w.fold, w.maxbits);
+  HERMES_LAUNCH_CHECK("pp_fold_kernel");
+  if (radial) {
+    const int nh = 3 * L * L + 1;
+    const size_t psm = sizeof(float) * (size_t)(L + 1);
+    HERMES_CUDA_TRY(cudaMemsetAsync(w.hist, 0, sizeof(unsigned long long) * NP * (size_t)nh, s));
+    pp_hist_kernel<NP><<<fold_grid, kHistThreads, psm, s>>>(w.fold, L, phi_power, w.maxbits, w.hist, nh);
+    HERMES_LAUNCH_CHECK("pp_hist_kernel");
+    *nblk = (nh + kRadialPerBlock - 1) / kRadialPerBlock;
+    const dim3 grid((unsigned)*nblk, (unsigned)((a.n_bins + kRadialBins - 1) / kRadialBins));
+    pp_radial_bins_kernel<NP><<<grid, kHistThreads, psm, s>>>(w.wins, a.n_bins, L, phi_power, w.maxbits, w.hist, nh,
+                                                              w.partial, w.k0);
+    HERMES_LAUNCH_CHECK("pp_radial_bins_kernel");
+    return HERMES_OK;
+  }
+  const int nbp = cylz_nbp(a.n_bins);
+  const long long tab_threads = ncol * nbp;
+  cyl_perp_table_kernel<<<(unsigned)((tab_threads + 255) / 256), 256, sizeof(float) * (size_t)a.np, s>>>(
+      w.wins, a.n_bins, nbp, phi_power, a.np, L, a.bw, w.atab);
+  HERMES_LAUNCH_CHECK("cyl_perp_table_kernel");
+  const size_t csm = cylz_smem(a.np, L, NP);
+  HERMES_CUDA_TRY(cudaFuncSetAttribute(pair_products_cylz_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)csm));
+  // every block resident at once over all bin groups (whole waves), so
+  // each block's table of B(z) is reused over many columns and the groups
+  // read the same columns at about the same time
+  int per_sm = 1;
+  HERMES_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pair_products_cylz_kernel<NP>, kPPThreads, csm));
+  if (per_sm < 1) per_sm = 1;
+  const int groups = nbp / kCylBins, per_block = (kPPThreads / 32) * CylCols<NP>::value;
+  long long cblk = (long long)per_sm * nsm / groups;
+  const long long max_tasks = (ncol + per_block - 1) / per_block;
+  if (cblk > max_tasks) cblk = max_tasks;
+  if (cblk > max_blocks) cblk = max_blocks;  // partial sums sized for max_blocks blocks
+  if (cblk < 1) cblk = 1;
+  pair_products_cylz_kernel<NP><<<dim3((unsigned)cblk, (unsigned)groups), kPPThreads, csm, s>>>(
+      a, w.fold, w.wins, phi_power, w.atab, nbp, w.partial, w.k0);
+  HERMES_LAUNCH_CHECK("pair_products_cylz_kernel");
+  *nblk = (int)cblk;
+  return HERMES_OK;
+}
+}  // namespace
+
 extern "C" int hermes_pair_products_workspace_size(int J, int n_bins, int n_pairs, size_t* bytes) {
   if (!bytes) return fail(HERMES_ERR_INVALID, "bytes is NULL");
   if (J < 2 || J > 10) return fail(HERMES_ERR_INVALID, "J=%d outside [2,10]", J);
   if (n_bins < 1 || n_pairs < 1 || n_pairs > kMaxPairs)
     return fail(HERMES_ERR_INVALID, "pair_products: n_bins >= 1 and 1 <= n_pairs <= %d", kMaxPairs);
-  const size_t H = ((size_t)1 << J) / 2 + 1;
-  Carver c(nullptr, 0);
-  c.take<WinDev>(n_bins);
-  c.take<double>((size_t)pp_mode_blocks(J) * n_bins * n_pairs);
-  c.take<double>((size_t)n_bins * n_pairs);
-  c.take<double>((size_t)n_bins);
-  c.take<float>(H * H * (size_t)cylz_nbp(n_bins));  // A table of cylindrical bins
-  *bytes = c.used;
+  *bytes = pp_carve(nullptr, 0, J, n_bins, n_pairs).used;
   return HERMES_OK;
 }
 
@@ -661,52 +740,29 @@ extern "C" int hermes_pair_products(const void* const* spectra, int n_spec, cons
     rc = prepare_window(bins[b], L, &hw[b]);
     if (rc) return rc;
   }
-  Carver c(workspace, workspace_bytes);
-  WinDev* dwin = c.take<WinDev>(n_bins);
+  const PPWs w = pp_carve(workspace, workspace_bytes, J, n_bins, n_pairs);
+  WinDev* dwin = w.wins;
   const long long nblk = pp_mode_blocks(J);
-  double* partial = c.take<double>((size_t)nblk * n_bins * n_pairs);
-  double* dout = c.take<double>((size_t)n_bins * n_pairs);
-  double* dk0 = c.take<double>((size_t)n_bins);
-  const int H = L / 2 + 1;
-  const int nbp = cylz_nbp(n_bins);
-  float* atab = c.take<float>((size_t)H * H * nbp);
+  double *partial = w.partial, *dout = w.dout, *dk0 = w.k0;
   cudaStream_t s = as_stream(stream);
   HERMES_CUDA_TRY(cudaMemcpyAsync(dwin, hw.data(), sizeof(WinDev) * n_bins, cudaMemcpyHostToDevice, s));
-  if (all_cyl_z(hw) && n_pairs <= 4 && cylz_smem(a.np, L, n_pairs) <= 200 * 1024) {
-    const long long tab_threads = (long long)H * H * nbp;
-    cyl_perp_table_kernel<<<(unsigned)((tab_threads + 255) / 256), 256, a.np * sizeof(float), s>>>(
-        dwin, n_bins, nbp, phi_power, a.np, L, bandwidth, atab);
-    HERMES_LAUNCH_CHECK("cyl_perp_table_kernel");
-    const size_t csm = cylz_smem(a.np, L, n_pairs);
-    const void* fn = n_pairs == 1 ? (const void*)pair_products_cylz_kernel<1>
-                   : n_pairs == 2 ? (const void*)pair_products_cylz_kernel<2>
-                   : n_pairs == 3 ? (const void*)pair_products_cylz_kernel<3>
-                                  : (const void*)pair_products_cylz_kernel<4>;
-    HERMES_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
-    // every block resident at once over all bin groups (whole waves), so
-    // each block's table of B(z) is reused over many columns and the groups
-    // read the same columns at about the same time
-    int dev = 0, nsm = 148, per_sm = 1;
-    HERMES_CUDA_TRY(cudaGetDevice(&dev));
-    HERMES_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    HERMES_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kPPThreads, csm));
-    if (per_sm < 1) per_sm = 1;
-    const int groups = nbp / kCylBins;
-    long long cblk = (long long)per_sm * nsm / groups;
-    const long long max_tasks = (long long)L * L / ((kPPThreads / 32) * (n_pairs == 1 ? 8 : 4));
-    if (cblk > max_tasks) cblk = max_tasks;
-    if (cblk > nblk) cblk = nblk;  // partial sums sized for nblk blocks
-    if (cblk < 1) cblk = 1;
-    dim3 cgrid((unsigned)cblk, (unsigned)groups);
+  // The folded passes, at any level and bin count: 30 shells x 2 pairs at
+  // J = 9 take 1.89 ms (fold 1.03, histogram 0.67, bins 0.19), 143.3 ms in
+  // the generic kernel; 20 shells at J = 7 0.06 ms, 1.68 ms there; 300 rings
+  // at J = 9 0.69 ms (fold 0.23, A table 0.28, columns 0.18), 1.74 ms over
+  // the unfolded columns.
+  const bool radial = bandwidth == 1 && all_radial(hw, exclude_k0 != 0);
+  if (radial || (all_cyl_z(hw) && cylz_smem(a.np, L, n_pairs) <= 200 * 1024)) {
+    int fblk = 0;
     switch (n_pairs) {
-      case 1: pair_products_cylz_kernel<1><<<cgrid, kPPThreads, csm, s>>>(a, dwin, phi_power, atab, nbp, partial, dk0); break;
-      case 2: pair_products_cylz_kernel<2><<<cgrid, kPPThreads, csm, s>>>(a, dwin, phi_power, atab, nbp, partial, dk0); break;
-      case 3: pair_products_cylz_kernel<3><<<cgrid, kPPThreads, csm, s>>>(a, dwin, phi_power, atab, nbp, partial, dk0); break;
-      default: pair_products_cylz_kernel<4><<<cgrid, kPPThreads, csm, s>>>(a, dwin, phi_power, atab, nbp, partial, dk0); break;
+      case 1: rc = pp_folded<1>(a, w, phi_power, radial, nblk, &fblk, s); break;
+      case 2: rc = pp_folded<2>(a, w, phi_power, radial, nblk, &fblk, s); break;
+      case 3: rc = pp_folded<3>(a, w, phi_power, radial, nblk, &fblk, s); break;
+      default: rc = pp_folded<4>(a, w, phi_power, radial, nblk, &fblk, s); break;
     }
-    HERMES_LAUNCH_CHECK("pair_products_cylz_kernel");
+    if (rc) return rc;
     const double cscale = 1.0 / ((double)L * L * L * (double)L * L * L);
-    reduce_partials_kernel<<<n_bins * n_pairs, 256, 0, s>>>(partial, (int)cblk, n_bins * n_pairs, cscale, dout);
+    reduce_partials_kernel<<<n_bins * n_pairs, 256, 0, s>>>(partial, fblk, n_bins * n_pairs, cscale, dout);
     HERMES_LAUNCH_CHECK("reduce_partials_kernel");
     HERMES_CUDA_TRY(cudaMemcpyAsync(out, dout, sizeof(double) * n_bins * n_pairs, cudaMemcpyDeviceToHost, s));
     if (k0_out) HERMES_CUDA_TRY(cudaMemcpyAsync(k0_out, dk0, sizeof(double) * n_bins, cudaMemcpyDeviceToHost, s));
