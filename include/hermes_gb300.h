@@ -118,6 +118,16 @@ int hermes_deposit_get_tile(int J, int* tx, int* ty, int* tz);
 int hermes_phi_prepare(const double* phi, int n_phi, int phi_res, int L, int bandwidth,
                        double* power_out, double* gamma_out, void* stream);
 
+/* ---- passes over one field ---------------------------------------------------
+ * dev_out[0] = sum of x[0 .. n) in float64 (the coefficient sum behind the
+ * reference's field_integral and the k = 0 mode, io/sfc_field.py:305-324), in
+ * a fixed order.  workspace: at least 16 KiB of device memory. */
+int hermes_field_sum(const float* x, int64_t n, double* dev_out, void* workspace, size_t workspace_bytes,
+                     void* stream);
+/* out[i] = (float)(x[i] - r): a field minus a mean density
+ * (theory/corr3pcf_multipole.py:944-952); out may be x. */
+int hermes_field_shift(const float* x, int64_t n, double r, float* out, void* stream);
+
 /* ---- spectral windows ------------------------------------------------------
  * Built-in window transfer functions (utils/window_functions.py:441-458),
  * evaluated on the fly inside the passes below instead of being materialised

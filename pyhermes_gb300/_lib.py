@@ -34,6 +34,8 @@ SIGNATURES = {
     "hermes_deposit_get_tile": (_c_int, [_c_int, ctypes.POINTER(_c_int), ctypes.POINTER(_c_int),
                                          ctypes.POINTER(_c_int)]),
     "hermes_deposit_noalloc": (_c_int, [_p, _p, _c_i64, _c_int, _dbl, _p, _c_int, _c_int, _p, _p, _p, _p]),
+    "hermes_field_sum": (_c_int, [_p, _c_i64, _p, _p, _c_sz, _p]),
+    "hermes_field_shift": (_c_int, [_p, _c_i64, _dbl, _p, _p]),
     "hermes_fft_r2c": (_c_int, [_p, _p, _c_int, _p]),
     "hermes_fft_c2r": (_c_int, [_p, _p, _c_int, _p]),
     "hermes_window_workspace_size": (_c_int, [_c_int, ctypes.POINTER(_c_sz)]),

@@ -24,6 +24,7 @@ import time
 import numpy as np
 import torch
 
+from .kernels import field_sum
 from .params import plain_copy, task_params
 from .sfc_field import (ResultFileIO, SFCField, check_fout, describe_input, normalize_task_weight_normalization,
                         read_numpy_pickle, write_numpy_pickle)
@@ -211,8 +212,8 @@ def compute_pair_product_at_sample(sample, sfc_field1, sfc_field2=None, binning_
     specs, pair = ([s1], (0, 0)) if e2 is e1 else ([s1, rfft_field(e2)], (0, 1))
     v, k0 = pair_products(specs, [pair], [window], exclude_k0=True)
     # the k = 0 term in float64
-    dc1 = float(e1.double().sum().item())
-    dc2 = dc1 if e2 is e1 else float(e2.double().sum().item())
+    dc1 = float(field_sum(e1))
+    dc2 = dc1 if e2 is e1 else float(field_sum(e2))
     return float(v[0, 0] + dc1 * dc2 * k0[0] / float(e1.shape[0]) ** 6)
 
 
@@ -269,6 +270,15 @@ class Corr2PCFData(ResultFileIO):
 
 def _is_scalar(v):
     return isinstance(v, (float, int, np.floating))
+
+
+def field_difference(a, b):
+    """a - b as a contiguous float32 tensor, rounded once (float32
+    coefficients are subtracted as they are: the same value, without float64
+    copies of both)."""
+    if a.dtype == torch.float32 and b.dtype == torch.float32:
+        return (a - b).contiguous()
+    return (a.double() - b.double()).to(torch.float32).contiguous()
 
 
 def field_mean_density(field, value_unit="grid"):
@@ -383,17 +393,28 @@ class Corr_2PCF:
                                                                 device=self.device)
         return field @ w
 
+    def _vertex_field(self, value, win, what):
+        """One vertex: the input in the task's normalisation after its window."""
+        field = self._resolve_field(value, what)
+        base = self._field_in_task_normalization(field)
+        if win is None and base is not field:
+            return base  # already a copy of the input
+        return self._apply_window(base, win)
+
     def prepare_input_fields(self):
         self._resolve_sampling()
         needs_data, needs_random = self._required_flags()
         self.data = {}
         self.rand = {}
+        # a second vertex with the first one's input and no windows shares its coefficients
+        plain = self.window1 is None and self.window2 is None
         for i in (1, 2):
             win = getattr(self, f"window{i}")
             if needs_data:
-                base = self._field_in_task_normalization(self._resolve_field(getattr(self, f"sfc_field{i}"),
-                                                                             f"field vertex {i}"))
-                self.data[i] = self._apply_window(base, win)
+                if i == 2 and plain and isinstance(self.sfc_field1, SFCField) and self.sfc_field2 is self.sfc_field1:
+                    self.data[i] = self.data[1]._same_coefficients()
+                else:
+                    self.data[i] = self._vertex_field(getattr(self, f"sfc_field{i}"), win, f"field vertex {i}")
             if needs_random:
                 r = getattr(self, f"random{i}")
                 if r is None or r == "":
@@ -407,9 +428,10 @@ class Corr_2PCF:
                     if ref.field_mean_density(value_unit="grid") is None:
                         raise ValueError("random='uniform' requires a SFCField field with a defined field_integral.")
                     self.rand[i] = field_mean_density(ref)
+                elif i == 2 and plain and isinstance(r, SFCField) and r is self.random1:
+                    self.rand[i] = self.rand[1]._same_coefficients()
                 else:
-                    base = self._field_in_task_normalization(self._resolve_field(r, f"random vertex {i}"))
-                    self.rand[i] = self._apply_window(base, win)
+                    self.rand[i] = self._vertex_field(r, win, f"random vertex {i}")
         self._fields_prepared = True
 
     # ---- products ---------------------------------------------------------------
@@ -453,7 +475,7 @@ class Corr_2PCF:
     @staticmethod
     def _dc(field):
         """float64 sum of a field (its k = 0 Fourier coefficient)."""
-        return float(field.epsilon_device.double().sum().item())
+        return float(field_sum(field.epsilon_device))
 
     def run(self, save_result=True, overwrite=False):
         t0 = time.perf_counter()
@@ -477,6 +499,22 @@ class Corr_2PCF:
                 return self.rand[side]
             return ("delta", side)
 
+        def shared(group):
+            # both vertices hold the same coefficient tensor
+            a, b = group.get(1), group.get(2)
+            return isinstance(a, SFCField) and isinstance(b, SFCField) and a.epsilon_device is b.epsilon_device
+
+        same = {"D": shared(self.data), "R": shared(self.rand)}
+        same["d"] = same["D"] and same["R"]
+
+        def operand_key(k):
+            # the transformed field behind an operand: a vertex that shares
+            # the first one's field shares its spectrum; with a scalar random
+            # (delta's mean is taken out at k = 0) a delta is its data field
+            if k[0] == "d" and _is_scalar(self.rand[int(k[1])]):
+                k = "D" + k[1]
+            return k[0] + "1" if same[k[0]] else k
+
         field_keys, spectra, reals, dcs = {}, [], [], {}
         pairs, pair_products_of = [], {}
         scalar_results = {}
@@ -493,20 +531,18 @@ class Corr_2PCF:
                 continue
             keys = []
             for k in (a, b):
-                side = int(k[1])
-                if k[0] == "d" and not _is_scalar(self.rand[side]):
-                    spec_key = k  # delta against a random field: transform D - R itself
-                    fld_t = (self.data[side].epsilon_device.double()
-                             - self.rand[side].epsilon_device.double()).to(torch.float32)
-                else:
-                    spec_key = k if k[0] != "d" else "D" + k[1]
-                    fld = self.data[side] if spec_key[0] == "D" else self.rand[side]
-                    fld_t = fld.epsilon_device.to(torch.float32)
+                spec_key = operand_key(k)
                 if spec_key not in field_keys:
+                    side = int(spec_key[1])
+                    if spec_key[0] == "d":  # delta against a random field: transform D - R itself
+                        fld_t = field_difference(self.data[side].epsilon_device, self.rand[side].epsilon_device)
+                    else:
+                        fld = self.data[side] if spec_key[0] == "D" else self.rand[side]
+                        fld_t = fld.epsilon_device.to(torch.float32).contiguous()
                     field_keys[spec_key] = len(spectra)
-                    spectra.append(rfft_field(fld_t.contiguous()))
-                    reals.append(fld_t.contiguous())
-                    dcs[spec_key] = float(fld_t.double().sum().item())
+                    spectra.append(rfft_field(fld_t))
+                    reals.append(fld_t)
+                    dcs[spec_key] = float(field_sum(fld_t))
                 keys.append(field_keys[spec_key])
             pair_products_of[prod] = len(pairs)
             pairs.append(tuple(keys))
@@ -547,13 +583,10 @@ class Corr_2PCF:
                 a, b = operand[prod]
 
                 def dc_of(k):
-                    side = int(k[1])
-                    if k[0] == "d":
-                        r = self.rand[side]
-                        if not _is_scalar(r):
-                            return dcs[k]
-                        return dcs["D" + k[1]] - float(r) * float(L) ** 3
-                    return dcs[k]
+                    dc = dcs[operand_key(k)]
+                    if k[0] == "d" and _is_scalar(self.rand[int(k[1])]):
+                        return dc - float(self.rand[int(k[1])]) * float(L) ** 3
+                    return dc
 
                 # the k = 0 term in float64 (mean-subtracted fields lose it in float32)
                 results[prod] = (vals[:, col] + dc_of(a) * dc_of(b) * k0 / N2).reshape(shape)

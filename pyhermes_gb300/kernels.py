@@ -36,6 +36,28 @@ def to_device(a, dtype, device="cuda"):
     return torch.as_tensor(np.ascontiguousarray(a), dtype=dtype, device=device)
 
 
+def field_sum(t):
+    """float64 sum of a tensor as a Python number: hermes_field_sum for a
+    contiguous float32 CUDA tensor, else torch."""
+    if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
+        return t.sum(dtype=torch.complex128 if t.is_complex() else torch.float64).item()
+    buf = torch.empty(2049, dtype=torch.float64, device=t.device)  # the sum, then the blocks' partial sums
+    _lib.check(_lib.load().hermes_field_sum(_ptr(t), t.numel(), _ptr(buf), ctypes.c_void_p(buf.data_ptr() + 8), 16384,
+                                            _stream_ptr(t.device)), "hermes_field_sum")
+    return buf[0].item()
+
+
+def field_shift(t, r):
+    """t - r rounded once to float32, r a Python float: hermes_field_shift for
+    a contiguous float32 CUDA tensor, else torch."""
+    if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
+        return (t.double() - r).to(torch.float32)
+    out = torch.empty_like(t)
+    _lib.check(_lib.load().hermes_field_shift(_ptr(t), t.numel(), float(r), _ptr(out), _stream_ptr(t.device)),
+               "hermes_field_shift")
+    return out
+
+
 class DepositWorkspace:
     """Reusable scratch for hermes_deposit (grows on demand)."""
 

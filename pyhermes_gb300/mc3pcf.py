@@ -34,7 +34,8 @@ import numpy as np
 import torch
 
 from . import _lib
-from .kernels import _ptr, _stream_ptr
+from .corr2pcf import field_difference
+from .kernels import _ptr, _stream_ptr, field_shift
 from .params import task_params
 from .phi import sample_scaling_function
 from .sfc_field import (ResultFileIO, SFCField, check_fout, describe_input, normalize_task_weight_normalization,
@@ -425,8 +426,8 @@ class Corr_3PCF:
         def delta(i):
             r = rand[i]
             if isinstance(r, float):
-                return (data[i].epsilon_device.double() - r).float().contiguous()
-            return (data[i].epsilon_device.double() - r.epsilon_device.double()).float().contiguous()
+                return field_shift(data[i].epsilon_device, r).contiguous()
+            return field_difference(data[i].epsilon_device, r.epsilon_device)
 
         seed_base_rot = self.base_seed + 1
         n = self.mu_arr.size

@@ -29,11 +29,12 @@ import numpy as np
 import torch
 
 from . import _lib
-from .kernels import _ptr, _stream_ptr
-from .params import task_params
+from .kernels import _ptr, _stream_ptr, field_shift
+from .params import plain_copy, task_params
 from .phi import cal_gamma, sample_scaling_function
 from .sfc_field import (ResultFileIO, SFCField, check_fout, describe_input, normalize_task_weight_normalization,
                         read_numpy_pickle, write_numpy_pickle)
+from .corr2pcf import field_difference
 from .window import WindowFunc, phi_power_device, rfft_field
 
 logger = logging.getLogger("pyhermes_gb300.Corr_3PCF_Multipole")
@@ -451,13 +452,15 @@ class GraphedMultipole:
 
 
 def combine_multipole_m_terms(m_values, l):
-    """corr3pcf_multipoles.py:173-180."""
-    coeff = complex(m_values[0])
+    """corr3pcf_multipoles.py:173-180, for one sample's summands or, elementwise,
+    for arrays of them."""
+    sign = 1.0
+    coeff = np.array(m_values[0], dtype=np.complex128)
     for m in range(1, l + 1):
-        coeff += ((-1) ** m) * complex(m_values[m])
-        coeff += ((-1) ** (-m)) * np.conj(complex(m_values[m]))
-    coeff *= (-1) ** l
-    return coeff.real
+        sign = -sign
+        coeff = coeff + sign * np.asarray(m_values[m])
+        coeff = coeff + sign * np.conj(m_values[m])
+    return ((-1.0) ** l * coeff).real
 
 
 class MultipoleEngine:
@@ -581,7 +584,17 @@ class MultipoleEngine:
 
     def ddd(self, pairs, l_min, l_max):
         """DDD_l for samples given as (r12, r13) physical radii -> [n_samples, n_l]."""
-        pairs = [(as_bin(a), as_bin(b)) for a, b in pairs]
+        made = {}
+
+        def bin_of(v):
+            # one BinSpec per distinct radius (a grid of samples repeats each many times)
+            if isinstance(v, BinSpec):
+                return v
+            if v not in made:
+                made[v] = as_bin(v)
+            return made[v]
+
+        pairs = [(bin_of(a), bin_of(b)) for a, b in pairs]
 
         def order(bins):
             return sorted(set(bins), key=lambda b: (b.type, sorted(b.len_args.items()), str(b.key()[2])))
@@ -600,13 +613,13 @@ class MultipoleEngine:
             lms = [(l, m) for l in range(l_min, l_max + 1) for m in range(l + 1)]
             S = self.summands_shared(lms, r12)
             shared = {lm: S[k] for k, lm in enumerate(lms)}
+        ia, ib = [i12[a] for a, _ in pairs], [i13[b] for _, b in pairs]
         for li, l in enumerate(range(l_min, l_max + 1)):
             if shared is not None:
                 Sm = [shared[(l, m)] for m in range(0, l + 1)]
             else:
                 Sm = [self.summands(l, m, r12, r13) for m in range(0, l + 1)]
-            for s, (a, b) in enumerate(pairs):
-                res[s, li] = combine_multipole_m_terms([Sm[m][i12[a], i13[b]] for m in range(l + 1)], l)
+            res[:, li] = combine_multipole_m_terms([S[ia, ib] for S in Sm], l)
         return res
 
     def ddd_plain(self, pairs, l_min, l_max):
@@ -934,10 +947,10 @@ class Corr_3PCF_Multipole:
         """theory/corr3pcf_multipole.py:296-324: mapping targets 'X' or
         'len_args.X' / 'other_args.X' take a sampling parameter (by name)
         or a number."""
-        params = copy.deepcopy(template)
+        params = plain_copy(template)
         mapping = params.pop("mapping", {}) or {}
-        params["len_args"] = copy.deepcopy(params.get("len_args", {}) or {})
-        params["other_args"] = copy.deepcopy(params.get("other_args", {}) or {})
+        params["len_args"] = params.get("len_args", {}) or {}
+        params["other_args"] = params.get("other_args", {}) or {}
         for target, source in mapping.items():
             if isinstance(source, str):
                 if source not in sample:
@@ -994,11 +1007,16 @@ class Corr_3PCF_Multipole:
         normalized = {}
         for i in (1, 2, 3):
             if needs_data:
-                base = self._normalized(self._resolve(getattr(self, f"sfc_field{i}"), f"field vertex {i}"))
+                # a vertex with the input of an earlier one takes that one's normalised field
+                value = getattr(self, f"sfc_field{i}")
+                j = next((j for j in normalized if isinstance(value, SFCField) and getattr(self, f"sfc_field{j}") is value),
+                         None)
+                base = ref if i == 1 else normalized[j] if j else \
+                    self._normalized(self._resolve(value, f"field vertex {i}"))
                 normalized[i] = base
                 self.rho_vertices[i - 1] = base.field_mean_density(value_unit="grid")
                 w = getattr(self, f"window{i}")
-                self.data[i] = base @ WindowFunc(w, base.sfc_info, device=self.device) if w else base.copy()
+                self.data[i] = base @ WindowFunc(w, base.sfc_info, device=self.device) if w else base._same_coefficients()
             if needs_random:
                 r = getattr(self, f"random{i}")
                 if r is None or r == "":
@@ -1007,9 +1025,14 @@ class Corr_3PCF_Multipole:
                     self.rand[i] = self._uniform_random_after_window(normalized.get(i, ref), self.rho_vertices[i - 1],
                                                                      getattr(self, f"window{i}"), i)
                 else:
-                    base = self._normalized(self._resolve(r, f"random vertex {i}"))
                     w = getattr(self, f"window{i}")
-                    self.rand[i] = base @ WindowFunc(w, base.sfc_info, device=self.device) if w else base.copy()
+                    j = next((j for j in range(1, i) if not w and not getattr(self, f"window{j}")
+                              and isinstance(r, SFCField) and getattr(self, f"random{j}") is r), None)
+                    if j:
+                        self.rand[i] = self.rand[j]._same_coefficients()
+                        continue
+                    base = self._normalized(self._resolve(r, f"random vertex {i}"))
+                    self.rand[i] = base @ WindowFunc(w, base.sfc_info, device=self.device) if w else base
         self.radial_profile_diagnostics = self._radial_profile_diagnostics()
         self._fields_prepared = True
 
@@ -1040,14 +1063,24 @@ class Corr_3PCF_Multipole:
             return self.data[i].epsilon_device.to(torch.float32)
         if product == "delta_ddd_l":
             r = self.rand[i]
-            d = self.data[i].epsilon_device.double()
+            d = self.data[i].epsilon_device
             if isinstance(r, float):
-                return (d - r).to(torch.float32)
-            return (d - r.epsilon_device.double()).to(torch.float32)
+                return field_shift(d, r)
+            return field_difference(d, r.epsilon_device)
         r = self.rand[i]
         if isinstance(r, float):
             return torch.full((self.reference.L,) * 3, r, dtype=torch.float32, device=self.device)
         return r.epsilon_device.to(torch.float32)
+
+    def _same_vertex(self, product, i, j):
+        """Whether vertices i and j have the same field in a product."""
+        def same(group):
+            a, b = group.get(i), group.get(j)
+            if isinstance(a, float) or isinstance(b, float):
+                return isinstance(a, float) and isinstance(b, float) and a == b
+            return a is not None and b is not None and a.epsilon_device is b.epsilon_device
+
+        return (product == "rrr_l" or same(self.data)) and (product == "ddd_l" or same(self.rand))
 
     def _pairs(self):
         """(bin12, bin13) per sample: thin-shell radii as floats, other radial
@@ -1095,7 +1128,12 @@ class Corr_3PCF_Multipole:
                     vals[:, 0] = self.rand[1] * self.rand[2] * self.rand[3]
                 setattr(data, product, vals * scale)
                 continue
-            e1, e2, e3 = (self._eps(product, i) for i in (1, 2, 3))
+            eps = {}
+            for i in (1, 2, 3):
+                # vertices that share their data (and random) coefficients share the product's field
+                j = next((j for j in eps if self._same_vertex(product, i, j)), None)
+                eps[i] = eps[j] if j else self._eps(product, i)
+            e1, e2, e3 = eps[1], eps[2], eps[3]
             same23 = (self.sfc_field2 is self.sfc_field3 or self.sfc_field2 == self.sfc_field3) and \
                 self.window2 == self.window3 and (product != "delta_ddd_l" or self.random2 == self.random3)
             eng = MultipoleEngine(e1, e2, e2 if same23 else e3, phi, ref.J, ref.box_size, ref.phi_resolution,

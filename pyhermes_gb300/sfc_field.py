@@ -257,11 +257,21 @@ class SFCField:
         new.format_sfc_params()
         return new
 
+    def _same_coefficients(self):
+        """A field object of its own with this field's metadata that shares
+        its coefficient arrays (read-only use: no copy is made)."""
+        new = self._spawn_like()
+        new._eps_dev, new._eps_host = self._eps_dev, self._eps_host
+        new.format_sfc_params()
+        return new
+
     def _derived_field_integral(self, field):
         t = field.epsilon_device
         if t is None:
             return None
-        total = t.to(torch.complex128 if t.is_complex() else torch.float64).sum().item()
+        from .kernels import field_sum
+
+        total = field_sum(t)
         if isinstance(total, complex):
             if not (np.isfinite(total.real) and np.isfinite(total.imag)):
                 return None
