@@ -587,6 +587,8 @@ struct ContractArgs {
   int J, CX;
   GammaC gm;
   double* partial;   // [gridDim.x][16][16][2]
+  double* items;     // several tiles side by side: [NBL][NBL][2][n_items1], S of every tile
+  int n_items1;      // work items of one tile
   int* status;       // first bounded wait that gave up (tensor-core kernel), else 0
 };
 
@@ -632,10 +634,13 @@ __device__ __forceinline__ void ct_stage_a2(const float2* __restrict__ f2, int s
   }
 }
 
+// NT: tiles side by side in z, NTHR: threads of the block.
+template <int NT = 1, int NTHR = ct::kThreads>
 __device__ __forceinline__ void ct_stage_eps(const float* __restrict__ eps1, float* buf, int xe, int y0, int z0, int L, int Lm) {
+  constexpr int EZ = NT * ct::TZ + 2;
   const long long xb = (long long)(xe & Lm) * L;
-  for (int c = threadIdx.x; c < ct::kEpsPlane; c += ct::kThreads) {
-    const int ey = c / ct::EZ, ez = c - ey * ct::EZ;
+  for (int c = threadIdx.x; c < ct::EY * EZ; c += NTHR) {
+    const int ey = c / EZ, ez = c - ey * EZ;
     cp_async4(buf + c, eps1 + (xb + ((y0 + ey) & Lm)) * L + ((z0 + ez) & Lm));
   }
 }
@@ -870,7 +875,41 @@ __global__ void __launch_bounds__(ct::kThreads, 2) mp_contract_kernel(ContractAr
 namespace hf {
 constexpr int kHCol = 20;                      // floats per column: [5 uy][4] (3 used)
 constexpr int kHPlane = ct::kCols * kHCol;
+// floats between the h planes of tiles side by side (4 banks apart, so the
+// 16-byte reads of a half-warp's tiles do not conflict)
+constexpr int kHTile = kHPlane + 4;
+template <int NT>
+constexpr int kHSlot = NT == 1 ? kHPlane : NT * kHTile;  // one plane of all tiles
 }  // namespace hf
+
+// h plane from a staged eps plane of NT > 1 tiles: H[tile][col][uy+2][l1z],
+// the same sums as ct_compute_h.  kPer threads per column (each a range of
+// the five uy), so that 512 threads cover the tiles' columns once.
+template <int NT>
+__device__ __forceinline__ void ct_compute_h_tiles(const float* __restrict__ w, const float* __restrict__ e,
+                                                   float* __restrict__ h) {
+  constexpr int EZ = NT * ct::TZ + 2, kPer = 8 / NT;  // 512 / (64 NT)
+  const int part = threadIdx.x / (ct::kCols * NT), cc = threadIdx.x % (ct::kCols * NT);
+  const int tile = cc / ct::kCols, col = cc % ct::kCols;
+  const int cy = col / ct::TZ, cz = tile * ct::TZ + (col & (ct::TZ - 1));
+  float ev[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) ev[i][j] = e[(cy + i) * EZ + cz + j];
+  float* dst = h + tile * hf::kHTile + col * hf::kHCol;
+#pragma unroll
+  for (int rep = 0; rep < (5 + kPer - 1) / kPer; ++rep) {
+    const int ay = rep * kPer + part;
+    if (ay < 5) {
+      const float w0 = w[ay * 3], w1 = w[ay * 3 + 1], w2 = w[ay * 3 + 2];
+      float o[3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) o[j] = fmaf(w2, ev[2][j], fmaf(w1, ev[1][j], w0 * ev[0][j]));
+      *reinterpret_cast<float4*>(dst + ay * 4) = make_float4(o[0], o[1], o[2], 0.f);
+    }
+  }
+}
 
 // h plane from a staged eps plane: H[col][uy+2][l1z].  Four threads per
 // column; thread `part` writes uy + 2 = part (and 4 for part 0).
@@ -935,9 +974,16 @@ constexpr int kA3Buf = kBinStride * kA3P;
 static_assert(kA3Buf >= ct::kA3Plane, "a3 buffer");
 constexpr uint32_t kIdesc = hermes::tc::idesc_bf16_f32(128, kN, true, true);
 // 1 KB slack for the runtime 1024-byte alignment of the swizzled operands
+template <int NT>
 constexpr size_t kSmem = 1024 + 2 * kOpBytes + 2 * kRawBytes + sizeof(float2) * 2 * kA3Buf +
-                         sizeof(float) * (3 * hf::kHPlane + 2 * ct::kEpsPlane) +
+                         sizeof(float) * (3 * hf::kHSlot<NT> + 2 * ct::EY * (NT * ct::TZ + 2)) +
                          sizeof(double) * 2 * kMaxBins * kMaxBins + 128;
+static_assert(kSmem<8> <= 227 * 1024 && 2 * (kSmem<1> + 1024) <= 228 * 1024, "shared memory of the contraction");
+// Threads of a block: one tile runs as two blocks of 256 threads per SM (2 x 2
+// columns a thread); tiles side by side need their own h planes, so one
+// block of 512 threads (2 x 1 columns a thread) fills the SM.
+template <int NT>
+constexpr int kThr = NT == 1 ? ct::kThreads : 512;
 }  // namespace tcc
 
 // (lower half, upper half) -> packed BF16x2, round to nearest even
@@ -969,29 +1015,32 @@ __device__ __forceinline__ void tc_put_pair(unsigned char* op, int cell, int b, 
 }
 
 // a3 plane x_a from bin-major fields (bin b at src3 + b * bstride) -> buf
-// [16][kA3P] float2; bins nb3 .. 15 are written as zeros.  The copies are
-// 16 bytes, two cells (2p, 2p + 1) of one row: with z0 a multiple of 8 the
-// pair starts at an even z and never straddles the periodic wrap, so both
-// ends are 16-byte aligned.  Thread t copies bin t >> 4, pairs
-// p = (t & 15) + 16 i of the 72 in the 12 x 12 plane; the (row, pair
-// column) of the next one is a fixed step (16 pairs = two rows of 6 and 4).
+// [16 slots][kA3P] float2; slot = tile * (16 / NT) + bin, bins nb3 and up
+// are written as zeros.  The copies are 16 bytes, two cells (2p, 2p + 1) of
+// one row: with z0 a multiple of 8 the pair starts at an even z and never
+// straddles the periodic wrap, so both ends are 16-byte aligned.  kPer
+// threads copy a slot, thread j the pairs j + kPer i of the 72 in the
+// 12 x 12 plane; the (row, pair column) of the next one is a fixed step
+// (rows hold six pairs).
+template <int NT>
 __device__ __forceinline__ void ct_stage_a3_bm(const float2* __restrict__ src3, long long bstride, int nb3,
                                                float2* buf, int xa, int y0, int z0, int L, int Lm) {
-  static_assert(ct::kThreads == 16 * kBinStride && ct::HY * ct::HZ == 144 && ct::HZ == 12 && ct::TZ % 8 == 0,
-                "a3 staging map");
   constexpr int kPairs = ct::HY * ct::HZ / 2;  // 72
-  const int bb = threadIdx.x >> 4, j = threadIdx.x & 15;
-  float2* dst = buf + bb * tcc::kA3P + 2 * j;
-  const int n = j < kPairs - 64 ? 5 : 4;
-  if (bb < nb3) {
-    const float2* src = src3 + bb * bstride + (long long)(xa & Lm) * L * L;
+  constexpr int kPer = tcc::kThr<NT> / kBinStride, NBL = kBinStride / NT;
+  static_assert(ct::HY * ct::HZ == 144 && ct::HZ == 12 && ct::TZ % 8 == 0, "a3 staging map");
+  const int slot = threadIdx.x / kPer, j = threadIdx.x % kPer;
+  const int bin = slot % NBL, zt = z0 + ct::TZ * (slot / NBL);
+  float2* dst = buf + slot * tcc::kA3P + 2 * j;
+  const int n = (kPairs - j + kPer - 1) / kPer;
+  if (bin < nb3) {
+    const float2* src = src3 + bin * bstride + (long long)(xa & Lm) * L * L;
     int hy = j / 6;
     int hz = 2 * (j - 6 * hy);
 #pragma unroll 1
     for (int i = 0; i < n; ++i) {
-      cp_async16(dst + 32 * i, src + ((y0 - 2 + hy) & Lm) * L + ((z0 - 2 + hz) & Lm));
-      hz += 8;
-      hy += 2;
+      cp_async16(dst + 2 * kPer * i, src + ((y0 - 2 + hy) & Lm) * L + ((zt - 2 + hz) & Lm));
+      hz += 2 * (kPer % 6);
+      hy += kPer / 6;
       if (hz >= ct::HZ) {
         hz -= ct::HZ;
         hy += 1;
@@ -999,17 +1048,29 @@ __device__ __forceinline__ void ct_stage_a3_bm(const float2* __restrict__ src3, 
     }
   } else {
 #pragma unroll 1
-    for (int i = 0; i < n; ++i) *reinterpret_cast<float4*>(dst + 32 * i) = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < n; ++i) *reinterpret_cast<float4*>(dst + 2 * kPer * i) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 
 // kBM: fields in the bin-major layout [bin][cell] that cuFFT writes (a2 by a
 // 4-D TMA map over (z, y, x, bin), a3 staged per bin); otherwise the
 // bin-interleaved [cell][16] layout or a single [cell] field.
-template <bool kBM>
-__global__ void __launch_bounds__(ct::kThreads, 2)
+//
+// NT > 1 (bin-major, at most 16 / NT bins): the 16 slots of the operands are
+// NT tiles side by side in z times NBL = 16 / NT bins instead of 16 bins, of
+// which few would be used.  Slot (t, b2) of A and (t', b3) of B meet in D as
+// before; the t = t' blocks are the tiles' own products (each with the same
+// operands in the same order as when the tile runs alone), the others are
+// not read.  A tile's S goes to A.items, and mp_reduce_items_kernel adds the
+// tiles in the order of the one-tile blocks: the result is the same bits.
+template <bool kBM, int NT>
+__global__ void __launch_bounds__(tcc::kThr<NT>, NT == 1 ? 2 : 1)
 mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map) {
+  static_assert(kBM || NT == 1, "tiles side by side read bin-major fields");
   namespace tc = hermes::tc;
+  constexpr int kThr = tcc::kThr<NT>, NBL = kBinStride / NT;
+  constexpr int CZ = NT == 1 ? 2 : 1, NC = 2 * CZ;  // columns of a thread: 2 (y) x CZ (z)
+  constexpr int kHS = hf::kHSlot<NT>, kEps = ct::EY * (NT * ct::TZ + 2);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* base = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   unsigned char* abf = base;                                       // A operand (a2 split)
@@ -1018,8 +1079,8 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
   float2* abuf = reinterpret_cast<float2*>(reinterpret_cast<unsigned char*>(araw) + 2 * tcc::kRawBytes);
   double* dacc = reinterpret_cast<double*>(abuf + 2 * tcc::kA3Buf);  // [16][16][2]
   float* hring = reinterpret_cast<float*>(dacc + 2 * kMaxBins * kMaxBins);  // [3][kHPlane]
-  float* epsb = hring + 3 * hf::kHPlane;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(epsb + 2 * ct::kEpsPlane);  // tma[2], mma
+  float* epsb = hring + 3 * kHS;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(epsb + 2 * kEps);  // tma[2], mma
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3);
   float* gsm = reinterpret_cast<float*>(tmem_slot + 1);                  // 15 h-pass weights
   int* s_abort = reinterpret_cast<int*>(gsm + 16);
@@ -1027,13 +1088,21 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
 
   const int J = A.J, L = 1 << J, Lm = L - 1, CX = A.CX;
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int b = tid & 15;
-  // 2x2 column block of this half-warp: the two half-warps of a warp take
+  const int b = tid & 15;  // operand slot: bin (NT = 1) or (tile, bin)
+  // column block of this half-warp: the two half-warps of a warp take
   // blocks 4 cells apart in z, so their rows of the swizzled G operand fall
   // in complementary halves of the 128-byte rows (no bank conflict)
   const int hw = (tid >> 4) & 1, wq = tid >> 5;
-  const int cy = 2 * (wq >> 1), cz = 4 * hw + 2 * (wq & 1);
-  const int nty = L / ct::TY, ntz = L / ct::TZ;
+  const int cy = NT == 1 ? 2 * (wq >> 1) : 2 * (wq >> 2);
+  const int cz = NT == 1 ? 4 * hw + 2 * (wq & 1) : 4 * hw + (wq & 3);
+  const int nty = L / ct::TY, ntz = L / (NT * ct::TZ);
+  auto stage_eps = [&](float* buf, int xe, int y0, int z0) { ct_stage_eps<NT, kThr>(A.eps1, buf, xe, y0, z0, L, Lm); };
+  auto compute_h = [&](const float* e, float* h, const float* w) {
+    if constexpr (NT == 1)
+      ct_compute_h(w, e, h);
+    else
+      ct_compute_h_tiles<NT>(w, e, h);
+  };
   const int n_items = (L / CX) * nty * ntz;
   const int nsteps = CX + 4;
   const bool tma_a2 = kBM || A.s2 == kBinStride;
@@ -1054,7 +1123,7 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
     if (tma_a2) tc::tma_prefetch_desc(&a2map);
   }
   if (warp == 0) tc::tmem_alloc(tmem_slot, tcc::kTmemCols);
-  for (int i = tid; i < 2 * kMaxBins * kMaxBins; i += ct::kThreads) dacc[i] = 0.0;
+  for (int i = tid; i < 2 * kMaxBins * kMaxBins; i += kThr) dacc[i] = 0.0;
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
@@ -1065,31 +1134,31 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
 
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const int tz = item % ntz, ty = (item / ntz) % nty, xc = item / (ntz * nty);
-    const int x0 = xc * CX, y0 = ty * ct::TY, z0 = tz * ct::TZ;
+    const int x0 = xc * CX, y0 = ty * ct::TY, z0 = tz * (NT * ct::TZ);
     // prologue: h(x0-2), h(x0-1), h(x0) into ring slots 0, 1, 2; a3 plane x0-2
-    ct_stage_eps(A.eps1, epsb, x0 - 2, y0, z0, L, Lm);
-    ct_stage_eps(A.eps1, epsb + ct::kEpsPlane, x0 - 1, y0, z0, L, Lm);
+    stage_eps(epsb, x0 - 2, y0, z0);
+    stage_eps(epsb + kEps, x0 - 1, y0, z0);
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
-    ct_compute_h(gsm, epsb, hring);
-    ct_compute_h(gsm, epsb + ct::kEpsPlane, hring + hf::kHPlane);
+    compute_h(epsb, hring, gsm);
+    compute_h(epsb + kEps, hring + kHS, gsm);
     __syncthreads();
-    if (kBM)
-      ct_stage_a3_bm(A.src3, A.bstride, A.nb3s, abuf, x0 - 2, y0, z0, L, Lm);
+    if constexpr (kBM)
+      ct_stage_a3_bm<NT>(A.src3, A.bstride, A.nb3s, abuf, x0 - 2, y0, z0, L, Lm);
     else
       ct_stage_a3(A.src3, A.s3, abuf, x0 - 2, y0, z0, L, Lm);
-    ct_stage_eps(A.eps1, epsb, x0, y0, z0, L, Lm);
+    stage_eps(epsb, x0, y0, z0);
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
-    ct_compute_h(gsm, epsb, hring + 2 * hf::kHPlane);
+    compute_h(epsb, hring + 2 * kHS, gsm);
 
-    float2 G[5][4];
+    float2 G[5][NC];
 #pragma unroll
     for (int q = 0; q < 5; ++q)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) G[q][c] = make_float2(0.f, 0.f);
+      for (int c = 0; c < NC; ++c) G[q][c] = make_float2(0.f, 0.f);
     bool first_mma = true;
 
     // Two block barriers per step: the first makes the h plane computed at
@@ -1100,20 +1169,23 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
       if (st + 1 < nsteps) {
         // a3 plane xa+1 and eps plane xa+3: their buffers' last readers (the
         // stencil one step back, the h pass two steps back) are done
-        if (kBM)
-          ct_stage_a3_bm(A.src3, A.bstride, A.nb3s, abuf + ((st + 1) & 1) * tcc::kA3Buf, xa + 1, y0, z0, L, Lm);
+        if constexpr (kBM)
+          ct_stage_a3_bm<NT>(A.src3, A.bstride, A.nb3s, abuf + ((st + 1) & 1) * tcc::kA3Buf, xa + 1, y0, z0, L, Lm);
         else
           ct_stage_a3(A.src3, A.s3, abuf + ((st + 1) & 1) * tcc::kA3Buf, xa + 1, y0, z0, L, Lm);
-        ct_stage_eps(A.eps1, epsb + ((st + 1) & 1) * ct::kEpsPlane, xa + 3, y0, z0, L, Lm);
+        stage_eps(epsb + ((st + 1) & 1) * kEps, xa + 3, y0, z0);
         // a2 plane of the next step's product (its buffer's last reader, the
         // split two steps back, finished before the last block barrier)
         if (tma_a2 && tid == 0 && st + 1 >= 4) {
           uint64_t* bar = &bars[(st + 1) & 1];
           tc::fence_proxy_async_smem();
           tc::mbar_arrive_expect_tx(bar, tcc::kRawBytes);
-          if (kBM)
-            tc::tma_load_4d(araw + ((st + 1) & 1) * (tcc::kRawBytes / 4), &a2map, bar, 2 * z0, y0, (xa - 1) & Lm, 0);
-          else
+          if (kBM) {
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+              tc::tma_load_4d(araw + ((st + 1) & 1) * (tcc::kRawBytes / 4) + t * (NBL * 2 * ct::kCols), &a2map, bar,
+                              2 * (z0 + ct::TZ * t), y0, (xa - 1) & Lm, 0);
+          } else
             tc::tma_load_4d(araw + ((st + 1) & 1) * (tcc::kRawBytes / 4), &a2map, bar, 0, z0, y0, (xa - 1) & Lm);
         }
       }
@@ -1121,18 +1193,28 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
       __syncthreads();
       {
         const float2* ap = abuf + (st & 1) * tcc::kA3Buf;
-        const float* hp0 = hring + (st % 3) * hf::kHPlane;
-        const float* hp1 = hring + ((st + 1) % 3) * hf::kHPlane;
-        const float* hp2 = hring + ((st + 2) % 3) * hf::kHPlane;
-        float2 T[3][4];
+        const int ht = NT == 1 ? 0 : (b / NBL) * hf::kHTile;
+        const float* hp0 = hring + (st % 3) * kHS + ht;
+        const float* hp1 = hring + ((st + 1) % 3) * kHS + ht;
+        const float* hp2 = hring + ((st + 2) % 3) * kHS + ht;
+        float2 T[3][NC];
 #pragma unroll
         for (int d = 0; d < 3; ++d)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) T[d][c] = make_float2(0.f, 0.f);
+          for (int c = 0; c < NC; ++c) T[d][c] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int r = 0; r < 6; ++r) {
           float2 av[6];
-          if (kBM) {  // two cells per 16-byte load (cz even, kA3P even)
+          if (kBM && CZ == 1) {  // the pairs around five cells that start at an odd or even z
+            const float4* row4 = reinterpret_cast<const float4*>(ap + b * tcc::kA3P + (cy + r) * ct::HZ + (cz & ~1));
+            const float4 p0 = row4[0], p1 = row4[1], p2 = row4[2];
+            const bool odd = cz & 1;  // the same for the whole warp
+            av[0] = odd ? make_float2(p0.z, p0.w) : make_float2(p0.x, p0.y);
+            av[1] = odd ? make_float2(p1.x, p1.y) : make_float2(p0.z, p0.w);
+            av[2] = odd ? make_float2(p1.z, p1.w) : make_float2(p1.x, p1.y);
+            av[3] = odd ? make_float2(p2.x, p2.y) : make_float2(p1.z, p1.w);
+            av[4] = odd ? make_float2(p2.z, p2.w) : make_float2(p2.x, p2.y);
+          } else if (kBM) {  // two cells per 16-byte load (cz even, kA3P even)
             const float4* row4 = reinterpret_cast<const float4*>(ap + b * tcc::kA3P + (cy + r) * ct::HZ + cz);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
@@ -1145,9 +1227,9 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
             for (int k = 0; k < 6; ++k) av[k] = ap[((cy + r) * ct::HZ + cz + k) * kBinStride + b];
           }
           // Rz_{l1z}(row, cz + dz) = sum_{l2z} Gamma[l1z][l2z] a3(row, cz + dz + l1z - l2z)
-          float2 rz[2][3];
+          float2 rz[CZ][3];
 #pragma unroll
-          for (int dz = 0; dz < 2; ++dz)
+          for (int dz = 0; dz < CZ; ++dz)
 #pragma unroll
             for (int l1z = 0; l1z < 3; ++l1z) {
               const float g0 = A.gm.g[l1z * 3], g1 = A.gm.g[l1z * 3 + 1], g2 = A.gm.g[l1z * 3 + 2];
@@ -1160,16 +1242,16 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
             const int uy = r - 2 - dy;
             if (uy < -2 || uy > 2) continue;
 #pragma unroll
-            for (int dz = 0; dz < 2; ++dz) {
+            for (int dz = 0; dz < CZ; ++dz) {
               const int hoff = ((cy + dy) * ct::TZ + cz + dz) * hf::kHCol + (uy + 2) * 4;
 #pragma unroll
               for (int d = 0; d < 3; ++d) {
                 const float4 h4 = *reinterpret_cast<const float4*>((d == 0 ? hp0 : (d == 1 ? hp1 : hp2)) + hoff);
-                float2 t = T[d][dy * 2 + dz];
+                float2 t = T[d][dy * CZ + dz];
                 t = __ffma2_rn(make_float2(h4.x, h4.x), rz[dz][0], t);
                 t = __ffma2_rn(make_float2(h4.y, h4.y), rz[dz][1], t);
                 t = __ffma2_rn(make_float2(h4.z, h4.z), rz[dz][2], t);
-                T[d][dy * 2 + dz] = t;
+                T[d][dy * CZ + dz] = t;
               }
             }
           }
@@ -1180,7 +1262,7 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
           for (int l1x = 0; l1x < 3; ++l1x) {
             const float gx = A.gm.g[l1x * 3 + d];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) G[d - l1x + 2][c] = __ffma2_rn(make_float2(gx, gx), T[d][c], G[d - l1x + 2][c]);
+            for (int c = 0; c < NC; ++c) G[d - l1x + 2][c] = __ffma2_rn(make_float2(gx, gx), T[d][c], G[d - l1x + 2][c]);
           }
       }
       // G(xa - 2) and the a2 plane xa - 2 become the operands of this plane's MMA
@@ -1192,13 +1274,15 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
           mma_pending = false;
         }
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < NC; ++c) {
           float2 g = G[0][c];
           if (A.conj_src) g = make_float2(A.sign * g.x, -A.sign * g.y);
-          tc_put_pair(gbf, (cy + (c >> 1)) * ct::TZ + cz + (c & 1), b, g.x, g.y);
+          tc_put_pair(gbf, (cy + c / CZ) * ct::TZ + cz + c % CZ, b, g.x, g.y);
         }
-        // this thread's operand row (cell) and bins 4q .. 4q+3; with bin-major
-        // planes ([bin][cell] in shared memory) a warp takes 32 cells of one q
+        // this thread's operand row (cell) and slots kS q .. kS q + kS - 1; with
+        // bin-major planes ([slot][cell] in shared memory) a warp takes 32
+        // cells of one q
+        constexpr int kS = 1024 / kThr;
         const int cell = kBM ? (tid & 63) : (tid >> 2), q = kBM ? (tid >> 6) : (tid & 3);
         float v[8];
         if (kBM) {
@@ -1206,8 +1290,8 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
           if (!tc::mbar_wait(&bars[st & 1], par)) *s_abort = 1;  // a2 plane (TMA)
           const float* src = araw + (st & 1) * (tcc::kRawBytes / 4) + cell * 2;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float2 p = *reinterpret_cast<const float2*>(src + (4 * q + i) * 128);
+          for (int i = 0; i < kS; ++i) {
+            const float2 p = *reinterpret_cast<const float2*>(src + (kS * q + i) * 128);
             v[2 * i] = p.x;
             v[2 * i + 1] = p.y;
           }
@@ -1231,26 +1315,34 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
         if (st & 1) tma_ph1 ^= (tma_a2 ? 1u : 0u); else tma_ph0 ^= (tma_a2 ? 1u : 0u);
         uint32_t hv[4], mv[4], lv[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) split3(v[2 * i], v[2 * i + 1], hv[i], mv[i], lv[i]);
+        for (int i = 0; i < kS; ++i) split3(v[2 * i], v[2 * i + 1], hv[i], mv[i], lv[i]);
         unsigned char* atom = abf + (cell >> 3) * 1024;
-        // elements 8q .. 8q+7 of the row: chunk q (hi), 4 + q (mid), q of column 1 (lo)
-        *reinterpret_cast<uint4*>(atom + tc::sw128_offset(cell & 7, q)) = make_uint4(hv[0], hv[1], hv[2], hv[3]);
-        *reinterpret_cast<uint4*>(atom + tc::sw128_offset(cell & 7, 4 + q)) = make_uint4(mv[0], mv[1], mv[2], mv[3]);
-        *reinterpret_cast<uint4*>(atom + tcc::kAtomCol + tc::sw128_offset(cell & 7, q)) =
-            make_uint4(lv[0], lv[1], lv[2], lv[3]);
+        if constexpr (kS == 4) {
+          // elements 8q .. 8q+7 of the row: chunk q (hi), 4 + q (mid), q of column 1 (lo)
+          *reinterpret_cast<uint4*>(atom + tc::sw128_offset(cell & 7, q)) = make_uint4(hv[0], hv[1], hv[2], hv[3]);
+          *reinterpret_cast<uint4*>(atom + tc::sw128_offset(cell & 7, 4 + q)) = make_uint4(mv[0], mv[1], mv[2], mv[3]);
+          *reinterpret_cast<uint4*>(atom + tcc::kAtomCol + tc::sw128_offset(cell & 7, q)) =
+              make_uint4(lv[0], lv[1], lv[2], lv[3]);
+        } else {  // elements 4q .. 4q+3: half (q & 1) of the chunks of q / 2
+          const uint32_t half = (q & 1) * 8;
+          *reinterpret_cast<uint2*>(atom + tc::sw128_offset(cell & 7, q >> 1) + half) = make_uint2(hv[0], hv[1]);
+          *reinterpret_cast<uint2*>(atom + tc::sw128_offset(cell & 7, 4 + (q >> 1)) + half) = make_uint2(mv[0], mv[1]);
+          *reinterpret_cast<uint2*>(atom + tcc::kAtomCol + tc::sw128_offset(cell & 7, q >> 1) + half) =
+              make_uint2(lv[0], lv[1]);
+        }
         tc::fence_proxy_async_smem();
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) G[q][c] = G[q + 1][c];
+        for (int c = 0; c < NC; ++c) G[q][c] = G[q + 1][c];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) G[4][c] = make_float2(0.f, 0.f);
+      for (int c = 0; c < NC; ++c) G[4][c] = make_float2(0.f, 0.f);
       cp_async_wait<0>();
       __syncthreads();
       if (*s_abort) break;
       // h(xa + 3) for the next step, into the ring slot this step's T_0 used
-      if (st + 1 < nsteps) ct_compute_h(gsm, epsb + ((st + 1) & 1) * ct::kEpsPlane, hring + (st % 3) * hf::kHPlane);
+      if (st + 1 < nsteps) compute_h(epsb + ((st + 1) & 1) * kEps, hring + (st % 3) * kHS, gsm);
       if (full) {
         if (tid == 0) {
           tc::tc_fence_after();
@@ -1294,7 +1386,7 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
     }
     tc::tc_fence_before();
     __syncthreads();
-    {
+    if (kThr == 256 || tid < 256) {
       const int b2 = tid >> 4, b3 = tid & 15;
       double sr = 0.0, si = 0.0;
 #pragma unroll
@@ -1309,14 +1401,24 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
           si += (double)rr[1] + (double)ri[0];
         }
       }
-      dacc[(b2 * kMaxBins + b3) * 2] += sr;
-      dacc[(b2 * kMaxBins + b3) * 2 + 1] += si;
+      if constexpr (NT == 1) {
+        dacc[(b2 * kMaxBins + b3) * 2] += sr;
+        dacc[(b2 * kMaxBins + b3) * 2 + 1] += si;
+      } else if (b2 / NBL == b3 / NBL) {
+        const int item1 = (xc * nty + ty) * (ntz * NT) + tz * NT + b2 / NBL;
+        const size_t o = ((size_t)(b2 % NBL) * NBL + b3 % NBL) * 2;
+        A.items[o * A.n_items1 + item1] = sr;
+        A.items[(o + 1) * A.n_items1 + item1] = si;
+      }
     }
     __syncthreads();  // stage (a3 buffer) idle before the next item's prologue
   }
   const int why = *s_abort;
-  for (int i = tid; i < 2 * kMaxBins * kMaxBins; i += ct::kThreads)
-    A.partial[(long long)blockIdx.x * 2 * kMaxBins * kMaxBins + i] = why ? __longlong_as_double(0x7ff8000000000000LL) : dacc[i];
+  if constexpr (NT == 1) {
+    for (int i = tid; i < 2 * kMaxBins * kMaxBins; i += kThr)
+      A.partial[(long long)blockIdx.x * 2 * kMaxBins * kMaxBins + i] =
+          why ? __longlong_as_double(0x7ff8000000000000LL) : dacc[i];
+  }
   if (why && tid == 0 && A.status) atomicCAS(A.status, 0, why);
   __syncthreads();
   if (warp == 0) {
@@ -1339,6 +1441,32 @@ __global__ void mp_reduce_kernel(const double* __restrict__ partial, int nblocks
     __syncthreads();
   }
   if (threadIdx.x == 0) out[o] = sh[0] * scale;
+}
+
+// out[b2][b3][part] of nbl x nbl bins from the tiles' S (zero outside): the
+// order of mp_reduce_kernel over nblocks one-tile blocks, block b holding the
+// sum of tiles b, b + nblocks, ...  NaN when a wait of the contraction gave up.
+__global__ void __launch_bounds__(256)
+mp_reduce_items_kernel(const double* __restrict__ items, int n_items, int nbl, int nblocks, const int* __restrict__ status,
+                       double* __restrict__ out, double scale) {
+  const int b2 = blockIdx.x >> 5, b3 = (blockIdx.x >> 1) & 15, part = blockIdx.x & 1;
+  double s = 0.0;
+  if (b2 < nbl && b3 < nbl) {
+    const double* v = items + ((size_t)(b2 * nbl + b3) * 2 + part) * n_items;
+    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
+      double p = 0.0;
+      for (int i = b; i < n_items; i += nblocks) p += v[i];
+      s += p;
+    }
+  }
+  __shared__ double sh[256];
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[blockIdx.x] = *status ? __longlong_as_double(0x7ff8000000000000LL) : sh[0] * scale;
 }
 
 // ---- plain reference-form contraction of one (a2, a3) pair -----------------
@@ -1458,6 +1586,11 @@ YlmConst make_ylm_pair(int l) {
   return Y;
 }
 
+// Planes of a contraction's work item: 128 from L = 256 up (what the tile
+// autotuner picks there: the 4-plane halo costs 3% and work items still
+// outnumber the blocks), else min(64, L).
+int default_chunk(int L) { return L >= 256 ? 128 : (L < ct::kMaxCX ? L : ct::kMaxCX); }
+
 size_t table_floats(int J) {
   const long long L = 1LL << J;
   return (size_t)(3 * L * L + 1) * kBinStride;
@@ -1476,6 +1609,8 @@ struct MpWs {
   double* partial;   // per-block partial sums [1024][16][16][2]
   double* dout;      // reduced S [16][16][2]
   int* status;       // bounded-wait status of the tensor-core contraction
+  double* items;     // S of every tile of a contraction of at most 8 bins
+  size_t n_item_values;
   float2* binmajor;  // nb > 1: bin-major fields [nb][L^3]
   size_t used;
 };
@@ -1489,6 +1624,10 @@ MpWs carve_ws(void* ws, size_t cap, int J, int nb) {
   w.partial = c.take<double>((size_t)1024 * kMaxBins * kMaxBins * 2);
   w.dout = c.take<double>((size_t)kMaxBins * kMaxBins * 2);
   w.status = c.take<int>(16);
+  // 8 x 8 x 2 values of every (x-chunk, 8 x 8 column tile) at the default chunk
+  const size_t L = (size_t)1 << J;
+  w.n_item_values = 128 * (L / default_chunk((int)L)) * (L / ct::TY) * (L / ct::TZ);
+  w.items = c.take<double>(w.n_item_values);
   w.binmajor = nb > 1 ? c.take<float2>((size_t)nb << (3 * J)) : nullptr;
   w.used = c.used;
   return w;
@@ -1783,15 +1922,15 @@ static int make_a2_map(const void* fields, int L, CUtensorMap* map) {
 }
 
 // 4-D tensor map over bin-major fields [bin][x][y][z] (float32 view: z as 2L
-// floats), box 16 floats (8 z) x 8 (y) x 1 (x) x 16 (bins; bins >= nb read
+// floats), box 16 floats (8 z) x 8 (y) x 1 (x) x box_bins (bins >= nb read
 // as zeros): one contraction tile's a2 plane as [bin][8 y][8 z] complex.
-static int make_a2_map_bm(const void* fields, int L, int nb, CUtensorMap* map) {
+static int make_a2_map_bm(const void* fields, int L, int nb, int box_bins, CUtensorMap* map) {
   auto enc = tensor_map_encoder();
   if (!enc) return fail(HERMES_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
   const cuuint64_t dims[4] = {2 * (cuuint64_t)L, (cuuint64_t)L, (cuuint64_t)L, (cuuint64_t)nb};
   const cuuint64_t row = sizeof(float) * 2 * (cuuint64_t)L;
   const cuuint64_t strides[3] = {row, row * L, row * L * L};
-  const cuuint32_t box[4] = {2 * ct::TZ, ct::TY, 1, kBinStride};
+  const cuuint32_t box[4] = {2 * ct::TZ, ct::TY, 1, (cuuint32_t)box_bins};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(fields), dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1801,6 +1940,26 @@ static int make_a2_map_bm(const void* fields, int L, int nb, CUtensorMap* map) {
 }
 
 enum { kEngineTensor = 0, kEngineSimt = 1, kEngineTensorBinMajor = 2 };
+
+// Tiles side by side in the tensor-core contraction of nb bins (1, 2, 4 or
+// 8, with 16 / tiles >= nb bin slots each): the count with the fewest rounds
+// of work.  Two blocks of one tile share an SM, so a round of those counts
+// two; a block of several tiles has the SM to itself, and a round counts 1.1
+// for the h planes of the tiles.  At J = 8, 2 bins take 0.85 ms with 8 tiles
+// (2 rounds) and 3.02 ms with one (7 rounds of 2).
+static int contract_tiles(int nb, int per_tile, int L, int ctas_per_sm, int nsm) {
+  const int slots = ctas_per_sm * nsm;
+  int best = 1;
+  double cost = ctas_per_sm * (double)((per_tile + slots - 1) / slots);
+  for (int t = 2; t <= 8 && t * nb <= kBinStride && t * ct::TZ <= L; t *= 2) {
+    const double c = 1.1 * (double)((per_tile / t + nsm - 1) / nsm);
+    if (c < cost) {
+      best = t;
+      cost = c;
+    }
+  }
+  return best;
+}
 
 // Launches the contraction and the float64 reduction into dout [16][16][2]
 // (already multiplied by `scale`), with no host synchronisation.  engine:
@@ -1822,10 +1981,7 @@ static int mp_contract_launch(const float* eps1, const void* fields2, int nb2, c
   if (nb3 < 1 || nb3 > kMaxBins) return fail(HERMES_ERR_INVALID, "multipole_contract: nb3=%d", nb3);
   if (J < 4 || J > 10) return fail(HERMES_ERR_INVALID, "multipole_contract: J=%d outside [4,10]", J);
   const int L = 1 << J;
-  // default x-chunk: 128 planes from L = 256 up (what the tile autotuner picks
-  // there: the 4-plane halo costs 3% and work items still outnumber the CTAs),
-  // else min(64, L)
-  if (chunk_x == 0) chunk_x = L >= 256 ? 128 : (L < ct::kMaxCX ? L : ct::kMaxCX);
+  if (chunk_x == 0) chunk_x = default_chunk(L);
   if (chunk_x < 1 || chunk_x > L || (chunk_x & (chunk_x - 1)) != 0)
     return fail(HERMES_ERR_INVALID, "multipole_contract: chunk_x=%d must be a power of two in [1, L=%d]", chunk_x, L);
   if (ctas_per_sm == 0) ctas_per_sm = 2;
@@ -1836,20 +1992,30 @@ static int mp_contract_launch(const float* eps1, const void* fields2, int nb2, c
   if (!workspace || workspace_bytes < need)
     return fail(HERMES_ERR_WORKSPACE, "multipole_contract: workspace %zu < %zu", workspace_bytes, need);
   const MpWs w = carve_ws(workspace, workspace_bytes, J, 1);
-  static bool smem_set[3][64] = {{false}};
+  const int nsm = sm_count();
+  const int n_items1 = (L / chunk_x) * (L / ct::TY) * (L / ct::TZ);
+  int tiles = engine == kEngineTensorBinMajor ? contract_tiles(std::max(nb2, nb3), n_items1, L, ctas_per_sm, nsm) : 1;
+  const int nbl = kBinStride / tiles;
+  if (tiles > 1 && (size_t)(2 * nbl * nbl) * n_items1 > w.n_item_values) tiles = 1;  // a short chunk_x: more items
+  const void* fn = engine == kEngineSimt     ? (const void*)mp_contract_kernel
+                   : engine == kEngineTensor ? (const void*)mp_contract_tc_kernel<false, 1>
+                   : tiles == 1              ? (const void*)mp_contract_tc_kernel<true, 1>
+                   : tiles == 2              ? (const void*)mp_contract_tc_kernel<true, 2>
+                   : tiles == 4              ? (const void*)mp_contract_tc_kernel<true, 4>
+                                             : (const void*)mp_contract_tc_kernel<true, 8>;
+  const size_t smem = engine == kEngineSimt ? ct::kSmem
+                      : tiles == 1          ? tcc::kSmem<1>
+                      : tiles == 2          ? tcc::kSmem<2>
+                      : tiles == 4          ? tcc::kSmem<4>
+                                            : tcc::kSmem<8>;
+  const int variant = engine == kEngineTensorBinMajor ? 2 + (tiles == 1 ? 0 : tiles == 2 ? 1 : tiles == 4 ? 2 : 3)
+                                                      : (engine == kEngineSimt ? 1 : 0);
+  static bool smem_set[6][64] = {{false}};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !smem_set[engine][dev]) {  // once per device, before any stream capture
-    if (engine == kEngineTensor)
-      HERMES_CUDA_TRY(cudaFuncSetAttribute(mp_contract_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)tcc::kSmem));
-    else if (engine == kEngineTensorBinMajor)
-      HERMES_CUDA_TRY(cudaFuncSetAttribute(mp_contract_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)tcc::kSmem));
-    else
-      HERMES_CUDA_TRY(cudaFuncSetAttribute(mp_contract_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)ct::kSmem));
-    if (dev >= 0 && dev < 64) smem_set[engine][dev] = true;
+  if (dev < 0 || dev >= 64 || !smem_set[variant][dev]) {  // once per device, before any stream capture
+    HERMES_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (dev >= 0 && dev < 64) smem_set[variant][dev] = true;
   }
   // field layout follows hermes_multipole_fields: [cell][16] for nb > 1, [cell] for nb == 1
   ContractArgs A;
@@ -1868,31 +2034,35 @@ static int mp_contract_launch(const float* eps1, const void* fields2, int nb2, c
   A.gm = make_gamma(gamma);
   A.partial = w.partial;
   A.status = w.status;
-  const int n_items = (L / A.CX) * (L / ct::TY) * (L / ct::TZ);
-  int nblk = ctas_per_sm * sm_count();
-  if (nblk > n_items) nblk = n_items;
-  if (nblk > 1024) nblk = 1024;
+  A.items = w.items;
+  A.n_items1 = n_items1;
+  // blocks of one-tile items; several tiles run in fewer blocks and are added in this order
+  int nblk1 = ctas_per_sm * nsm;
+  if (nblk1 > n_items1) nblk1 = n_items1;
+  if (nblk1 > 1024) nblk1 = 1024;
+  const int nblk = tiles == 1 ? nblk1 : std::min(nsm, n_items1 / tiles);
   if (engine == kEngineTensor || engine == kEngineTensorBinMajor) {
     CUtensorMap map;
     memset(&map, 0, sizeof(map));
     if (engine == kEngineTensorBinMajor) {
-      rc = make_a2_map_bm(fields2, L, nb2, &map);
+      rc = make_a2_map_bm(fields2, L, nb2, kBinStride / tiles, &map);
       if (rc) return rc;
     } else if (A.s2 == kBinStride) {
       rc = make_a2_map(fields2, L, &map);
       if (rc) return rc;
     }
     HERMES_CUDA_TRY(cudaMemsetAsync(w.status, 0, sizeof(int), s));
-    if (engine == kEngineTensorBinMajor)
-      mp_contract_tc_kernel<true><<<nblk, ct::kThreads, tcc::kSmem, s>>>(A, map);
-    else
-      mp_contract_tc_kernel<false><<<nblk, ct::kThreads, tcc::kSmem, s>>>(A, map);
+    void* args[] = {&A, &map};
+    HERMES_CUDA_TRY(cudaLaunchKernel(fn, dim3(nblk), dim3(tiles > 1 ? 512 : ct::kThreads), args, smem, s));
     HERMES_LAUNCH_CHECK("mp_contract_tc_kernel");
   } else {
     mp_contract_kernel<<<nblk, ct::kThreads, ct::kSmem, s>>>(A);
     HERMES_LAUNCH_CHECK("mp_contract_kernel");
   }
-  mp_reduce_kernel<<<kMaxBins * kMaxBins * 2, 256, 0, s>>>(w.partial, nblk, kMaxBins * kMaxBins * 2, dout, scale);
+  if (tiles > 1)
+    mp_reduce_items_kernel<<<kMaxBins * kMaxBins * 2, 256, 0, s>>>(w.items, n_items1, nbl, nblk1, w.status, dout, scale);
+  else
+    mp_reduce_kernel<<<kMaxBins * kMaxBins * 2, 256, 0, s>>>(w.partial, nblk, kMaxBins * kMaxBins * 2, dout, scale);
   HERMES_LAUNCH_CHECK("mp_reduce_kernel");
   return HERMES_OK;
 }
