@@ -1,21 +1,31 @@
-// Inverse 512-point FFTs along the strided axes of complex64 fields
-// [nf][512][512][512] (x, y, z; z contiguous), in place, unnormalised
-// (a[k] <- sum_n a[n] e^{+2 pi i n k / 512}, cuFFT's CUFFT_INVERSE).
+// 512-point FFTs along the strided axes of complex64 fields [nf][512][512][..]
+// (x, y, z; z contiguous), in place, unnormalised: full fields of 512 columns
+// (the multipole fields) and half spectra of 257 columns of a real field.
 //
-// The multipole fields' inverse 3-D transform (15 fields of 512^3 at J=9)
-// spends two thirds of its time in cuFFT's two strided passes, which move
-// their 30 GB each at about half of HBM bandwidth.  Here a CTA owns 16
-// adjacent z columns of one (field, other-axis) slab and the 512 elements
-// of the transformed axis: every row it reads or writes is 128 contiguous
-// bytes, each element is read and written once, and the transform runs in
-// shared memory as three radix-8 stages
+// cuFFT's strided passes move their bytes at about half of HBM bandwidth.
+// Here a CTA owns 16 adjacent z columns of one (field, other-axis) slab and
+// the 512 elements of the transformed axis: every row it reads or writes is
+// 128 contiguous bytes, each element is read and written once, and the
+// transform runs in shared memory as three radix-8 stages
 // (512 = 8 * 8 * 8; n = n1 + 64 n2, k = k2 + 8 k1 with the 64-point part
-// split the same way), twiddles from a float64 table per CTA.
+// split the same way), twiddles from a float64 table per CTA.  Column 256 of a
+// half spectrum is one column wide: 16 slabs share a tile.
+//
+// Measured: 5.0 / 5.1 ms per y / x pass of 15 full fields (30 GB, 6.2 TB/s;
+// cuFFT 7.7 ms), 0.215 ms per y pass of a half spectrum (1.08 GB, 5 TB/s; cuFFT
+// 0.254 ms), 0.35 ms for the fused x pass (three passes took 1.04 ms).
+//
+// The last pass of a convolution's forward transform, the window and the
+// first pass of its inverse are one pass (kFused): a thread's eight outputs of
+// the forward transform, x[n1 + 64 n2], n2 = 0..7, are its eight inputs of
+// the inverse one.
+#include "fft_lines.cuh"
 #include "hermes_common.cuh"
 
 namespace hermes {
 namespace {
 
+enum { kInverse = 0, kForward = 1, kFused = 2 };
 constexpr int kLen = 512;
 constexpr int kPitch = kLen + 1;  // float2 per column in shared memory (odd: conflict-free columns)
 
@@ -55,6 +65,10 @@ __device__ __forceinline__ void cp_async16_cg(void* dst, const void* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait_group() {
@@ -75,34 +89,127 @@ __device__ __forceinline__ void cp_async_wait_group() {
 //   stage 1 (c, n1):      x[n1 + 64 n2], n2 = 0..7 -> Y[n1][k2] e^{2 pi i n1 k2 / 512}
 //   stage 2 (c, k2, m1):  Y[m1 + 8 m2][k2], m2 = 0..7 -> W[k2][m1][q2] e^{2 pi i m1 q2 / 64}
 //   stage 3 (c, k2, q2):  W[k2][m1][q2], m1 = 0..7 -> X[k2 + 8 q2 + 64 q1]
+// The forward transform is the inverse one on exchanged parts:
+// F(a) = swap(I(swap(a))), swap(re, im) = (im, re).
 constexpr int kCols = 16, kThreads = 512, kR = kCols * kLen / 8 / kThreads;
+constexpr int kBuf = kCols * kPitch;
+
+__device__ __forceinline__ float2 swapped(float2 a) { return make_float2(a.y, a.x); }
+
+// From registers x[n1 + 64 n2] (task (c, n1)) to the inputs of the last eight
+// point transforms (task (c, k2 + 8 q2), which idft8 turns into
+// X[k2 + 8 q2 + 64 q1]) through the tile buffer, whose other readers are past
+// the barrier at entry.  The caller's next barrier frees the buffer; the last
+// transforms come after it, so that they overlap the stores of other warps.
+__device__ __forceinline__ void fft512_registers(float2 (&v)[kR][8], float2* buf, const float2* tw) {
+  constexpr int C = kCols, T = kThreads;
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kR; ++r) {
+    const int i = threadIdx.x + T * r, c = i % C, n1 = i / C;
+    idft8(v[r]);
+    float2* s = buf + c * kPitch + n1 * 8;
+    s[0] = v[r][0];
+#pragma unroll
+    for (int k2 = 1; k2 < 8; ++k2) s[k2] = cmul(v[r][k2], tw[n1 * k2]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kR; ++r) {
+    const int i = threadIdx.x + T * r, c = i % C, rest = i / C, k2 = rest & 7, m1 = rest >> 3;
+    const float2* s = buf + c * kPitch + m1 * 8 + k2;
+#pragma unroll
+    for (int m2 = 0; m2 < 8; ++m2) v[r][m2] = s[64 * m2];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kR; ++r) {
+    const int i = threadIdx.x + T * r, c = i % C, rest = i / C, k2 = rest & 7, m1 = rest >> 3;
+    idft8(v[r]);
+    float2* s = buf + c * kPitch + k2 * 64 + m1 * 8;
+    s[0] = v[r][0];
+#pragma unroll
+    for (int q2 = 1; q2 < 8; ++q2) s[q2] = cmul(v[r][q2], tw[8 * m1 * q2]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kR; ++r) {
+    const int i = threadIdx.x + T * r, c = i % C, rest = i / C, k2 = rest & 7, q2 = rest >> 3;
+    const float2* s = buf + c * kPitch + k2 * 64 + q2;
+#pragma unroll
+    for (int m1 = 0; m1 < 8; ++m1) v[r][m1] = s[8 * m1];
+  }
+}
+
+// kHalf: half spectra of 257 columns with rows of kHalfPitch values, else full
+// fields of 512 columns.
+template <int kMode, bool kHalf>
 __global__ void __launch_bounds__(kThreads, 1)
-fft512_cols_kernel(float2* __restrict__ data, int nf, int axis) {
-  constexpr int C = kCols, T = kThreads, R = kR, kBuf = C * kPitch;
+fft512_cols_kernel(float2* __restrict__ data, int nf, int axis, FftWindow win) {
+  constexpr int C = kCols, T = kThreads, R = kR;
+  constexpr int kRow = kHalf ? kFft512HalfPitch : kLen;
   extern __shared__ __align__(16) float2 sm[];
   float2* tw = sm + 3 * kBuf;
-  for (int j = threadIdx.x; j < kLen; j += T) {
-    double sn, cs;
-    sincospi((double)j / 256.0, &sn, &cs);
-    tw[j] = make_float2((float)cs, (float)sn);
+  float* G = reinterpret_cast<float*>(tw + kLen);  // gaussian window factors (kFused)
+  // e^{2 pi i j / 512}: the first octant in float64 (slow on this part: 512
+  // evaluations cost as much as two tiles), the others are its reflections
+  for (int j = threadIdx.x; j <= kLen / 8; j += T) {
+    double sd, cd;
+    sincospi((double)j / 256.0, &sd, &cd);
+    const float sn = (float)sd, cs = (float)cd;
+    const int q = kLen / 4;  // a quarter turn
+    tw[j] = make_float2(cs, sn);
+    tw[q - j] = make_float2(sn, cs);
+    tw[q + j] = make_float2(-sn, cs);
+    tw[2 * q - j] = make_float2(-cs, sn);
+    tw[2 * q + j] = make_float2(-cs, -sn);
+    tw[3 * q - j] = make_float2(-sn, -cs);
+    tw[3 * q + j] = make_float2(sn, -cs);
+    if (j > 0) tw[4 * q - j] = make_float2(cs, -sn);
   }
-  const long long L = kLen, L2 = L * L, L3 = L2 * L;
-  const long long astride = axis == 1 ? L2 : L;
-  const long long rstride = axis == 1 ? L : L2;
-  const long long ntiles = (long long)nf * L * (L / C);
+  if (kMode == kFused && win.axis_factor)
+    for (int j = threadIdx.x; j < kLen; j += T) G[j] = win.axis_factor[j];
+  const long long L = kLen, L2 = L * kRow, L3 = L2 * L;
+  const long long astride = axis == 1 ? L2 : kRow;
+  const long long rstride = axis == 1 ? kRow : L2;
+  // tiles of 16 columns per slab, then (kHalf) tiles of column 256 over 16 slabs
+  constexpr int kFull = (kHalf ? kLen / 2 : kLen) / C;
+  const long long nfull = (long long)nf * L * kFull, ntiles = nfull + (kHalf ? nf * (L / C) : 0);
+  // slab index, first column and column stride of tile t of a half spectrum
+  auto half_tile = [&](long long t, int& a, int& z, long long& cs) {
+    const bool tail = t >= nfull;
+    a = (int)(tail ? (t - nfull) * C : t / kFull);
+    z = tail ? kLen / 2 : (int)(t % kFull) * C;
+    cs = tail ? astride : 1;
+  };
   auto tile_ptr = [&](long long t) {
-    const int zb = (int)(t % (L / C));
-    const long long fa = t / (L / C);
-    return data + (fa / L) * L3 + (fa % L) * astride + (long long)zb * C;
+    if constexpr (kHalf) {
+      int a, z;
+      long long cs;
+      half_tile(t, a, z, cs);
+      return data + a * astride + z;
+    } else {
+      const int zb = (int)(t % kFull);
+      const long long fa = t / kFull;
+      return data + (fa / L) * L3 + (fa % L) * astride + (long long)zb * C;
+    }
   };
   // tile t -> buffer (row-major), 4096 16-byte pieces, 8 per 128-byte row
   auto prefetch = [&](long long t, float2* buf) {
     if (t < ntiles) {
       const float2* g = tile_ptr(t);
+      if (!kHalf || t < nfull) {
 #pragma unroll
-      for (int q = 0; q < 4096 / T; ++q) {
-        const int j = threadIdx.x + T * q, row = j >> 3, part = j & 7;
-        cp_async16_cg(buf + row * C + 2 * part, g + (long long)row * rstride + 2 * part);
+        for (int q = 0; q < 4096 / T; ++q) {
+          const int j = threadIdx.x + T * q, row = j >> 3, part = j & 7;
+          cp_async16_cg(buf + row * C + 2 * part, g + (long long)row * rstride + 2 * part);
+        }
+      } else {
+#pragma unroll 4
+        for (int q = 0; q < 8192 / T; ++q) {
+          const int j = threadIdx.x + T * q, row = j >> 4, c = j & 15;
+          cp_async8(buf + row * C + c, g + row * rstride + c * astride);
+        }
       }
     }
     cp_async_commit();  // an empty group past the end keeps the group count uniform
@@ -112,88 +219,111 @@ fft512_cols_kernel(float2* __restrict__ data, int nf, int axis) {
   prefetch(t + gridDim.x, sm + kBuf);
   for (int k = 0; t < ntiles; t += gridDim.x, ++k) {
     float2* buf = sm + (k % 3) * kBuf;
-    prefetch(t + 2LL * gridDim.x, sm + ((k + 2) % 3) * kBuf);
-    cp_async_wait_group<2>();  // this tile's group is complete (two newer may be in flight)
+    cp_async_wait_group<1>();  // this tile's group is complete (the next one may be in flight)
     __syncthreads();
     float2 v[R][8];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int i = threadIdx.x + T * r, c = i % C, n1 = i / C;
 #pragma unroll
-      for (int n2 = 0; n2 < 8; ++n2) v[r][n2] = buf[(n1 + 64 * n2) * C + c];
+      for (int n2 = 0; n2 < 8; ++n2) {
+        const float2 e = buf[(n1 + 64 * n2) * C + c];
+        v[r][n2] = kMode == kInverse ? e : swapped(e);
+      }
     }
-    __syncthreads();
+    prefetch(t + 2LL * gridDim.x, sm + ((k + 2) % 3) * kBuf);
+    fft512_registers(v, buf, tw);
+    if (kMode == kFused) {
+      int a, z;  // axis 0: the slab index a is y
+      long long cs;
+      half_tile(t, a, z, cs);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = threadIdx.x + T * r, c = i % C, n1 = i / C;
-      idft8(v[r]);
-      float2* s = buf + c * kPitch + n1 * 8;
-      s[0] = v[r][0];
+      for (int r = 0; r < R; ++r) {
+        const int i = threadIdx.x + T * r, c = i % C, k0 = i / C;  // k0 = k2 + 8 q2
+        const int y = a + (cs == 1 ? 0 : c), zc = z + (cs == 1 ? c : 0);
+        const int yq = min(y, kLen - y);
+        idft8(v[r]);
 #pragma unroll
-      for (int k2 = 1; k2 < 8; ++k2) s[k2] = cmul(v[r][k2], tw[n1 * k2]);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = threadIdx.x + T * r, c = i % C, rest = i / C, k2 = rest & 7, m1 = rest >> 3;
-      const float2* s = buf + c * kPitch + m1 * 8 + k2;
-#pragma unroll
-      for (int m2 = 0; m2 < 8; ++m2) v[r][m2] = s[64 * m2];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = threadIdx.x + T * r, c = i % C, rest = i / C, k2 = rest & 7, m1 = rest >> 3;
-      idft8(v[r]);
-      float2* s = buf + c * kPitch + k2 * 64 + m1 * 8;
-      s[0] = v[r][0];
-#pragma unroll
-      for (int q2 = 1; q2 < 8; ++q2) s[q2] = cmul(v[r][q2], tw[8 * m1 * q2]);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = threadIdx.x + T * r, c = i % C, rest = i / C, k2 = rest & 7, q2 = rest >> 3;
-      const float2* s = buf + c * kPitch + k2 * 64 + q2;
-#pragma unroll
-      for (int m1 = 0; m1 < 8; ++m1) v[r][m1] = s[8 * m1];
+        for (int q1 = 0; q1 < 8; ++q1) {
+          const int kx = k0 + 64 * q1;
+          float K;
+          if (win.axis_factor) {
+            K = G[kx] * G[y] * G[zc] * win.scale;
+          } else {
+            const int xq = min(kx, kLen - kx), hi = max(xq, yq), lo = min(xq, yq);
+            K = __ldg(win.folded + (long long)(hi * (hi + 1) / 2 + lo) * (kLen / 2 + 1) + zc);
+          }
+          if (win.zero_k0 && kx == 0 && y == 0 && zc == 0) K = 0.f;
+          const float2 e = swapped(v[r][q1]);
+          v[r][q1] = make_float2(e.x * K * win.factor, e.y * K * win.factor);
+        }
+      }
+      fft512_registers(v, buf, tw);
     }
     __syncthreads();  // buffer free: the next iteration prefetches into it
     float2* g = tile_ptr(t);
+    [[maybe_unused]] const long long cs = kHalf && t >= nfull ? astride : 1;
+    auto store = [&](int r, int q1) {
+      const int i = threadIdx.x + T * r, c = i % C, k0 = i / C;
+      g[(long long)(k0 + 64 * q1) * rstride + (kHalf ? c * cs : c)] = kMode == kForward ? swapped(v[r][q1]) : v[r][q1];
+    };
+    // The order of the row stores decides the x pass (rows 2 MB apart): both
+    // transforms' rows of one q1 together 5.1 ms for 15 fields, one
+    // transform's eight rows after the other's 6.0 ms; the fused pass is
+    // 3% better the other way round.
+    if (kMode == kFused) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = threadIdx.x + T * r, c = i % C, rest = i / C, k2 = rest & 7, q2 = rest >> 3;
-      idft8(v[r]);
-      float2* gp = g + (long long)(k2 + 8 * q2) * rstride + c;
+      for (int r = 0; r < R; ++r) {
+        idft8(v[r]);
 #pragma unroll
-      for (int q1 = 0; q1 < 8; ++q1) gp[(long long)(64 * q1) * rstride] = v[r][q1];
+        for (int q1 = 0; q1 < 8; ++q1) store(r, q1);
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) idft8(v[r]);
+#pragma unroll
+      for (int q1 = 0; q1 < 8; ++q1)
+#pragma unroll
+        for (int r = 0; r < R; ++r) store(r, q1);
     }
   }
   cp_async_wait_group<0>();  // no copy outlives the kernel
 }
 
-}  // namespace
-
-// axis 0: x (element stride 512^2), axis 1: y (stride 512).
-int fft512_strided_inverse(float2* data, int nf, int axis, cudaStream_t s) {
-  constexpr size_t smem = sizeof(float2) * (3 * kCols * (size_t)kPitch + kLen);
+template <int kMode, bool kHalf>
+int launch_cols(float2* data, int nf, int axis, const FftWindow& win, cudaStream_t s) {
+  constexpr size_t smem = sizeof(float2) * (3 * (size_t)kBuf + kLen) + (kMode == kFused ? sizeof(float) * kLen : 0);
   static bool attr_set[64] = {false};
   int dev = 0;
   HERMES_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64 || !attr_set[dev]) {  // once per device, before any stream capture
-    HERMES_CUDA_TRY(cudaFuncSetAttribute(fft512_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HERMES_CUDA_TRY(cudaFuncSetAttribute(fft512_cols_kernel<kMode, kHalf>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem));
     if (dev >= 0 && dev < 64) attr_set[dev] = true;
   }
   int nsm = 0;
   HERMES_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const long long ntiles = (long long)nf * kLen * (kLen / kCols);
-  long long grid = nsm;
-  if (grid > ntiles) grid = ntiles;
-  fft512_cols_kernel<<<(int)grid, kThreads, smem, s>>>(data, nf, axis);
+  // one block per SM: every shape has more tiles (8224 at least) than SMs
+  fft512_cols_kernel<kMode, kHalf><<<nsm, kThreads, smem, s>>>(data, nf, axis, win);
   HERMES_LAUNCH_CHECK("fft512_cols_kernel");
   return HERMES_OK;
 }
 
+}  // namespace
+
+// axis 0: x, axis 1: y.
+int fft512_strided_inverse(float2* data, int nf, int axis, cudaStream_t s) {
+  return launch_cols<kInverse, false>(data, nf, axis, FftWindow{}, s);
+}
+
+int fft512_half_y(float2* data, bool forward, cudaStream_t s) {
+  return forward ? launch_cols<kForward, true>(data, 1, 1, FftWindow{}, s)
+                 : launch_cols<kInverse, true>(data, 1, 1, FftWindow{}, s);
+}
+
+int fft512_half_x_window_x(float2* data, const FftWindow& win, cudaStream_t s) {
+  return launch_cols<kFused, true>(data, 1, 0, win, s);
+}
 
 }  // namespace hermes
 

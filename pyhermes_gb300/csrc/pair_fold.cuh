@@ -198,7 +198,7 @@ pp_radial_bins_kernel(const WinDev* __restrict__ wins, int n_bins, int L, const 
     for (int b = 0; b < kRadialBins; ++b) {
       if (b < nb) {
         bool ok;
-        const double w = (double)window_iso_n2(wins[b0 + b], n2, &ok).x;
+        const double w = (double)window_radial_n2(wins[b0 + b], n2, &ok);
 #pragma unroll
         for (int p = 0; p < NP; ++p) acc[b][p] = fma(w, h[p], acc[b][p]);
       }

@@ -18,13 +18,14 @@
 
 #include "hermes_common.cuh"
 #include "window_eval.cuh"
+#include "fft_lines.cuh"
 #include "pair_fold.cuh"
 #include "pair_products.cuh"
 
 namespace hermes {
 
 // ---- cuFFT plan cache ----------------------------------------------------
-enum PlanKind { kR2C = 0, kC2R = 1, kC2C = 2, kC2CLines = 3 };
+enum PlanKind { kR2C = 0, kC2R = 1, kC2C = 2, kC2CLines = 3, kR2CLines = 4, kC2RLines = 5 };
 
 static std::mutex g_plan_mu;
 static std::map<std::tuple<int, int, int, int>, cufftHandle> g_plans;
@@ -45,6 +46,16 @@ int get_plan(int J, PlanKind kind, int batch, cufftHandle* out) {
     int n1[1] = {L};
     cufftResult r = cufftPlanMany(&h, 1, n1, nullptr, 1, L, nullptr, 1, L, CUFFT_C2C, batch * L * L);
     if (r != CUFFT_SUCCESS) return fail(HERMES_ERR_CUFFT, "cufftPlanMany(lines, J=%d, batch=%d) failed: %d", J, batch, (int)r);
+    g_plans[key] = h;
+    *out = h;
+    return HERMES_OK;
+  }
+  if (kind == kR2CLines || kind == kC2RLines) {  // the L^2 real z lines against rows of `batch` complex values
+    int n1[1] = {L}, real[1] = {L}, cplx[1] = {batch};
+    const bool fwd = kind == kR2CLines;
+    cufftResult r = cufftPlanMany(&h, 1, n1, fwd ? real : cplx, 1, fwd ? L : batch, fwd ? cplx : real, 1, fwd ? batch : L,
+                                  fwd ? CUFFT_R2C : CUFFT_C2R, L * L);
+    if (r != CUFFT_SUCCESS) return fail(HERMES_ERR_CUFFT, "cufftPlanMany(real lines, J=%d, pitch=%d) failed: %d", J, batch, (int)r);
     g_plans[key] = h;
     *out = h;
     return HERMES_OK;
@@ -176,32 +187,13 @@ __global__ void phi_power_to_f32(const double* __restrict__ p, int n, float* __r
   if (i < n) out[i] = (float)p[i];
 }
 
-// spec[k] *= K(k) * factor on the half spectrum [L][L][L/2+1].  The gaussian
-// exp(-q^2/2) factors over the axes, so its image sum is G(x) G(y) G(z) with
-// G(i) = sum over the axis images u of P(|u|) exp(-(2 pi u R / L)^2 / 2),
-// tabulated per block in shared memory (the other windows are evaluated per
-// mode by kernel_value).
+// spec[k] *= K(k) * factor on the half spectrum [L][L][L/2+1], the kernel
+// evaluated per mode (windows without a folded form).
 __global__ void spec_apply_window_kernel(float2* __restrict__ spec, WinDev w, int L,
                                          const double* __restrict__ pd, int np, int bw, float factor) {
   extern __shared__ float P[];
-  float* G = P + np;  // [L], gaussian only
   for (int i = threadIdx.x; i < np; i += blockDim.x) P[i] = (float)pd[i];
   __syncthreads();
-  const bool sep = w.type == HERMES_WIN_GAUSSIAN;
-  if (sep) {
-    for (int i = threadIdx.x; i < L; i += blockDim.x) {
-      float g = 0.f;
-      for (int kk = 0; kk < bw; ++kk) {
-        const int u1 = kk * L + i, u2 = kk * L + (L - i);
-        const float q1 = kTwoPi * ((float)u1 * w.rho_hi[0] + (float)u1 * w.rho_lo[0]);
-        const float q2 = kTwoPi * ((float)u2 * w.rho_hi[0] + (float)u2 * w.rho_lo[0]);
-        g = fmaf(P[u1], expf(-0.5f * q1 * q1), g);
-        g = fmaf(P[u2], expf(-0.5f * q2 * q2), g);
-      }
-      G[i] = g;
-    }
-    __syncthreads();
-  }
   const int H = L / 2 + 1;
   const long long total = (long long)L * L * H;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -209,15 +201,136 @@ __global__ void spec_apply_window_kernel(float2* __restrict__ spec, WinDev w, in
     const int z = (int)(m % H);
     const long long r = m / H;
     const int y = (int)(r % L), x = (int)(r / L);
-    float2 K;
-    if (sep) {
-      K = make_float2(G[x] * G[y] * G[z] * w.scale, 0.f);
-      if (w.zero_k0 && m == 0) K.x = 0.f;
-    } else {
-      K = kernel_value(w, x, y, z, L, P, bw);
-    }
+    const float2 K = kernel_value(w, x, y, z, L, P, bw);
     const float2 s = spec[m];
     spec[m] = make_float2((s.x * K.x - s.y * K.y) * factor, (s.x * K.y + s.y * K.x) * factor);
+  }
+}
+
+// Windows whose kernel is the same on the up to eight columns (+-x, +-y),
+// (+-y, +-x) (see pair_fold.cuh) are applied from small tables:
+//   kFoldAxes   gaussian: exp(-q^2/2) factors over the axes, so the image sum
+//               is G(x) G(y) G(z), G(i) = sum over the axis images u of
+//               P(|u|) exp(-(2 pi u R / L)^2 / 2)            (table: G[L])
+//   kFoldRadial a function of n2 = |k L|^2, bandwidth 1: eight reads of
+//               W[n2] per folded mode                        (W[3 L^2 + 1])
+//   kFoldCyl    cylindrical with the line of sight on z: A(x, y) B(z)
+//                                       (A[folded columns], then B[L/2+1])
+// The pass is then bound by the spectrum's bytes: sphere at J = 8 0.038 ms,
+// 0.450 ms with eight evaluations per mode; gaussian at J = 9 0.536 ms before,
+// part of the fused x pass now.
+enum FoldKind { kFoldNone = 0, kFoldAxes, kFoldRadial, kFoldCyl };
+
+FoldKind fold_kind(const WinDev& w, int bw) {
+  if (w.mode == HERMES_KMODE_COMPLEX_RFFT && !window_is_radial(w.type)) return kFoldNone;
+  if (w.type == HERMES_WIN_GAUSSIAN) return kFoldAxes;
+  if (window_is_radial(w.type)) return bw == 1 ? kFoldRadial : kFoldNone;
+  const bool cyl = w.type == HERMES_WIN_RING || w.type == HERMES_WIN_DISK || w.type == HERMES_WIN_CYLSHELL ||
+                   w.type == HERMES_WIN_CYLINDER;
+  return cyl && w.los_axis == 2 ? kFoldCyl : kFoldNone;
+}
+
+// floats of the largest table at any kind
+size_t fold_table_floats(int L) { return 3 * (size_t)L * L + 1 + L; }
+
+template <int kKind>
+__global__ void fold_table_kernel(WinDev w, int L, const double* __restrict__ pd, int bw, int n, float* __restrict__ tab) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float v = 0.f;
+  if (kKind == kFoldRadial) {
+    bool ok;
+    v = window_radial_n2(w, i, &ok);
+  } else if (kKind == kFoldAxes) {
+    for (int kk = 0; kk < bw; ++kk) {
+      const int u1 = kk * L + i, u2 = kk * L + (L - i);
+      const float q1 = kTwoPi * ((float)u1 * w.rho_hi[0] + (float)u1 * w.rho_lo[0]);
+      const float q2 = kTwoPi * ((float)u2 * w.rho_hi[0] + (float)u2 * w.rho_lo[0]);
+      v = fmaf((float)pd[u1], expf(-0.5f * q1 * q1), v);
+      v = fmaf((float)pd[u2], expf(-0.5f * q2 * q2), v);
+    }
+  } else {
+    const int ncol = (int)fold_columns(L);
+    if (i < ncol) {
+      int x, y;
+      fold_xy(i, x, y);
+      for (int t = 0; t < 4 * bw * bw; ++t) {
+        const int pair = t >> 2, ii = pair / bw, jj = pair - ii * bw;
+        const int pu = ii * L + ((t & 1) ? L - x : x), qu = jj * L + ((t & 2) ? L - y : y);
+        v = fmaf((float)pd[pu] * (float)pd[qu], cyl_perp(w, pu, qu), v);
+      }
+    } else {
+      const int z = i - ncol, sgn = w.mode == HERMES_KMODE_OCTANT ? 1 : -1;
+      for (int kk = 0; kk < bw; ++kk) {
+        const int cp = kk * L + z, cn = kk * L + (L - z);
+        v = fmaf((float)pd[cp], cyl_par(w, cp), v);
+        v = fmaf((float)pd[cn], cyl_par(w, sgn * cn), v);
+      }
+    }
+  }
+  tab[i] = v;
+}
+
+// Kernel value of folded column c = (x, y) at z, without scale.
+template <int kKind>
+__device__ __forceinline__ float folded_value(const float* __restrict__ tab, const float* P, int L, int ncol, int c, int x,
+                                              int y, int z) {
+  if (kKind == kFoldAxes) return __ldg(tab + x) * __ldg(tab + y) * __ldg(tab + z);
+  if (kKind == kFoldCyl) return __ldg(tab + c) * __ldg(tab + ncol + z);
+  const int ax[2] = {x, L - x}, ay[2] = {y, L - y}, az[2] = {z, L - z};
+  float re = 0.f;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float pab = P[ax[i]] * P[ay[j]];
+      const int s = ax[i] * ax[i] + ay[j] * ay[j];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) re = fmaf(pab * P[az[k]], __ldg(tab + s + az[k] * az[k]), re);
+    }
+  return re;
+}
+
+// One warp per folded column: spec *= K factor on the column's rows
+// (kStore: K itself into folded[column][L/2+1] instead, for the fused pass).
+template <int kKind, bool kStore>
+__global__ void __launch_bounds__(kHistThreads)
+folded_window_kernel(float2* __restrict__ spec, float* __restrict__ folded, const float* __restrict__ tab, int L,
+                     const double* __restrict__ pd, float scale, int zero_k0, float factor) {
+  extern __shared__ float P[];
+  if (kKind == kFoldRadial) {
+    for (int i = threadIdx.x; i <= L; i += kHistThreads) P[i] = (float)pd[i];
+    __syncthreads();
+  }
+  const int H = L / 2 + 1, Lm = L - 1, ncol = (int)fold_columns(L);
+  const int lane = threadIdx.x & 31, nw = gridDim.x * (kHistThreads / 32);
+  for (int c = blockIdx.x * (kHistThreads / 32) + (threadIdx.x >> 5); c < ncol; c += nw) {
+    int x, y;
+    fold_xy(c, x, y);
+    const bool rx = x != 0 && 2 * x != L, ry = y != 0 && 2 * y != L, sw = x != y;
+    const int xs[2] = {x, (L - x) & Lm}, ys[2] = {y, (L - y) & Lm};
+    for (int z = lane; z < H; z += 32) {
+      float K = folded_value<kKind>(tab, P, L, ncol, c, x, y, z) * scale;
+      if (zero_k0 && c == 0 && z == 0) K = 0.f;
+      if (kStore) {
+        folded[(size_t)c * H + z] = K;
+        continue;
+      }
+      float2 v[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const int i = r & 1, j = (r >> 1) & 1, s = r >> 2;
+        if ((i && !rx) || (j && !ry) || (s && !sw)) continue;
+        v[r] = spec[(s ? (long long)ys[j] * L + xs[i] : (long long)xs[i] * L + ys[j]) * H + z];
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const int i = r & 1, j = (r >> 1) & 1, s = r >> 2;
+        if ((i && !rx) || (j && !ry) || (s && !sw)) continue;
+        spec[(s ? (long long)ys[j] * L + xs[i] : (long long)xs[i] * L + ys[j]) * H + z] =
+            make_float2(v[r].x * K * factor, v[r].y * K * factor);
+      }
+    }
   }
 }
 
@@ -285,6 +398,20 @@ int check_power(int J, int bw) {
 
 using namespace hermes;
 
+// The z lines of a real 512^3 field against rows of kFft512HalfPitch complex
+// values (cuFFT's contiguous 1-D transforms), either way.
+static int real_lines(const float* field, float2* spec, float* out, cudaStream_t s) {
+  cufftHandle h;
+  int rc = get_plan(9, field ? kR2CLines : kC2RLines, kFft512HalfPitch, &h);
+  if (rc) return rc;
+  HERMES_CUFFT_TRY(cufftSetStream(h, s));
+  if (field)
+    HERMES_CUFFT_TRY(cufftExecR2C(h, const_cast<cufftReal*>(field), reinterpret_cast<cufftComplex*>(spec)));
+  else
+    HERMES_CUFFT_TRY(cufftExecC2R(h, reinterpret_cast<cufftComplex*>(spec), out));
+  return HERMES_OK;
+}
+
 extern "C" int hermes_fft_r2c(const float* field, void* spec, int J, void* stream) {
   if (J < 2 || J > 10) return fail(HERMES_ERR_INVALID, "fft: J=%d outside [2,10]", J);
   cufftHandle h;
@@ -305,11 +432,50 @@ extern "C" int hermes_fft_c2r(void* spec, float* field, int J, void* stream) {
   return HERMES_OK;
 }
 
+namespace {
+// The one workspace layout of hermes_window_apply.
+struct WindowWs {
+  float2* spec;   // half spectrum, rows of kFft512HalfPitch values at J = 9, L/2+1 else
+  float* tab;     // fold_table_floats
+  float* folded;  // J = 9: K of every folded mode
+  size_t used;
+};
+WindowWs window_carve(void* p, size_t cap, int J) {
+  const size_t L = (size_t)1 << J, H = L / 2 + 1;
+  Carver c(p, cap);
+  WindowWs w;
+  w.spec = c.take<float2>(L * L * (J == 9 ? (size_t)kFft512HalfPitch : H));
+  w.tab = c.take<float>(fold_table_floats((int)L));
+  w.folded = J == 9 ? c.take<float>((size_t)fold_columns((int)L) * H) : nullptr;
+  w.used = c.used;
+  return w;
+}
+}  // namespace
+
 extern "C" int hermes_window_workspace_size(int J, size_t* bytes) {
   if (!bytes) return fail(HERMES_ERR_INVALID, "bytes is NULL");
   if (J < 2 || J > 10) return fail(HERMES_ERR_INVALID, "J=%d outside [2,10]", J);
-  const size_t L = (size_t)1 << J;
-  *bytes = L * L * (L / 2 + 1) * sizeof(float2);
+  *bytes = window_carve(nullptr, 0, J).used;
+  return HERMES_OK;
+}
+
+template <int kKind>
+static int launch_folded(const WinDev& w, const WindowWs& ws, int J, const double* phi_power, int bw, float factor,
+                         bool fused, cudaStream_t s) {
+  const int L = 1 << J;
+  const int n = kKind == kFoldRadial ? 3 * L * L + 1 : (kKind == kFoldAxes ? L : (int)fold_columns(L) + L / 2 + 1);
+  fold_table_kernel<kKind><<<(n + 255) / 256, 256, 0, s>>>(w, L, phi_power, bw, n, ws.tab);
+  HERMES_LAUNCH_CHECK("fold_table_kernel");
+  if (fused && kKind == kFoldAxes) return HERMES_OK;  // the fused pass reads the factors
+  const int grid = grid_for(fold_columns(L) * 32, kHistThreads);
+  const size_t psm = sizeof(float) * (size_t)(L + 1);
+  if (fused)
+    folded_window_kernel<kKind, true><<<grid, kHistThreads, psm, s>>>(nullptr, ws.folded, ws.tab, L, phi_power, w.scale,
+                                                                      w.zero_k0, factor);
+  else
+    folded_window_kernel<kKind, false><<<grid, kHistThreads, psm, s>>>(ws.spec, nullptr, ws.tab, L, phi_power, w.scale,
+                                                                       w.zero_k0, factor);
+  HERMES_LAUNCH_CHECK("folded_window_kernel");
   return HERMES_OK;
 }
 
@@ -327,16 +493,36 @@ extern "C" int hermes_window_apply(const float* eps, float* out, int J, const he
   WinDev w;
   rc = prepare_window(*win, L, &w);
   if (rc) return rc;
-  float2* spec = static_cast<float2*>(workspace);
-  rc = hermes_fft_r2c(eps, spec, J, stream);
-  if (rc) return rc;
-  const int np = L * bandwidth + 1;
-  const long long total = (long long)L * L * (L / 2 + 1);
+  const WindowWs ws = window_carve(workspace, workspace_bytes, J);
+  cudaStream_t s = as_stream(stream);
+  const FoldKind kind = fold_kind(w, bandwidth);
   const float factor = (float)(1.0 / ((double)L * L * L));
-  spec_apply_window_kernel<<<grid_for(total, 256), 256, (np + L) * sizeof(float), as_stream(stream)>>>(
-      spec, w, L, phi_power, np, bandwidth, factor);
-  HERMES_LAUNCH_CHECK("spec_apply_window_kernel");
-  return hermes_fft_c2r(spec, out, J, stream);
+  const bool fused = J == 9 && kind != kFoldNone && (reinterpret_cast<uintptr_t>(ws.spec) & 15u) == 0;
+  if (!fused) {
+    rc = hermes_fft_r2c(eps, ws.spec, J, stream);
+    if (rc) return rc;
+  }
+  switch (kind) {
+    case kFoldAxes: rc = launch_folded<kFoldAxes>(w, ws, J, phi_power, bandwidth, factor, fused, s); break;
+    case kFoldRadial: rc = launch_folded<kFoldRadial>(w, ws, J, phi_power, bandwidth, factor, fused, s); break;
+    case kFoldCyl: rc = launch_folded<kFoldCyl>(w, ws, J, phi_power, bandwidth, factor, fused, s); break;
+    default: {
+      const int np = L * bandwidth + 1;
+      const long long total = (long long)L * L * (L / 2 + 1);
+      spec_apply_window_kernel<<<grid_for(total, 256), 256, np * sizeof(float), s>>>(ws.spec, w, L, phi_power, np,
+                                                                                    bandwidth, factor);
+      HERMES_LAUNCH_CHECK("spec_apply_window_kernel");
+    }
+  }
+  if (rc) return rc;
+  if (!fused) return hermes_fft_c2r(ws.spec, out, J, stream);
+  // J = 9: z lines, y, then x, the window and x back in one pass, y, z lines
+  const FftWindow fw = {kind == kFoldAxes ? ws.tab : nullptr, ws.folded, w.scale, factor, w.zero_k0};
+  rc = real_lines(eps, ws.spec, nullptr, s);
+  if (!rc) rc = fft512_half_y(ws.spec, true, s);
+  if (!rc) rc = fft512_half_x_window_x(ws.spec, fw, s);
+  if (!rc) rc = fft512_half_y(ws.spec, false, s);
+  return rc ? rc : real_lines(nullptr, ws.spec, out, s);
 }
 
 extern "C" int hermes_window_materialize(const hermes_window_t* win, const double* phi_power, int bandwidth,
@@ -578,14 +764,11 @@ static size_t cylz_smem(int np, int L, int n_pairs) {
 // Bins padded to whole groups of kCylBins (the A table's row stride).
 static int cylz_nbp(int n_bins) { return (n_bins + kCylBins - 1) / kCylBins * kCylBins; }
 
-// True when every bin is an isotropic window (a function of |k|^2 alone)
-// whose kernel keeps its k = 0 value, or the k = 0 mode is left out.
+// True when every bin is a function of |k|^2 alone whose kernel keeps its
+// k = 0 value, or the k = 0 mode is left out.
 static bool all_radial(const std::vector<WinDev>& hw, bool exclude_k0) {
-  for (const WinDev& w : hw) {
-    const bool iso = w.type == HERMES_WIN_SPHERE || w.type == HERMES_WIN_GAUSSIAN || w.type == HERMES_WIN_SHELL ||
-                     w.type == HERMES_WIN_THICK_SHELL || w.type == HERMES_WIN_GAUSSIAN_SHELL;
-    if (!iso || (w.zero_k0 && !exclude_k0)) return false;
-  }
+  for (const WinDev& w : hw)
+    if (!window_is_radial(w.type) || (w.zero_k0 && !exclude_k0)) return false;
   return !hw.empty();
 }
 

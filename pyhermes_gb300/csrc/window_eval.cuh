@@ -197,16 +197,55 @@ __device__ __forceinline__ float2 window_iso_n2(const WinDev& w, int n2, bool* o
   }
 }
 
+// Every window that is a function of n2 alone: the ones of window_iso_n2, the
+// wavelets and the Laplacians.
+__host__ __device__ __forceinline__ bool window_is_radial(int type) {
+  return type == HERMES_WIN_SPHERE || type == HERMES_WIN_GAUSSIAN || type == HERMES_WIN_SHELL ||
+         type == HERMES_WIN_THICK_SHELL || type == HERMES_WIN_GAUSSIAN_SHELL || type == HERMES_WIN_CW ||
+         type == HERMES_WIN_CWS || type == HERMES_WIN_GDW || type == HERMES_WIN_LAPLACIAN ||
+         type == HERMES_WIN_INVERSE_LAPLACIAN;
+}
+__device__ __forceinline__ float window_radial_n2(const WinDev& w, int n2, bool* ok) {
+  const float v = window_iso_n2(w, n2, ok).x;
+  if (*ok) return v;
+  *ok = true;
+  float nh, nl;
+  switch (w.type) {
+    case HERMES_WIN_CW:
+    case HERMES_WIN_CWS: {
+      df_sqrt_int(n2, nh, nl);
+      float q = kTwoPi * (nh + nl) * (w.rho_hi[0] + w.rho_lo[0]);
+      return w.c0 * cosine_wavelet_g(q);
+    }
+    case HERMES_WIN_GDW: {
+      df_sqrt_int(n2, nh, nl);
+      float q = kTwoPi * (nh + nl) * (w.rho_hi[0] + w.rho_lo[0]);
+      return w.c0 * q * q * expf(-0.5f * q * q);
+    }
+    case HERMES_WIN_LAPLACIAN: {
+      float k2 = (float)n2 * w.c0;  // c0 = 1/L^2
+      return -(kTwoPi * kTwoPi) * k2;
+    }
+    case HERMES_WIN_INVERSE_LAPLACIAN: {
+      if (n2 == 0) return 0.f;
+      float k2 = (float)n2 * w.c0;
+      return -1.f / ((kTwoPi * kTwoPi) * k2);
+    }
+    default:
+      *ok = false;
+      return 0.f;
+  }
+}
+
 // One window at integer frequency indices (a, b, c) = k * L (signed), for
 // the given magnitude n2 = a^2+b^2+c^2.  Returns (re, im).
 __device__ __forceinline__ float2 window_at(const WinDev& w, int a, int b, int c) {
   const int n2 = a * a + b * b + c * c;
   {
     bool ok;
-    const float2 v = window_iso_n2(w, n2, &ok);
-    if (ok) return v;
+    const float v = window_radial_n2(w, n2, &ok);
+    if (ok) return make_float2(v, 0.f);
   }
-  float nh, nl;
   switch (w.type) {
     case HERMES_WIN_CUBIC: {
       // sin(pi k_i L_i)/(pi k_i L_i) per axis; rho[i] = L_i / L (double-float)
@@ -264,30 +303,10 @@ __device__ __forceinline__ float2 window_at(const WinDev& w, int a, int b, int c
       }
       return make_float2(perp * parf, 0.f);
     }
-    case HERMES_WIN_CW:
-    case HERMES_WIN_CWS: {
-      df_sqrt_int(n2, nh, nl);
-      float q = kTwoPi * (nh + nl) * (w.rho_hi[0] + w.rho_lo[0]);
-      return make_float2(w.c0 * cosine_wavelet_g(q), 0.f);
-    }
-    case HERMES_WIN_GDW: {
-      df_sqrt_int(n2, nh, nl);
-      float q = kTwoPi * (nh + nl) * (w.rho_hi[0] + w.rho_lo[0]);
-      return make_float2(w.c0 * q * q * expf(-0.5f * q * q), 0.f);
-    }
     case HERMES_WIN_DIRECTIONAL_DERIVATIVE: {
       // 2 pi i k_par ; c0 = 1/L folded into the caller's units: k = idx / L
       float kpar = ((float)a * w.los[0] + (float)b * w.los[1] + (float)c * w.los[2]) * w.c0;
       return make_float2(0.f, kTwoPi * kpar);
-    }
-    case HERMES_WIN_LAPLACIAN: {
-      float k2 = (float)n2 * w.c0;  // c0 = 1/L^2
-      return make_float2(-(kTwoPi * kTwoPi) * k2, 0.f);
-    }
-    case HERMES_WIN_INVERSE_LAPLACIAN: {
-      if (n2 == 0) return make_float2(0.f, 0.f);
-      float k2 = (float)n2 * w.c0;
-      return make_float2(-1.f / ((kTwoPi * kTwoPi) * k2), 0.f);
     }
     default:
       return make_float2(__int_as_float(0x7fc00000), 0.f);
