@@ -32,6 +32,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include <cudaTypedefs.h>
@@ -882,32 +883,43 @@ template <int NT>
 constexpr int kHSlot = NT == 1 ? kHPlane : NT * kHTile;  // one plane of all tiles
 }  // namespace hf
 
-// h plane from a staged eps plane of NT > 1 tiles: H[tile][col][uy+2][l1z],
-// the same sums as ct_compute_h.  kPer threads per column (each a range of
-// the five uy), so that 512 threads cover the tiles' columns once.
+// h plane of NT tiles from a staged eps plane, H[tile][col][uy+2][l1z], by the
+// first 64 NT threads, one column each: the weights are then known at compile
+// time (9 of the 15 are not zero) and come from the kernel's parameters, and
+// one warp's instructions cover 32 columns.  The sums are those of
+// ct_compute_h (its terms of weight zero left out).
 template <int NT>
-__device__ __forceinline__ void ct_compute_h_tiles(const float* __restrict__ w, const float* __restrict__ e,
-                                                   float* __restrict__ h) {
-  constexpr int EZ = NT * ct::TZ + 2, kPer = 8 / NT;  // 512 / (64 NT)
-  const int part = threadIdx.x / (ct::kCols * NT), cc = threadIdx.x % (ct::kCols * NT);
-  const int tile = cc / ct::kCols, col = cc % ct::kCols;
+__device__ __forceinline__ void ct_compute_h_cols(const GammaC& gm, const float* __restrict__ e, float* __restrict__ h) {
+  constexpr int EZ = NT * ct::TZ + 2;
+  // NT = 1: the two blocks of an SM take warps of different schedulers
+  const int tid = (int)threadIdx.x - (NT == 1 && 2 * blockIdx.x >= gridDim.x ? ct::kCols : 0);
+  if (tid < 0 || tid >= ct::kCols * NT) return;
+  const int tile = tid / ct::kCols, col = tid % ct::kCols;
   const int cy = col / ct::TZ, cz = tile * ct::TZ + (col & (ct::TZ - 1));
   float ev[3][3];
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) ev[i][j] = e[(cy + i) * EZ + cz + j];
-  float* dst = h + tile * hf::kHTile + col * hf::kHCol;
+  float* dst = h + (NT == 1 ? 0 : tile * hf::kHTile) + col * hf::kHCol;
 #pragma unroll
-  for (int rep = 0; rep < (5 + kPer - 1) / kPer; ++rep) {
-    const int ay = rep * kPer + part;
-    if (ay < 5) {
-      const float w0 = w[ay * 3], w1 = w[ay * 3 + 1], w2 = w[ay * 3 + 2];
-      float o[3];
+  for (int ay = 0; ay < 5; ++ay) {
+    float o[3];
 #pragma unroll
-      for (int j = 0; j < 3; ++j) o[j] = fmaf(w2, ev[2][j], fmaf(w1, ev[1][j], w0 * ev[0][j]));
-      *reinterpret_cast<float4*>(dst + ay * 4) = make_float4(o[0], o[1], o[2], 0.f);
+    for (int j = 0; j < 3; ++j) {
+      float v = 0.f;
+      bool first = true;
+#pragma unroll
+      for (int l1 = 0; l1 < 3; ++l1) {  // weight Gamma[l1][l1 - ay + 2]
+        const int l2 = l1 - ay + 2;
+        if (l2 >= 0 && l2 <= 2) {
+          v = first ? gm.g[l1 * 3 + l2] * ev[l1][j] : fmaf(gm.g[l1 * 3 + l2], ev[l1][j], v);
+          first = false;
+        }
+      }
+      o[j] = v;
     }
+    *reinterpret_cast<float4*>(dst + ay * 4) = make_float4(o[0], o[1], o[2], 0.f);
   }
 }
 
@@ -974,9 +986,13 @@ constexpr int kA3Buf = kBinStride * kA3P;
 static_assert(kA3Buf >= ct::kA3Plane, "a3 buffer");
 constexpr uint32_t kIdesc = hermes::tc::idesc_bf16_f32(128, kN, true, true);
 // 1 KB slack for the runtime 1024-byte alignment of the swizzled operands
+// h planes kept: the three a step reads and, where shared memory has room, the
+// one it computes for the next step (then one block barrier per step is enough)
+template <int NT>
+constexpr int kRing = NT < 8 ? 4 : 3;
 template <int NT>
 constexpr size_t kSmem = 1024 + 2 * kOpBytes + 2 * kRawBytes + sizeof(float2) * 2 * kA3Buf +
-                         sizeof(float) * (3 * hf::kHSlot<NT> + 2 * ct::EY * (NT * ct::TZ + 2)) +
+                         sizeof(float) * (kRing<NT> * hf::kHSlot<NT> + 2 * ct::EY * (NT * ct::TZ + 2)) +
                          sizeof(double) * 2 * kMaxBins * kMaxBins + 128;
 static_assert(kSmem<8> <= 227 * 1024 && 2 * (kSmem<1> + 1024) <= 228 * 1024, "shared memory of the contraction");
 // Threads of a block: one tile runs as two blocks of 256 threads per SM (2 x 2
@@ -1014,43 +1030,46 @@ __device__ __forceinline__ void tc_put_pair(unsigned char* op, int cell, int b, 
   *reinterpret_cast<uint32_t*>(op + tcc::kAtomCol + row + hermes::tc::sw128_offset(r, b >> 2) + byte) = l;
 }
 
-// a3 plane x_a from bin-major fields (bin b at src3 + b * bstride) -> buf
-// [16 slots][kA3P] float2; slot = tile * (16 / NT) + bin, bins nb3 and up
-// are written as zeros.  The copies are 16 bytes, two cells (2p, 2p + 1) of
-// one row: with z0 a multiple of 8 the pair starts at an even z and never
-// straddles the periodic wrap, so both ends are 16-byte aligned.  kPer
-// threads copy a slot, thread j the pairs j + kPer i of the 72 in the
-// 12 x 12 plane; the (row, pair column) of the next one is a fixed step
-// (rows hold six pairs).
+// a3 planes of bin-major fields (bin b at src3 + b * bstride) -> buf
+// [16 slots][kA3P] float2, slot = tile * (16 / NT) + bin.  The copies are
+// 16 bytes, two cells (2p, 2p + 1) of one row: with z0 a multiple of 8 the
+// pair starts at an even z and never straddles the periodic wrap, so both
+// ends are 16-byte aligned.  kPer threads copy a slot, thread j the pairs
+// j + kPer i of the 72 in the 12 x 12 plane.  A work item's planes share
+// their (y, z) offsets: a thread keeps those of its kN pairs in registers.
+// (One 96-byte bulk copy per row instead was slower, 33.8 against 25.5 ms at
+// J = 9 and 15 bins.)  Slots of bins >= nb3 are zeroed once by the kernel.
 template <int NT>
-__device__ __forceinline__ void ct_stage_a3_bm(const float2* __restrict__ src3, long long bstride, int nb3,
-                                               float2* buf, int xa, int y0, int z0, int L, int Lm) {
-  constexpr int kPairs = ct::HY * ct::HZ / 2;  // 72
-  constexpr int kPer = tcc::kThr<NT> / kBinStride, NBL = kBinStride / NT;
-  static_assert(ct::HY * ct::HZ == 144 && ct::HZ == 12 && ct::TZ % 8 == 0, "a3 staging map");
-  const int slot = threadIdx.x / kPer, j = threadIdx.x % kPer;
-  const int bin = slot % NBL, zt = z0 + ct::TZ * (slot / NBL);
-  float2* dst = buf + slot * tcc::kA3P + 2 * j;
-  const int n = (kPairs - j + kPer - 1) / kPer;
-  if (bin < nb3) {
-    const float2* src = src3 + bin * bstride + (long long)(xa & Lm) * L * L;
-    int hy = j / 6;
-    int hz = 2 * (j - 6 * hy);
-#pragma unroll 1
-    for (int i = 0; i < n; ++i) {
-      cp_async16(dst + 2 * kPer * i, src + ((y0 - 2 + hy) & Lm) * L + ((zt - 2 + hz) & Lm));
-      hz += 2 * (kPer % 6);
-      hy += kPer / 6;
-      if (hz >= ct::HZ) {
-        hz -= ct::HZ;
-        hy += 1;
-      }
+struct A3Copy {
+  static constexpr int kPairs = ct::HY * ct::HZ / 2;  // 72
+  static constexpr int kPer = tcc::kThr<NT> / kBinStride, kN = (kPairs + kPer - 1) / kPer;
+  const float2* src;  // the bin's field
+  int off[kN];        // float2 offsets in an x plane
+  bool active;        // the slot holds a bin
+
+  __device__ __forceinline__ void set(const float2* __restrict__ src3, long long bstride, int nb3, int y0, int z0, int L,
+                                      int Lm) {
+    constexpr int NBL = kBinStride / NT;
+    const int slot = threadIdx.x / kPer, j = threadIdx.x % kPer;
+    active = slot % NBL < nb3;
+    src = src3 + (slot % NBL) * bstride;
+    const int zt = z0 + ct::TZ * (slot / NBL);
+#pragma unroll
+    for (int i = 0; i < kN; ++i) {
+      const int p = j + kPer * i, hy = p / (ct::HZ / 2), hz = 2 * (p % (ct::HZ / 2));
+      off[i] = ((y0 - 2 + hy) & Lm) * L + ((zt - 2 + hz) & Lm);
     }
-  } else {
-#pragma unroll 1
-    for (int i = 0; i < n; ++i) *reinterpret_cast<float4*>(dst + 2 * kPer * i) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-}
+  __device__ __forceinline__ void plane(float2* buf, int xa, int L, int Lm) const {
+    if (!active) return;
+    const int slot = threadIdx.x / kPer, j = threadIdx.x % kPer;
+    const float2* s = src + (long long)(xa & Lm) * L * L;
+    float2* dst = buf + slot * tcc::kA3P + 2 * j;
+#pragma unroll
+    for (int i = 0; i < kN; ++i)
+      if ((i + 1) * kPer <= kPairs || j + kPer * i < kPairs) cp_async16(dst + 2 * kPer * i, s + off[i]);
+  }
+};
 
 // kBM: fields in the bin-major layout [bin][cell] that cuFFT writes (a2 by a
 // 4-D TMA map over (z, y, x, bin), a3 staged per bin); otherwise the
@@ -1063,6 +1082,13 @@ __device__ __forceinline__ void ct_stage_a3_bm(const float2* __restrict__ src3, 
 // operands in the same order as when the tile runs alone), the others are
 // not read.  A tile's S goes to A.items, and mp_reduce_items_kernel adds the
 // tiles in the order of the one-tile blocks: the result is the same bits.
+//
+// What bounds it (ncu, J = 8, 15 bins): shared-memory wavefronts 66% of their
+// peak (264 per warp and plane: 120 for the h planes, 72 for a3, 33 for its
+// staging), issue slots 51%, FMA pipe 45%; the FMAs alone would take 9 ms at
+// J = 9.  22.5 ms at J = 9 and 15 bins; 25.5 ms with the a3 addresses computed
+// anew for every plane, the h plane spread over four threads a column and two
+// block barriers a step.
 template <bool kBM, int NT>
 __global__ void __launch_bounds__(tcc::kThr<NT>, NT == 1 ? 2 : 1)
 mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map) {
@@ -1079,12 +1105,14 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
   float2* abuf = reinterpret_cast<float2*>(reinterpret_cast<unsigned char*>(araw) + 2 * tcc::kRawBytes);
   double* dacc = reinterpret_cast<double*>(abuf + 2 * tcc::kA3Buf);  // [16][16][2]
   float* hring = reinterpret_cast<float*>(dacc + 2 * kMaxBins * kMaxBins);  // [3][kHPlane]
-  float* epsb = hring + 3 * kHS;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(epsb + 2 * kEps);  // tma[2], mma
+  constexpr bool kOneBar = kBM && tcc::kRing<NT> == 4;
+  float* epsb = hring + tcc::kRing<NT> * kHS;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(epsb + 2 * kEps);  // a2 planes [2], mma
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3);
   float* gsm = reinterpret_cast<float*>(tmem_slot + 1);                  // 15 h-pass weights
   int* s_abort = reinterpret_cast<int*>(gsm + 16);
-  float* stage = reinterpret_cast<float*>(abuf);                          // [96][33] at item end
+  // [96][33] at item end (kBM: not in abuf, whose zero slots stay)
+  float* stage = kBM ? araw : reinterpret_cast<float*>(abuf);
 
   const int J = A.J, L = 1 << J, Lm = L - 1, CX = A.CX;
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -1098,10 +1126,10 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
   const int nty = L / ct::TY, ntz = L / (NT * ct::TZ);
   auto stage_eps = [&](float* buf, int xe, int y0, int z0) { ct_stage_eps<NT, kThr>(A.eps1, buf, xe, y0, z0, L, Lm); };
   auto compute_h = [&](const float* e, float* h, const float* w) {
-    if constexpr (NT == 1)
-      ct_compute_h(w, e, h);
+    if constexpr (kBM)
+      ct_compute_h_cols<NT>(A.gm, e, h);
     else
-      ct_compute_h_tiles<NT>(w, e, h);
+      ct_compute_h(w, e, h);
   };
   const int n_items = (L / CX) * nty * ntz;
   const int nsteps = CX + 4;
@@ -1124,6 +1152,9 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
   }
   if (warp == 0) tc::tmem_alloc(tmem_slot, tcc::kTmemCols);
   for (int i = tid; i < 2 * kMaxBins * kMaxBins; i += kThr) dacc[i] = 0.0;
+  if (kBM)
+    for (int i = tid; i < 2 * tcc::kA3Buf; i += kThr)
+      if (i % tcc::kA3Buf / tcc::kA3P % NBL >= A.nb3s) abuf[i] = make_float2(0.f, 0.f);
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
@@ -1144,15 +1175,20 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
     compute_h(epsb, hring, gsm);
     compute_h(epsb + kEps, hring + kHS, gsm);
     __syncthreads();
-    if constexpr (kBM)
-      ct_stage_a3_bm<NT>(A.src3, A.bstride, A.nb3s, abuf, x0 - 2, y0, z0, L, Lm);
-    else
+    A3Copy<NT> a3;
+    if constexpr (kBM) {
+      a3.set(A.src3, A.bstride, A.nb3s, y0, z0, L, Lm);
+      a3.plane(abuf, x0 - 2, L, Lm);
+    } else {
       ct_stage_a3(A.src3, A.s3, abuf, x0 - 2, y0, z0, L, Lm);
+    }
     stage_eps(epsb, x0, y0, z0);
+    if (kOneBar) stage_eps(epsb + kEps, x0 + 1, y0, z0);
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
     compute_h(epsb, hring + 2 * kHS, gsm);
+    if (kOneBar) __syncthreads();
 
     float2 G[5][NC];
 #pragma unroll
@@ -1161,19 +1197,26 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
       for (int c = 0; c < NC; ++c) G[q][c] = make_float2(0.f, 0.f);
     bool first_mma = true;
 
-    // Two block barriers per step: the first makes the h plane computed at
-    // the end of the previous step visible; the second the staged a3 / eps
-    // planes (each thread waited for its own copies) and the MMA operands.
+    // The block barrier at the end of a step makes the staged a3 / eps planes
+    // (each thread waited for its own copies), the MMA operands and, with a
+    // ring of four (kOneBar), the h plane of the next step visible.  With a
+    // ring of three that h plane overwrites one the step reads: it is
+    // computed after the barrier, and a second one at the start of the step
+    // makes it visible.
     for (int st = 0; st < nsteps; ++st) {
       const int xa = x0 - 2 + st;
       if (st + 1 < nsteps) {
         // a3 plane xa+1 and eps plane xa+3: their buffers' last readers (the
         // stencil one step back, the h pass two steps back) are done
-        if constexpr (kBM)
-          ct_stage_a3_bm<NT>(A.src3, A.bstride, A.nb3s, abuf + ((st + 1) & 1) * tcc::kA3Buf, xa + 1, y0, z0, L, Lm);
-        else
+        if constexpr (kBM) {
+          a3.plane(abuf + ((st + 1) & 1) * tcc::kA3Buf, xa + 1, L, Lm);
+        } else {
           ct_stage_a3(A.src3, A.s3, abuf + ((st + 1) & 1) * tcc::kA3Buf, xa + 1, y0, z0, L, Lm);
-        stage_eps(epsb + ((st + 1) & 1) * kEps, xa + 3, y0, z0);
+        }
+        if (kOneBar)
+          stage_eps(epsb + (st & 1) * kEps, xa + 4, y0, z0);
+        else
+          stage_eps(epsb + ((st + 1) & 1) * kEps, xa + 3, y0, z0);
         // a2 plane of the next step's product (its buffer's last reader, the
         // split two steps back, finished before the last block barrier)
         if (tma_a2 && tid == 0 && st + 1 >= 4) {
@@ -1190,13 +1233,18 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
         }
       }
       cp_async_commit();
-      __syncthreads();
-      {
+      if (kOneBar)
+        compute_h(epsb + ((st + 1) & 1) * kEps, hring + ((st + 3) & 3) * kHS, gsm);  // h(xa + 3)
+      else
+        __syncthreads();
+      auto stencil = [&](auto odd_start) {
+        constexpr int kOdd = decltype(odd_start)::value;
         const float2* ap = abuf + (st & 1) * tcc::kA3Buf;
         const int ht = NT == 1 ? 0 : (b / NBL) * hf::kHTile;
-        const float* hp0 = hring + (st % 3) * kHS + ht;
-        const float* hp1 = hring + ((st + 1) % 3) * kHS + ht;
-        const float* hp2 = hring + ((st + 2) % 3) * kHS + ht;
+        constexpr int kRing = kOneBar ? 4 : 3;
+        const float* hp0 = hring + (st % kRing) * kHS + ht;
+        const float* hp1 = hring + ((st + 1) % kRing) * kHS + ht;
+        const float* hp2 = hring + ((st + 2) % kRing) * kHS + ht;
         float2 T[3][NC];
 #pragma unroll
         for (int d = 0; d < 3; ++d)
@@ -1205,17 +1253,8 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
 #pragma unroll
         for (int r = 0; r < 6; ++r) {
           float2 av[6];
-          if (kBM && CZ == 1) {  // the pairs around five cells that start at an odd or even z
-            const float4* row4 = reinterpret_cast<const float4*>(ap + b * tcc::kA3P + (cy + r) * ct::HZ + (cz & ~1));
-            const float4 p0 = row4[0], p1 = row4[1], p2 = row4[2];
-            const bool odd = cz & 1;  // the same for the whole warp
-            av[0] = odd ? make_float2(p0.z, p0.w) : make_float2(p0.x, p0.y);
-            av[1] = odd ? make_float2(p1.x, p1.y) : make_float2(p0.z, p0.w);
-            av[2] = odd ? make_float2(p1.z, p1.w) : make_float2(p1.x, p1.y);
-            av[3] = odd ? make_float2(p2.x, p2.y) : make_float2(p1.z, p1.w);
-            av[4] = odd ? make_float2(p2.z, p2.w) : make_float2(p2.x, p2.y);
-          } else if (kBM) {  // two cells per 16-byte load (cz even, kA3P even)
-            const float4* row4 = reinterpret_cast<const float4*>(ap + b * tcc::kA3P + (cy + r) * ct::HZ + cz);
+          if (kBM) {  // two cells per 16-byte load (cz - kOdd and kA3P are even)
+            const float4* row4 = reinterpret_cast<const float4*>(ap + b * tcc::kA3P + (cy + r) * ct::HZ + cz - kOdd);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
               const float4 p = row4[k];
@@ -1233,9 +1272,9 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
 #pragma unroll
             for (int l1z = 0; l1z < 3; ++l1z) {
               const float g0 = A.gm.g[l1z * 3], g1 = A.gm.g[l1z * 3 + 1], g2 = A.gm.g[l1z * 3 + 2];
-              float2 t = __fmul2_rn(make_float2(g2, g2), av[dz + l1z]);
-              t = __ffma2_rn(make_float2(g1, g1), av[dz + l1z + 1], t);
-              rz[dz][l1z] = __ffma2_rn(make_float2(g0, g0), av[dz + l1z + 2], t);
+              float2 t = __fmul2_rn(make_float2(g2, g2), av[kOdd + dz + l1z]);
+              t = __ffma2_rn(make_float2(g1, g1), av[kOdd + dz + l1z + 1], t);
+              rz[dz][l1z] = __ffma2_rn(make_float2(g0, g0), av[kOdd + dz + l1z + 2], t);
             }
 #pragma unroll
           for (int dy = 0; dy < 2; ++dy) {
@@ -1262,8 +1301,18 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
           for (int l1x = 0; l1x < 3; ++l1x) {
             const float gx = A.gm.g[l1x * 3 + d];
 #pragma unroll
-            for (int c = 0; c < NC; ++c) G[d - l1x + 2][c] = __ffma2_rn(make_float2(gx, gx), T[d][c], G[d - l1x + 2][c]);
+            for (int c = 0; c < NC; ++c)
+              G[d - l1x + 2][c] = d - l1x + 2 == 4 ? __fmul2_rn(make_float2(gx, gx), T[d][c])
+                                                   : __ffma2_rn(make_float2(gx, gx), T[d][c], G[d - l1x + 2][c]);
           }
+      };
+      if constexpr (CZ == 1) {  // a warp's columns all start at an even or all at an odd z
+        if (cz & 1)
+          stencil(std::integral_constant<int, 1>{});
+        else
+          stencil(std::integral_constant<int, 0>{});
+      } else {
+        stencil(std::integral_constant<int, 0>{});
       }
       // G(xa - 2) and the a2 plane xa - 2 become the operands of this plane's MMA
       const bool full = st >= 4;
@@ -1336,13 +1385,11 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
       for (int q = 0; q < 4; ++q)
 #pragma unroll
         for (int c = 0; c < NC; ++c) G[q][c] = G[q + 1][c];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) G[4][c] = make_float2(0.f, 0.f);
       cp_async_wait<0>();
       __syncthreads();
       if (*s_abort) break;
       // h(xa + 3) for the next step, into the ring slot this step's T_0 used
-      if (st + 1 < nsteps) compute_h(epsb + ((st + 1) & 1) * kEps, hring + (st % 3) * kHS, gsm);
+      if (!kOneBar && st + 1 < nsteps) compute_h(epsb + ((st + 1) & 1) * kEps, hring + (st % 3) * kHS, gsm);
       if (full) {
         if (tid == 0) {
           tc::tc_fence_after();
@@ -1411,9 +1458,14 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
         A.items[(o + 1) * A.n_items1 + item1] = si;
       }
     }
-    __syncthreads();  // stage (a3 buffer) idle before the next item's prologue
+    if (kBM) tc::fence_proxy_async_smem();  // stage, before the next item's a2 planes
+    __syncthreads();  // stage idle before the next item
   }
   const int why = *s_abort;
+  if (kBM && why) {  // a wait gave up: give the copies in flight a moment before leaving
+    tc::mbar_wait(&bars[0], tma_ph0, 1u << 14);
+    tc::mbar_wait(&bars[1], tma_ph1, 1u << 14);
+  }
   if constexpr (NT == 1) {
     for (int i = tid; i < 2 * kMaxBins * kMaxBins; i += kThr)
       A.partial[(long long)blockIdx.x * 2 * kMaxBins * kMaxBins + i] =
@@ -1942,17 +1994,18 @@ static int make_a2_map_bm(const void* fields, int L, int nb, int box_bins, CUten
 enum { kEngineTensor = 0, kEngineSimt = 1, kEngineTensorBinMajor = 2 };
 
 // Tiles side by side in the tensor-core contraction of nb bins (1, 2, 4 or
-// 8, with 16 / tiles >= nb bin slots each): the count with the fewest rounds
-// of work.  Two blocks of one tile share an SM, so a round of those counts
-// two; a block of several tiles has the SM to itself, and a round counts 1.1
-// for the h planes of the tiles.  At J = 8, 2 bins take 0.85 ms with 8 tiles
-// (2 rounds) and 3.02 ms with one (7 rounds of 2).
+// 8, with 16 / tiles >= nb bin slots each): the count with the least work,
+// rounds of items times the cost of a round.  Two blocks of one tile share an
+// SM, and their round of 132 planes takes 0.42 ms; a block of 2, 4 or 8 tiles
+// has the SM to itself and takes 0.30, 0.32 and 0.40 ms.  At J = 8, 2 bins take
+// 0.80 ms with 8 tiles, 2.93 ms with one.
 static int contract_tiles(int nb, int per_tile, int L, int ctas_per_sm, int nsm) {
-  const int slots = ctas_per_sm * nsm;
+  const double round[4] = {0.21 * ctas_per_sm, 0.30, 0.32, 0.40};
   int best = 1;
-  double cost = ctas_per_sm * (double)((per_tile + slots - 1) / slots);
-  for (int t = 2; t <= 8 && t * nb <= kBinStride && t * ct::TZ <= L; t *= 2) {
-    const double c = 1.1 * (double)((per_tile / t + nsm - 1) / nsm);
+  double cost = 1e30;
+  for (int k = 0, t = 1; k < 4 && (t == 1 || (t * nb <= kBinStride && t * ct::TZ <= L)); ++k, t *= 2) {
+    const int slots = t == 1 ? ctas_per_sm * nsm : nsm;
+    const double c = round[k] * (double)((per_tile / t + slots - 1) / slots);
     if (c < cost) {
       best = t;
       cost = c;
