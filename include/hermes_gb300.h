@@ -433,8 +433,13 @@ int hermes_mc_sample(const float* eps1, const float* eps2, const float* eps3, in
  * sectors instead of 9 rows of 1-2 sectors.  hermes_mc_triplets_bricks and
  * hermes_mc_sample_bricks take the same arguments as hermes_mc_triplets and
  * hermes_mc_sample with eps1..eps3 in that layout and return the same values
- * bit for bit (the same float32 products in the same order). */
+ * bit for bit (the same float32 products in the same order).  Fields that are
+ * 32-byte aligned are read by whole bricks, others cell by cell. */
 int hermes_field_to_bricks(const float* field, int J, float* bricks, void* stream);
+/* keys[i] = 30-bit Morton (Z-curve) key of the cell of centre i (centers:
+ * device float64 [n][3], grid units): sorted by it, centres that run together
+ * gather nearby cells. */
+int hermes_mc_morton_keys(const double* centers, int64_t n, int J, int32_t* keys, void* stream);
 int hermes_mc_triplets_bricks(const float* eps1, const float* eps2, const float* eps3, int J,
                               const double* centers, const double* center_w, int64_t n_centers,
                               const double* offsets, int n_rot, const double* phi, int n_phi,

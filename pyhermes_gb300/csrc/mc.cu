@@ -10,6 +10,8 @@
 // GPU sums exactly the same (centre, offset) pairs.  One thread per centre
 // loads the centre once, gathers n1 once and loops over the rotations;
 // products are float32, sums float64 with a fixed-order block reduction.
+#include <algorithm>
+
 #include "hermes_common.cuh"
 
 namespace {
@@ -38,33 +40,152 @@ __device__ __forceinline__ size_t mc_cell(int x, int y, int z, int J) {
   return brick << 3 | (size_t)((x & 1) << 2 | (y & 1) << 1 | (z & 1));
 }
 
-// 27-point interpolation of a float32 field at scaled position (sx, sy, sz).
-template <bool kBricks = false>
+// One axis of the stencil: phi at fraction f + 0, 1, 2 units weights the cells
+// c, c - 1, c - 2 (v2, v1, v0).  Every gather reduces z, then y, then x with
+// this sum, so all layouts give the same bits.
+__device__ __forceinline__ float mc_axis_sum(float v0, float v1, float v2, float p0, float p1, float p2) {
+  return fmaf(p0, v2, fmaf(p1, v1, p2 * v0));
+}
+
+// 27-point interpolation of a float32 field at scaled position (sx, sy, sz),
+// cell by cell.
+template <bool kBricks>
 __device__ __forceinline__ float mc_interp(const float* __restrict__ grid, const float* __restrict__ phis, int res,
                                            int J, double sx, double sy, double sz) {
-  const int L = 1 << J;
+  const int L = 1 << J, m = L - 1;
   int cx, cy, cz, fx, fy, fz;
   mc_axis(sx, res, L, cx, fx);
   mc_axis(sy, res, L, cy, fy);
   mc_axis(sz, res, L, cz, fz);
-  const int m = L - 1;
-  float acc = 0.f;
+  const float pz0 = phis[fz], pz1 = phis[fz + res], pz2 = phis[fz + 2 * res];
+  const float py0 = phis[fy], py1 = phis[fy + res], py2 = phis[fy + 2 * res];
+  float rx[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const int xg = (cx - a) & m;
-    const float px = phis[fx + a * res];
+    float ry[3];
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-      const int yg = (cy - b) & m;
-      const float py = phis[fy + b * res];
+      float v[3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int zg = (cz - c) & m;
-        acc += __ldg(grid + mc_cell<kBricks>(xg, yg, zg, J)) * px * py * phis[fz + c * res];
-      }
+      for (int c = 0; c < 3; ++c)
+        v[c] = __ldg(grid + mc_cell<kBricks>((cx - 2 + a) & m, (cy - 2 + b) & m, (cz - 2 + c) & m, J));
+      ry[b] = mc_axis_sum(v[0], v[1], v[2], pz0, pz1, pz2);
     }
+    rx[a] = mc_axis_sum(ry[0], ry[1], ry[2], py0, py1, py2);
   }
-  return acc;
+  return mc_axis_sum(rx[0], rx[1], rx[2], phis[fx], phis[fx + res], phis[fx + 2 * res]);
+}
+
+// ---- brick-layout gather --------------------------------------------------------
+// A 3 x 3 x 3 stencil lies in exactly 8 bricks.  mc_interp above reads its 27
+// cells one by one: 27 loads per lane, and as many table reads for phi, each of
+// a warp's 32 addresses in another 128-byte line, which is what bounds it
+// (about one line per SM and clock).  Here a lane reads each brick with one
+// 32-byte load, phi from shared memory, and reduces z, y, x in turn.  Of the
+// four cells per axis of the two bricks the stencil's three are picked by
+// selects (a cell outside the stencil never enters a product).
+// 2e5 centres x 100 rotations at J = 9: 2.75 ms (3.03 ms cell by cell), and
+// 1.31 ms with the rotations of a centre side by side (mc_triplet_kernel).
+struct __align__(16) McPhi {
+  float4 p[1024];  // phi at fraction f + 0, 1, 2 units
+};
+
+__device__ __forceinline__ void mc_load_phi(McPhi* sp, const float* __restrict__ phis, int res) {
+  for (int i = threadIdx.x; i < res; i += blockDim.x) sp->p[i] = make_float4(phis[i], phis[i + res], phis[i + 2 * res], 0.f);
+  __syncthreads();
+}
+
+// mc_axis for a power-of-two res = 2^rl and 0 <= s < 2^30, from the bits of s
+// (the integer part and the next rl bits of the mantissa are exactly floor(s)
+// and int((s - floor(s)) res)): float64 floor, subtract, multiply and
+// conversions take 16 cycles of the SM per warp each.
+__device__ __forceinline__ void mc_axis_bits(double s, int res, int rl, int L, int& c, int& f) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(s);
+  const int ex = (int)(b >> 52);  // the sign bit makes it too large
+  if (rl < 0 || ex >= 1023 + 30 || ex == 0) {
+    mc_axis(s, res, L, c, f);
+    return;
+  }
+  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+  const int sh = 1075 - ex, t = sh - rl;  // s = m 2^-sh, sh >= 23
+  c = sh >= 64 ? 0 : (int)(m >> sh) & (L - 1);
+  f = t >= 64 ? 0 : (int)(m >> t) & (res - 1);
+}
+
+__device__ __forceinline__ void mc_brick(const float* __restrict__ p, float (&v)[8]) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+      : "l"(p));
+}
+
+// the three of a0 .. a3 that start at a1 (odd) or a0
+__device__ __forceinline__ float mc_reduce3(float a0, float a1, float a2, float a3, bool odd, float4 w) {
+  return mc_axis_sum(odd ? a1 : a0, odd ? a2 : a1, odd ? a3 : a2, w.x, w.y, w.z);
+}
+
+__device__ __forceinline__ float mc_interp_bricks(const float* __restrict__ bricks, const McPhi* sp, int res, int rl, int J,
+                                                  double sx, double sy, double sz) {
+  const int L = 1 << J, h = J - 1, hm = (1 << h) - 1;
+  int cx, cy, cz, fx, fy, fz;
+  mc_axis_bits(sx, res, rl, L, cx, fx);
+  mc_axis_bits(sy, res, rl, L, cy, fy);
+  mc_axis_bits(sz, res, rl, L, cz, fz);
+  const float4 wx = sp->p[fx], wy = sp->p[fy], wz = sp->p[fz];
+  const bool ox = cx & 1, oy = cy & 1, oz = cz & 1;
+  // brick coordinates: the lower one, then the one that holds the cell
+  const int bx[2] = {((cx >> 1) - 1) & hm, cx >> 1}, by[2] = {((cy >> 1) - 1) & hm, cy >> 1};
+  const int z0 = ((cz >> 1) - 1) & hm, z1 = cz >> 1;
+  float rx[4];  // the four cells along x, reduced over y and z
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    float ry[2][4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const size_t row = (((size_t)bx[i] << h) + by[j]) << h;
+      float lo[8], hi[8];
+      mc_brick(bricks + ((row + z0) << 3), lo);
+      mc_brick(bricks + ((row + z1) << 3), hi);
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          const int k = 4 * x + 2 * y;
+          ry[x][2 * j + y] = mc_reduce3(lo[k], lo[k + 1], hi[k], hi[k + 1], oz, wz);
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x) rx[2 * i + x] = mc_reduce3(ry[x][0], ry[x][1], ry[x][2], ry[x][3], oy, wy);
+  }
+  return mc_reduce3(rx[0], rx[1], rx[2], rx[3], ox, wx);
+}
+
+// Interpolation in the layout of the kernel's fields: C order, bricks cell by
+// cell (fields that are not 32-byte aligned), bricks by whole bricks.
+enum { kCOrder = 0, kBrickCells = 1, kBricks = 2 };
+template <int kLayout>
+__device__ __forceinline__ float mc_value(const float* __restrict__ grid, const float* __restrict__ phis, const McPhi* sp,
+                                          int res, int rl, int J, double sx, double sy, double sz) {
+  if constexpr (kLayout == kBricks)
+    return mc_interp_bricks(grid, sp, res, rl, J, sx, sy, sz);
+  else
+    return mc_interp<kLayout == kBrickCells>(grid, phis, res, J, sx, sy, sz);
+}
+
+// Morton key (30 bits) of the cell of every centre (grid units).
+__global__ void mc_morton_kernel(const double* __restrict__ centers, int64_t n, int L, int* __restrict__ keys) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    unsigned key = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      unsigned v = (unsigned)(long long)floor(centers[3 * i + a]) & (unsigned)(L - 1);  // 10 bits
+      v = (v | (v << 16)) & 0x030000FFu;
+      v = (v | (v << 8)) & 0x0300F00Fu;
+      v = (v | (v << 4)) & 0x030C30C3u;
+      v = (v | (v << 2)) & 0x09249249u;
+      key |= v << a;
+    }
+    keys[i] = (int)key;
+  }
 }
 
 __global__ void mc_phi_kernel(const double* __restrict__ phi, int n, float* __restrict__ out) {
@@ -75,29 +196,40 @@ __global__ void mc_interp_kernel(const float* __restrict__ grid, int J, const do
                                  const float* __restrict__ phis, int res, double dx, double dy, double dz,
                                  double* __restrict__ out) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = (double)mc_interp(grid, phis, res, J, pos[3 * i] + dx, pos[3 * i + 1] + dy, pos[3 * i + 2] + dz);
+    out[i] = (double)mc_interp<false>(grid, phis, res, J, pos[3 * i] + dx, pos[3 * i + 1] + dy, pos[3 * i + 2] + dz);
 }
 
 // sum_i w_i n1_i sum_r n2(x_i + d2_r) n3(x_i + d3_r); n1 = eps1 interpolated
 // (box-random centres) or rho1 (particle centres: eps1 == NULL).  When
-// samples != NULL also writes the per-(centre, rotation) products f_ir.
-// kBricks: the fields are in the brick layout (mc_cell).
-template <bool kBricks>
+// samples != NULL also writes the per-(centre, rotation) products f_ir.  A centre's rotations
+// are shared by n_part threads (part p takes r = p, p + n_part, ...).  A warp
+// holds 32 neighbouring centres of one part, and the parts of those centres
+// are neighbouring warps: the threads in flight then cover a small part of the
+// box (1/8 of it for 2e5 centres in 12 parts), whose bricks L2 holds, and not
+// all centres with a few rotations each, whose bricks it does not.
+template <int kLayout>
 __global__ void __launch_bounds__(256)
 mc_triplet_kernel(const float* __restrict__ eps1, const float* __restrict__ eps2, const float* __restrict__ eps3,
                   int J, const double* __restrict__ centers, const double* __restrict__ cw, int64_t nc,
-                  const double* __restrict__ offsets, int n_rot, const float* __restrict__ phis, int res,
-                  double rho1, double* __restrict__ partial, float* __restrict__ samples) {
+                  const double* __restrict__ offsets, int n_rot, int n_part, const float* __restrict__ phis, int res,
+                  int rl, double rho1, double* __restrict__ partial, float* __restrict__ samples) {
+  __shared__ McPhi sphi[1];  // kBricks
+  if (kLayout == kBricks) mc_load_phi(sphi, phis, res);
   double acc = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += (int64_t)gridDim.x * blockDim.x) {
+  const int64_t items = (nc + 31) / 32 * n_part * 32;
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < items; k += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t w32 = k >> 5;
+    const int part = (int)(w32 % n_part);
+    const int64_t i = w32 / n_part * 32 + (k & 31);
+    if (i >= nc) continue;
     const double x = centers[3 * i], y = centers[3 * i + 1], z = centers[3 * i + 2];
-    const float n1 = eps1 ? mc_interp<kBricks>(eps1, phis, res, J, x, y, z) : (float)rho1;
+    const float n1 = eps1 ? mc_value<kLayout>(eps1, phis, sphi, res, rl, J, x, y, z) : (float)rho1;
     const float w = cw ? (float)cw[i] : 1.f;
     float s = 0.f;
-    for (int r = 0; r < n_rot; ++r) {
+    for (int r = part; r < n_rot; r += n_part) {
       const double* o = offsets + 6 * r;
-      const float n2 = mc_interp<kBricks>(eps2, phis, res, J, x + o[0], y + o[1], z + o[2]);
-      const float n3 = mc_interp<kBricks>(eps3, phis, res, J, x + o[3], y + o[4], z + o[5]);
+      const float n2 = mc_value<kLayout>(eps2, phis, sphi, res, rl, J, x + o[0], y + o[1], z + o[2]);
+      const float n3 = mc_value<kLayout>(eps3, phis, sphi, res, rl, J, x + o[3], y + o[4], z + o[5]);
       const float f = w * n1 * n2 * n3;
       if (samples) samples[i * n_rot + r] = f;
       s += f;
@@ -171,13 +303,15 @@ __device__ __forceinline__ void mc_triangle(double R1, double R2, double mu, dou
 // [n][6] or drawn (phi, cos theta1, alpha uniform, as the reference's three
 // uniforms); value f_k = w_k n1(c) n2(c + o1) n3(c + o2) (w_k = 1 when w is
 // NULL).  Block partial sums of f and f^2.
-template <bool kBricks>
+template <int kLayout>
 __global__ void __launch_bounds__(256)
 mc_sample_kernel(const float* __restrict__ eps1, const float* __restrict__ eps2, const float* __restrict__ eps3,
                  int J, const double* __restrict__ pool, long long M, const long long* __restrict__ idx,
                  const double* __restrict__ w, const double* __restrict__ offsets, long long n, double R1, double R2,
-                 double mu,
-                 unsigned long long seed, const float* __restrict__ phis, int res, double* __restrict__ partial) {
+                 double mu, unsigned long long seed, const float* __restrict__ phis, int res, int rl,
+                 double* __restrict__ partial) {
+  __shared__ McPhi sphi[1];  // kBricks
+  if (kLayout == kBricks) mc_load_phi(sphi, phis, res);
   double acc = 0.0, acc2 = 0.0;
   for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
     unsigned long long st = seed ^ ((unsigned long long)k * 0xD1B54A32D192ED03ull);
@@ -198,9 +332,9 @@ mc_sample_kernel(const float* __restrict__ eps1, const float* __restrict__ eps2,
       mc_triangle(R1, R2, mu, a, 2.0 * bb - 1.0, c, o);
     }
     const double x = pool[3 * i], y = pool[3 * i + 1], z = pool[3 * i + 2];
-    const float n1 = mc_interp<kBricks>(eps1, phis, res, J, x, y, z);
-    const float n2 = mc_interp<kBricks>(eps2, phis, res, J, x + o[0], y + o[1], z + o[2]);
-    const float n3 = mc_interp<kBricks>(eps3, phis, res, J, x + o[3], y + o[4], z + o[5]);
+    const float n1 = mc_value<kLayout>(eps1, phis, sphi, res, rl, J, x, y, z);
+    const float n2 = mc_value<kLayout>(eps2, phis, sphi, res, rl, J, x + o[0], y + o[1], z + o[2]);
+    const float n3 = mc_value<kLayout>(eps3, phis, sphi, res, rl, J, x + o[3], y + o[4], z + o[5]);
     double f = (double)(n1 * n2 * n3);
     if (w) f *= w[k];
     acc += f;
@@ -239,6 +373,12 @@ __global__ void mc_to_bricks_kernel(const float* __restrict__ src, int J, float*
     dst[i] = __ldg(src + mc_cell<false>(x, y, z, J));
   }
 }
+
+bool bricks_aligned(const float* a, const float* b, const float* c) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 31u) == 0;
+}
+
+int log2_or_negative(int v) { return (v & (v - 1)) == 0 ? __builtin_ctz((unsigned)v) : -1; }
 
 int mc_grid() {
   int dev = 0, nsm = 148;
@@ -303,12 +443,16 @@ static int mc_triplets(const float* eps1, const float* eps2, const float* eps3, 
   int rc = mc_prepare(phi, n_phi, phi_res, workspace, workspace_bytes, &phis, &partial, s);
   if (rc) return rc;
   const int g = mc_grid();
-  if (bricks)
-    mc_triplet_kernel<true><<<g, 256, 0, s>>>(eps1, eps2, eps3, J, centers, center_w, n_centers, offsets, n_rot, phis,
-                                              phi_res, rho1, partial, samples_out);
-  else
-    mc_triplet_kernel<false><<<g, 256, 0, s>>>(eps1, eps2, eps3, J, centers, center_w, n_centers, offsets, n_rot,
-                                               phis, phi_res, rho1, partial, samples_out);
+  // about 8 rotations a thread: each part interpolates its centre's n1 again
+  // (6% at 8); fewer parts leave the grid short of threads or spread the
+  // threads in flight over the box
+  const int n_part = std::max(1, n_rot / 8);
+  const int rl = log2_or_negative(phi_res);
+  const auto kernel = !bricks                               ? mc_triplet_kernel<kCOrder>
+                      : bricks_aligned(eps1, eps2, eps3) ? mc_triplet_kernel<kBricks>
+                                                         : mc_triplet_kernel<kBrickCells>;
+  kernel<<<g, 256, 0, s>>>(eps1, eps2, eps3, J, centers, center_w, n_centers, offsets, n_rot, n_part, phis, phi_res, rl,
+                           rho1, partial, samples_out);
   HERMES_LAUNCH_CHECK("mc_triplet_kernel");
   mc_sum_kernel<<<1, 256, 0, s>>>(partial, g, partial + g);
   HERMES_LAUNCH_CHECK("mc_sum_kernel");
@@ -331,14 +475,12 @@ static int mc_sample(const float* eps1, const float* eps2, const float* eps3, in
   int rc = mc_prepare(phi, n_phi, phi_res, workspace, workspace_bytes, &phis, &partial, s);
   if (rc) return rc;
   const int g = mc_grid();
-  if (bricks)
-    mc_sample_kernel<true><<<g, 256, 0, s>>>(eps1, eps2, eps3, J, pool, (long long)M,
-                                             reinterpret_cast<const long long*>(idx), weights, offsets, (long long)n,
-                                             R1, R2, mu, (unsigned long long)seed, phis, phi_res, partial);
-  else
-    mc_sample_kernel<false><<<g, 256, 0, s>>>(eps1, eps2, eps3, J, pool, (long long)M,
-                                              reinterpret_cast<const long long*>(idx), weights, offsets, (long long)n,
-                                              R1, R2, mu, (unsigned long long)seed, phis, phi_res, partial);
+  const int rl = log2_or_negative(phi_res);
+  const auto kernel = !bricks                               ? mc_sample_kernel<kCOrder>
+                      : bricks_aligned(eps1, eps2, eps3) ? mc_sample_kernel<kBricks>
+                                                         : mc_sample_kernel<kBrickCells>;
+  kernel<<<g, 256, 0, s>>>(eps1, eps2, eps3, J, pool, (long long)M, reinterpret_cast<const long long*>(idx), weights,
+                           offsets, (long long)n, R1, R2, mu, (unsigned long long)seed, phis, phi_res, rl, partial);
   HERMES_LAUNCH_CHECK("mc_sample_kernel");
   mc_sum_kernel<<<1, 256, 0, s>>>(partial, g, partial + 2 * g);
   HERMES_LAUNCH_CHECK("mc_sum_kernel");
@@ -383,6 +525,16 @@ extern "C" int hermes_mc_sample_bricks(const float* eps1, const float* eps2, con
                                        void* workspace, size_t workspace_bytes, void* stream) {
   return mc_sample(eps1, eps2, eps3, J, pool, M, idx, weights, offsets, n, R1, R2, mu, seed, phi, n_phi, phi_res,
                    sums_out, workspace, workspace_bytes, stream, true);
+}
+
+extern "C" int hermes_mc_morton_keys(const double* centers, int64_t n, int J, int32_t* keys, void* stream) {
+  if (n < 0 || (n > 0 && (!centers || !keys))) return fail(HERMES_ERR_INVALID, "mc_morton_keys: bad argument");
+  if (J < 2 || J > 10) return fail(HERMES_ERR_INVALID, "mc_morton_keys: J=%d outside [2,10]", J);
+  if (n == 0) return HERMES_OK;
+  const int grid = (int)std::min<int64_t>((n + 255) / 256, mc_grid());
+  mc_morton_kernel<<<grid, 256, 0, hermes::as_stream(stream)>>>(centers, n, 1 << J, keys);
+  HERMES_LAUNCH_CHECK("mc_morton_kernel");
+  return HERMES_OK;
 }
 
 extern "C" int hermes_field_to_bricks(const float* field, int J, float* bricks, void* stream) {

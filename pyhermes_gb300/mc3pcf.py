@@ -130,6 +130,11 @@ def rotation_offsets(R1, R2, mu, n_rot, seed_base_rot=-1, mu_index=-1, rng=None)
 def morton_order(centers, L):
     """Permutation putting centres (grid units) in Morton (Z-curve) order of
     their cells, so threads that run together gather nearby cells."""
+    if centers.is_cuda and centers.dtype == torch.float64 and centers.is_contiguous() and 4 <= L <= 1024:
+        keys = torch.empty(centers.shape[0], dtype=torch.int32, device=centers.device)
+        _lib.check(_lib.load().hermes_mc_morton_keys(_ptr(centers), centers.shape[0], int(L).bit_length() - 1, _ptr(keys),
+                                                     _stream_ptr(centers.device)), "hermes_mc_morton_keys")
+        return torch.argsort(keys)
     c = torch.floor(centers).to(torch.int64) & (L - 1)
     key = torch.zeros(c.shape[0], dtype=torch.int64, device=c.device)
     for bit in range(int(L).bit_length() - 1):
