@@ -40,55 +40,23 @@ __device__ __forceinline__ size_t mc_cell(int x, int y, int z, int J) {
   return brick << 3 | (size_t)((x & 1) << 2 | (y & 1) << 1 | (z & 1));
 }
 
-// One axis of the stencil: phi at fraction f + 0, 1, 2 units weights the cells
-// c, c - 1, c - 2 (v2, v1, v0).  Every gather reduces z, then y, then x with
-// this sum, so all layouts give the same bits.
-__device__ __forceinline__ float mc_axis_sum(float v0, float v1, float v2, float p0, float p1, float p2) {
-  return fmaf(p0, v2, fmaf(p1, v1, p2 * v0));
-}
-
-// 27-point interpolation of a float32 field at scaled position (sx, sy, sz),
-// cell by cell.
-template <bool kBricks>
-__device__ __forceinline__ float mc_interp(const float* __restrict__ grid, const float* __restrict__ phis, int res,
-                                           int J, double sx, double sy, double sz) {
-  const int L = 1 << J, m = L - 1;
-  int cx, cy, cz, fx, fy, fz;
-  mc_axis(sx, res, L, cx, fx);
-  mc_axis(sy, res, L, cy, fy);
-  mc_axis(sz, res, L, cz, fz);
-  const float pz0 = phis[fz], pz1 = phis[fz + res], pz2 = phis[fz + 2 * res];
-  const float py0 = phis[fy], py1 = phis[fy + res], py2 = phis[fy + 2 * res];
-  float rx[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    float ry[3];
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      float v[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        v[c] = __ldg(grid + mc_cell<kBricks>((cx - 2 + a) & m, (cy - 2 + b) & m, (cz - 2 + c) & m, J));
-      ry[b] = mc_axis_sum(v[0], v[1], v[2], pz0, pz1, pz2);
-    }
-    rx[a] = mc_axis_sum(ry[0], ry[1], ry[2], py0, py1, py2);
-  }
-  return mc_axis_sum(rx[0], rx[1], rx[2], phis[fx], phis[fx + res], phis[fx + 2 * res]);
-}
-
-// ---- brick-layout gather --------------------------------------------------------
-// A 3 x 3 x 3 stencil lies in exactly 8 bricks.  mc_interp above reads its 27
-// cells one by one: 27 loads per lane, and as many table reads for phi, each of
-// a warp's 32 addresses in another 128-byte line, which is what bounds it
-// (about one line per SM and clock).  Here a lane reads each brick with one
-// 32-byte load, phi from shared memory, and reduces z, y, x in turn.  Of the
-// four cells per axis of the two bricks the stencil's three are picked by
-// selects (a cell outside the stencil never enters a product).
-// 2e5 centres x 100 rotations at J = 9: 2.75 ms (3.03 ms cell by cell), and
-// 1.31 ms with the rotations of a centre side by side (mc_triplet_kernel).
+// phi samples of a block, one 16-byte read per axis (the table in global memory
+// costs one 128-byte line per lane and read).
 struct __align__(16) McPhi {
   float4 p[1024];  // phi at fraction f + 0, 1, 2 units
 };
+
+// The same from the table in global memory: one interpolation a thread does
+// not pay for filling the block's copy (1e6 positions at J = 8: 68 us, 77 us with it).
+struct McPhiGlobal {
+  const float* phis;
+  int res;
+};
+
+__device__ __forceinline__ float4 mc_weights(const McPhi* sp, int f) { return sp->p[f]; }
+__device__ __forceinline__ float4 mc_weights(const McPhiGlobal* g, int f) {
+  return make_float4(__ldg(g->phis + f), __ldg(g->phis + f + g->res), __ldg(g->phis + f + 2 * g->res), 0.f);
+}
 
 __device__ __forceinline__ void mc_load_phi(McPhi* sp, const float* __restrict__ phis, int res) {
   for (int i = threadIdx.x; i < res; i += blockDim.x) sp->p[i] = make_float4(phis[i], phis[i + res], phis[i + 2 * res], 0.f);
@@ -112,6 +80,66 @@ __device__ __forceinline__ void mc_axis_bits(double s, int res, int rl, int L, i
   f = t >= 64 ? 0 : (int)(m >> t) & (res - 1);
 }
 
+// One axis of the stencil: phi at fraction f + 0, 1, 2 units weights the cells
+// c, c - 1, c - 2 (v2, v1, v0).  Every gather reduces z, then y, then x with
+// this sum, so all layouts give the same bits.
+__device__ __forceinline__ float mc_axis_sum(float v0, float v1, float v2, float p0, float p1, float p2) {
+  return fmaf(p0, v2, fmaf(p1, v1, p2 * v0));
+}
+
+// The cells cz - 2, cz - 1, cz of a C-order row that starts on 16 bytes, from
+// the one or two aligned quads that hold them (also across the wrap).
+__device__ __forceinline__ void mc_row_quads(const float* __restrict__ row, int cz, int m, float (&v)[3]) {
+  const int z = (cz - 2) & m, o = z & 3;
+  const float4 a = __ldg(reinterpret_cast<const float4*>(row) + (z >> 2));
+  float4 b = a;
+  if (o > 1) b = __ldg(reinterpret_cast<const float4*>(row) + (cz >> 2));
+  v[0] = o == 0 ? a.x : (o == 1 ? a.y : (o == 2 ? a.z : a.w));
+  v[1] = o == 0 ? a.y : (o == 1 ? a.z : (o == 2 ? a.w : b.x));
+  v[2] = o == 0 ? a.z : (o == 1 ? a.w : (o == 2 ? b.x : b.y));
+}
+
+// 27-point interpolation of a float32 field at scaled position (sx, sy, sz),
+// row by row (kQuads: C order, 16-byte aligned) or cell by cell.
+template <bool kBricks, bool kQuads, class Phi>
+__device__ __forceinline__ float mc_interp(const float* __restrict__ grid, const Phi* sp, int res, int rl, int J,
+                                           double sx, double sy, double sz) {
+  const int L = 1 << J, m = L - 1;
+  int cx, cy, cz, fx, fy, fz;
+  mc_axis_bits(sx, res, rl, L, cx, fx);
+  mc_axis_bits(sy, res, rl, L, cy, fy);
+  mc_axis_bits(sz, res, rl, L, cz, fz);
+  const float4 wx = mc_weights(sp, fx), wy = mc_weights(sp, fy), wz = mc_weights(sp, fz);
+  float rx[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    float ry[3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      float v[3];
+      if (kQuads) {
+        mc_row_quads(grid + mc_cell<false>((cx - 2 + a) & m, (cy - 2 + b) & m, 0, J), cz, m, v);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          v[c] = __ldg(grid + mc_cell<kBricks>((cx - 2 + a) & m, (cy - 2 + b) & m, (cz - 2 + c) & m, J));
+      }
+      ry[b] = mc_axis_sum(v[0], v[1], v[2], wz.x, wz.y, wz.z);
+    }
+    rx[a] = mc_axis_sum(ry[0], ry[1], ry[2], wy.x, wy.y, wy.z);
+  }
+  return mc_axis_sum(rx[0], rx[1], rx[2], wx.x, wx.y, wx.z);
+}
+
+// ---- brick-layout gather --------------------------------------------------------
+// A 3 x 3 x 3 stencil lies in exactly 8 bricks.  mc_interp above reads its 27
+// cells one by one: 27 loads per lane, each of a warp's 32 addresses in another
+// 128-byte line, which is what bounds it (about one line per SM and clock).
+// Here a lane reads each brick with one 32-byte load and reduces z, y, x in
+// turn.  Of the four cells per axis of the two bricks the stencil's three are
+// picked by selects (a cell outside the stencil never enters a product).
+// 2e5 centres x 100 rotations at J = 9: 2.75 ms (3.03 ms cell by cell), and
+// 1.31 ms with the rotations of a centre side by side (mc_triplet_kernel).
 __device__ __forceinline__ void mc_brick(const float* __restrict__ p, float (&v)[8]) {
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
       : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
@@ -159,16 +187,17 @@ __device__ __forceinline__ float mc_interp_bricks(const float* __restrict__ bric
   return mc_reduce3(rx[0], rx[1], rx[2], rx[3], ox, wx);
 }
 
-// Interpolation in the layout of the kernel's fields: C order, bricks cell by
-// cell (fields that are not 32-byte aligned), bricks by whole bricks.
-enum { kCOrder = 0, kBrickCells = 1, kBricks = 2 };
+// Interpolation in the layout of the kernel's fields: C order by quads or (a
+// field that is not 16-byte aligned) by cells, bricks by whole bricks or (not
+// 32-byte aligned) by cells.
+enum { kCOrder = 0, kCells = 1, kBrickCells = 2, kBricks = 3 };
 template <int kLayout>
-__device__ __forceinline__ float mc_value(const float* __restrict__ grid, const float* __restrict__ phis, const McPhi* sp,
-                                          int res, int rl, int J, double sx, double sy, double sz) {
+__device__ __forceinline__ float mc_value(const float* __restrict__ grid, const McPhi* sp, int res, int rl, int J,
+                                          double sx, double sy, double sz) {
   if constexpr (kLayout == kBricks)
     return mc_interp_bricks(grid, sp, res, rl, J, sx, sy, sz);
   else
-    return mc_interp<kLayout == kBrickCells>(grid, phis, res, J, sx, sy, sz);
+    return mc_interp<kLayout == kBrickCells, kLayout == kCOrder>(grid, sp, res, rl, J, sx, sy, sz);
 }
 
 // Morton key (30 bits) of the cell of every centre (grid units).
@@ -192,11 +221,13 @@ __global__ void mc_phi_kernel(const double* __restrict__ phi, int n, float* __re
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = (float)phi[i];
 }
 
-__global__ void mc_interp_kernel(const float* __restrict__ grid, int J, const double* __restrict__ pos, int64_t n,
-                                 const float* __restrict__ phis, int res, double dx, double dy, double dz,
+template <int kLayout>
+__global__ void __launch_bounds__(256) mc_interp_kernel(const float* __restrict__ grid, int J, const double* __restrict__ pos, int64_t n,
+                                 const float* __restrict__ phis, int res, int rl, double dx, double dy, double dz,
                                  double* __restrict__ out) {
+  const McPhiGlobal g = {phis, res};
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = (double)mc_interp<false>(grid, phis, res, J, pos[3 * i] + dx, pos[3 * i + 1] + dy, pos[3 * i + 2] + dz);
+    out[i] = (double)mc_interp<false, kLayout == kCOrder>(grid, &g, res, rl, J, pos[3 * i] + dx, pos[3 * i + 1] + dy, pos[3 * i + 2] + dz);
 }
 
 // sum_i w_i n1_i sum_r n2(x_i + d2_r) n3(x_i + d3_r); n1 = eps1 interpolated
@@ -213,8 +244,8 @@ mc_triplet_kernel(const float* __restrict__ eps1, const float* __restrict__ eps2
                   int J, const double* __restrict__ centers, const double* __restrict__ cw, int64_t nc,
                   const double* __restrict__ offsets, int n_rot, int n_part, const float* __restrict__ phis, int res,
                   int rl, double rho1, double* __restrict__ partial, float* __restrict__ samples) {
-  __shared__ McPhi sphi[1];  // kBricks
-  if (kLayout == kBricks) mc_load_phi(sphi, phis, res);
+  __shared__ McPhi sphi;
+  mc_load_phi(&sphi, phis, res);
   double acc = 0.0;
   const int64_t items = (nc + 31) / 32 * n_part * 32;
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < items; k += (int64_t)gridDim.x * blockDim.x) {
@@ -223,13 +254,13 @@ mc_triplet_kernel(const float* __restrict__ eps1, const float* __restrict__ eps2
     const int64_t i = w32 / n_part * 32 + (k & 31);
     if (i >= nc) continue;
     const double x = centers[3 * i], y = centers[3 * i + 1], z = centers[3 * i + 2];
-    const float n1 = eps1 ? mc_value<kLayout>(eps1, phis, sphi, res, rl, J, x, y, z) : (float)rho1;
+    const float n1 = eps1 ? mc_value<kLayout>(eps1, &sphi, res, rl, J, x, y, z) : (float)rho1;
     const float w = cw ? (float)cw[i] : 1.f;
     float s = 0.f;
     for (int r = part; r < n_rot; r += n_part) {
       const double* o = offsets + 6 * r;
-      const float n2 = mc_value<kLayout>(eps2, phis, sphi, res, rl, J, x + o[0], y + o[1], z + o[2]);
-      const float n3 = mc_value<kLayout>(eps3, phis, sphi, res, rl, J, x + o[3], y + o[4], z + o[5]);
+      const float n2 = mc_value<kLayout>(eps2, &sphi, res, rl, J, x + o[0], y + o[1], z + o[2]);
+      const float n3 = mc_value<kLayout>(eps3, &sphi, res, rl, J, x + o[3], y + o[4], z + o[5]);
       const float f = w * n1 * n2 * n3;
       if (samples) samples[i * n_rot + r] = f;
       s += f;
@@ -310,8 +341,8 @@ mc_sample_kernel(const float* __restrict__ eps1, const float* __restrict__ eps2,
                  const double* __restrict__ w, const double* __restrict__ offsets, long long n, double R1, double R2,
                  double mu, unsigned long long seed, const float* __restrict__ phis, int res, int rl,
                  double* __restrict__ partial) {
-  __shared__ McPhi sphi[1];  // kBricks
-  if (kLayout == kBricks) mc_load_phi(sphi, phis, res);
+  __shared__ McPhi sphi;
+  mc_load_phi(&sphi, phis, res);
   double acc = 0.0, acc2 = 0.0;
   for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
     unsigned long long st = seed ^ ((unsigned long long)k * 0xD1B54A32D192ED03ull);
@@ -332,9 +363,9 @@ mc_sample_kernel(const float* __restrict__ eps1, const float* __restrict__ eps2,
       mc_triangle(R1, R2, mu, a, 2.0 * bb - 1.0, c, o);
     }
     const double x = pool[3 * i], y = pool[3 * i + 1], z = pool[3 * i + 2];
-    const float n1 = mc_value<kLayout>(eps1, phis, sphi, res, rl, J, x, y, z);
-    const float n2 = mc_value<kLayout>(eps2, phis, sphi, res, rl, J, x + o[0], y + o[1], z + o[2]);
-    const float n3 = mc_value<kLayout>(eps3, phis, sphi, res, rl, J, x + o[3], y + o[4], z + o[5]);
+    const float n1 = mc_value<kLayout>(eps1, &sphi, res, rl, J, x, y, z);
+    const float n2 = mc_value<kLayout>(eps2, &sphi, res, rl, J, x + o[0], y + o[1], z + o[2]);
+    const float n3 = mc_value<kLayout>(eps3, &sphi, res, rl, J, x + o[3], y + o[4], z + o[5]);
     double f = (double)(n1 * n2 * n3);
     if (w) f *= w[k];
     acc += f;
@@ -374,8 +405,8 @@ __global__ void mc_to_bricks_kernel(const float* __restrict__ src, int J, float*
   }
 }
 
-bool bricks_aligned(const float* a, const float* b, const float* c) {
-  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 31u) == 0;
+bool aligned(uintptr_t bytes, const float* a, const float* b = nullptr, const float* c = nullptr) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & (bytes - 1)) == 0;
 }
 
 int log2_or_negative(int v) { return (v & (v - 1)) == 0 ? __builtin_ctz((unsigned)v) : -1; }
@@ -424,7 +455,9 @@ extern "C" int hermes_interp(const float* grid, int J, const double* scaled_pos,
   int rc = mc_prepare(phi, n_phi, phi_res, workspace, workspace_bytes, &phis, &partial, s);
   if (rc) return rc;
   if (n == 0) return HERMES_OK;
-  mc_interp_kernel<<<mc_grid(), 256, 0, s>>>(grid, J, scaled_pos, n, phis, phi_res, dx, dy, dz, out);
+  const auto kernel = aligned(16, grid) ? mc_interp_kernel<kCOrder> : mc_interp_kernel<kCells>;
+  kernel<<<mc_grid(), 256, 0, s>>>(grid, J, scaled_pos, n, phis, phi_res, log2_or_negative(phi_res), dx, dy,
+                                   dz, out);
   HERMES_LAUNCH_CHECK("mc_interp_kernel");
   return HERMES_OK;
 }
@@ -448,9 +481,9 @@ static int mc_triplets(const float* eps1, const float* eps2, const float* eps3, 
   // threads in flight over the box
   const int n_part = std::max(1, n_rot / 8);
   const int rl = log2_or_negative(phi_res);
-  const auto kernel = !bricks                               ? mc_triplet_kernel<kCOrder>
-                      : bricks_aligned(eps1, eps2, eps3) ? mc_triplet_kernel<kBricks>
-                                                         : mc_triplet_kernel<kBrickCells>;
+  const bool wide = aligned(bricks ? 32 : 16, eps1, eps2, eps3);
+  const auto kernel = bricks ? (wide ? mc_triplet_kernel<kBricks> : mc_triplet_kernel<kBrickCells>)
+                             : (wide ? mc_triplet_kernel<kCOrder> : mc_triplet_kernel<kCells>);
   kernel<<<g, 256, 0, s>>>(eps1, eps2, eps3, J, centers, center_w, n_centers, offsets, n_rot, n_part, phis, phi_res, rl,
                            rho1, partial, samples_out);
   HERMES_LAUNCH_CHECK("mc_triplet_kernel");
@@ -476,9 +509,9 @@ static int mc_sample(const float* eps1, const float* eps2, const float* eps3, in
   if (rc) return rc;
   const int g = mc_grid();
   const int rl = log2_or_negative(phi_res);
-  const auto kernel = !bricks                               ? mc_sample_kernel<kCOrder>
-                      : bricks_aligned(eps1, eps2, eps3) ? mc_sample_kernel<kBricks>
-                                                         : mc_sample_kernel<kBrickCells>;
+  const bool wide = aligned(bricks ? 32 : 16, eps1, eps2, eps3);
+  const auto kernel = bricks ? (wide ? mc_sample_kernel<kBricks> : mc_sample_kernel<kBrickCells>)
+                             : (wide ? mc_sample_kernel<kCOrder> : mc_sample_kernel<kCells>);
   kernel<<<g, 256, 0, s>>>(eps1, eps2, eps3, J, pool, (long long)M, reinterpret_cast<const long long*>(idx), weights,
                            offsets, (long long)n, R1, R2, mu, (unsigned long long)seed, phis, phi_res, rl, partial);
   HERMES_LAUNCH_CHECK("mc_sample_kernel");

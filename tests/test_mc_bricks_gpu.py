@@ -37,10 +37,14 @@ def test_bricks_give_the_same_bits(J):
     b, sb = mc3pcf.triplet_sum(*f, J, c, off, phi, samples=True, bricks=True)
     assert np.array_equal(sa.cpu().numpy(), sb.cpu().numpy(), equal_nan=True)
     assert bool(torch.isnan(sa).any()) and not bool(torch.isnan(sa).all())
-    # a field that is not 32-byte aligned is read cell by cell
+    # fields that are not 32-byte (bricks) or 16-byte (C order) aligned are read cell by cell
     off1 = torch.empty(8 ** J + 1, device="cuda")[1:].view_as(f[2]).copy_(f[2])
     _, sc = mc3pcf.triplet_sum(f[0], f[1], off1, J, c, off, phi, samples=True, bricks=True)
     assert np.array_equal(sb.cpu().numpy(), sc.cpu().numpy(), equal_nan=True)
+    _, sd = mc3pcf.triplet_sum(f[0], f[1], off1, J, c, off, phi, samples=True, bricks=False)
+    assert np.array_equal(sb.cpu().numpy(), sd.cpu().numpy(), equal_nan=True)
+    p = mc3pcf.interp(f[2], J, c, phi)
+    assert torch.equal(p, mc3pcf.interp(off1, J, c, phi))
 
 
 @pytest.mark.parametrize("nc,n_rot", [(8, 1), (8, 15), (9, 64), (300, 100), (5000, 17)])
