@@ -32,7 +32,6 @@
 #include <map>
 #include <mutex>
 #include <tuple>
-#include <type_traits>
 #include <vector>
 
 #include <cudaTypedefs.h>
@@ -883,8 +882,8 @@ template <int NT>
 constexpr int kHSlot = NT == 1 ? kHPlane : NT * kHTile;  // one plane of all tiles
 }  // namespace hf
 
-// h plane of NT tiles from a staged eps plane, H[tile][col][uy+2][l1z], by the
-// first 64 NT threads, one column each: the weights are then known at compile
+// h plane of NT tiles from a staged eps plane, H[tile][col][uy+2][l1z], one
+// column at a time by 64 threads (NT = 1) or all: the weights are known at compile
 // time (9 of the 15 are not zero) and come from the kernel's parameters, and
 // one warp's instructions cover 32 columns.  The sums are those of
 // ct_compute_h (its terms of weight zero left out).
@@ -892,34 +891,37 @@ template <int NT>
 __device__ __forceinline__ void ct_compute_h_cols(const GammaC& gm, const float* __restrict__ e, float* __restrict__ h) {
   constexpr int EZ = NT * ct::TZ + 2;
   // NT = 1: the two blocks of an SM take warps of different schedulers
-  const int tid = (int)threadIdx.x - (NT == 1 && 2 * blockIdx.x >= gridDim.x ? ct::kCols : 0);
-  if (tid < 0 || tid >= ct::kCols * NT) return;
-  const int tile = tid / ct::kCols, col = tid % ct::kCols;
-  const int cy = col / ct::TZ, cz = tile * ct::TZ + (col & (ct::TZ - 1));
-  float ev[3][3];
+  const int first = (int)threadIdx.x - (NT == 1 && 2 * blockIdx.x >= gridDim.x ? ct::kCols : 0);
+  if (first < 0) return;
+#pragma unroll 1
+  for (int cc = first; cc < ct::kCols * NT; cc += ct::kThreads) {
+    const int tile = cc / ct::kCols, col = cc % ct::kCols;
+    const int cy = col / ct::TZ, cz = tile * ct::TZ + (col & (ct::TZ - 1));
+    float ev[3][3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) ev[i][j] = e[(cy + i) * EZ + cz + j];
-  float* dst = h + (NT == 1 ? 0 : tile * hf::kHTile) + col * hf::kHCol;
+      for (int j = 0; j < 3; ++j) ev[i][j] = e[(cy + i) * EZ + cz + j];
+    float* dst = h + (NT == 1 ? 0 : tile * hf::kHTile) + col * hf::kHCol;
 #pragma unroll
-  for (int ay = 0; ay < 5; ++ay) {
-    float o[3];
+    for (int ay = 0; ay < 5; ++ay) {
+      float o[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      float v = 0.f;
-      bool first = true;
+      for (int j = 0; j < 3; ++j) {
+        float v = 0.f;
+        bool started = false;
 #pragma unroll
-      for (int l1 = 0; l1 < 3; ++l1) {  // weight Gamma[l1][l1 - ay + 2]
-        const int l2 = l1 - ay + 2;
-        if (l2 >= 0 && l2 <= 2) {
-          v = first ? gm.g[l1 * 3 + l2] * ev[l1][j] : fmaf(gm.g[l1 * 3 + l2], ev[l1][j], v);
-          first = false;
+        for (int l1 = 0; l1 < 3; ++l1) {  // weight Gamma[l1][l1 - ay + 2]
+          const int l2 = l1 - ay + 2;
+          if (l2 >= 0 && l2 <= 2) {
+            v = started ? fmaf(gm.g[l1 * 3 + l2], ev[l1][j], v) : gm.g[l1 * 3 + l2] * ev[l1][j];
+            started = true;
+          }
         }
+        o[j] = v;
       }
-      o[j] = v;
+      *reinterpret_cast<float4*>(dst + ay * 4) = make_float4(o[0], o[1], o[2], 0.f);
     }
-    *reinterpret_cast<float4*>(dst + ay * 4) = make_float4(o[0], o[1], o[2], 0.f);
   }
 }
 
@@ -995,11 +997,12 @@ constexpr size_t kSmem = 1024 + 2 * kOpBytes + 2 * kRawBytes + sizeof(float2) * 
                          sizeof(float) * (kRing<NT> * hf::kHSlot<NT> + 2 * ct::EY * (NT * ct::TZ + 2)) +
                          sizeof(double) * 2 * kMaxBins * kMaxBins + 128;
 static_assert(kSmem<8> <= 227 * 1024 && 2 * (kSmem<1> + 1024) <= 228 * 1024, "shared memory of the contraction");
-// Threads of a block: one tile runs as two blocks of 256 threads per SM (2 x 2
-// columns a thread); tiles side by side need their own h planes, so one
-// block of 512 threads (2 x 1 columns a thread) fills the SM.
-template <int NT>
-constexpr int kThr = NT == 1 ? ct::kThreads : 512;
+// Bins (operand slots) of a thread, which then shares each h value between
+// them, and threads of a block (2 x 2 columns a thread).
+template <bool kBM, int NT>
+constexpr int kNbt = kBM && NT == 1 ? 2 : 1;
+template <bool kBM, int NT>
+constexpr int kThr = ct::kThreads / kNbt<kBM, NT>;
 }  // namespace tcc
 
 // (lower half, upper half) -> packed BF16x2, round to nearest even
@@ -1030,6 +1033,17 @@ __device__ __forceinline__ void tc_put_pair(unsigned char* op, int cell, int b, 
   *reinterpret_cast<uint32_t*>(op + tcc::kAtomCol + row + hermes::tc::sw128_offset(r, b >> 2) + byte) = l;
 }
 
+// tc_put_pair of the slots 2 i and 2 i + 1 (8 bytes of each part).
+__device__ __forceinline__ void tc_put_two(unsigned char* op, int cell, int i, float2 a, float2 b) {
+  uint32_t h0, m0, l0, h1, m1, l1;
+  split3(a.x, a.y, h0, m0, l0);
+  split3(b.x, b.y, h1, m1, l1);
+  const uint32_t row = (cell >> 3) * 1024, r = cell & 7, byte = (i & 1) * 8;
+  *reinterpret_cast<uint2*>(op + row + hermes::tc::sw128_offset(r, i >> 1) + byte) = make_uint2(h0, h1);
+  *reinterpret_cast<uint2*>(op + row + hermes::tc::sw128_offset(r, 4 + (i >> 1)) + byte) = make_uint2(m0, m1);
+  *reinterpret_cast<uint2*>(op + tcc::kAtomCol + row + hermes::tc::sw128_offset(r, i >> 1) + byte) = make_uint2(l0, l1);
+}
+
 // a3 planes of bin-major fields (bin b at src3 + b * bstride) -> buf
 // [16 slots][kA3P] float2, slot = tile * (16 / NT) + bin.  The copies are
 // 16 bytes, two cells (2p, 2p + 1) of one row: with z0 a multiple of 8 the
@@ -1039,10 +1053,17 @@ __device__ __forceinline__ void tc_put_pair(unsigned char* op, int cell, int b, 
 // their (y, z) offsets: a thread keeps those of its kN pairs in registers.
 // (One 96-byte bulk copy per row instead was slower, 33.8 against 25.5 ms at
 // J = 9 and 15 bins.)  Slots of bins >= nb3 are zeroed once by the kernel.
+// Place of a slot in the buffer: a thread's two slots 2 i and 2 i + 1 (one tile)
+// are i and i + 8, so that the 16-byte reads of eight lanes still start 4
+// banks apart.
+template <int NT>
+__host__ __device__ constexpr int a3_position(int slot) {
+  return tcc::kNbt<true, NT> == 2 ? (slot >> 1) + 8 * (slot & 1) : slot;
+}
 template <int NT>
 struct A3Copy {
   static constexpr int kPairs = ct::HY * ct::HZ / 2;  // 72
-  static constexpr int kPer = tcc::kThr<NT> / kBinStride, kN = (kPairs + kPer - 1) / kPer;
+  static constexpr int kThr = tcc::kThr<true, NT>, kPer = kThr / kBinStride, kN = (kPairs + kPer - 1) / kPer;
   const float2* src;  // the bin's field
   int off[kN];        // float2 offsets in an x plane
   bool active;        // the slot holds a bin
@@ -1064,7 +1085,7 @@ struct A3Copy {
     if (!active) return;
     const int slot = threadIdx.x / kPer, j = threadIdx.x % kPer;
     const float2* s = src + (long long)(xa & Lm) * L * L;
-    float2* dst = buf + slot * tcc::kA3P + 2 * j;
+    float2* dst = buf + a3_position<NT>(slot) * tcc::kA3P + 2 * j;
 #pragma unroll
     for (int i = 0; i < kN; ++i)
       if ((i + 1) * kPer <= kPairs || j + kPer * i < kPairs) cp_async16(dst + 2 * kPer * i, s + off[i]);
@@ -1083,19 +1104,23 @@ struct A3Copy {
 // not read.  A tile's S goes to A.items, and mp_reduce_items_kernel adds the
 // tiles in the order of the one-tile blocks: the result is the same bits.
 //
-// What bounds it (ncu, J = 8, 15 bins): shared-memory wavefronts 66% of their
-// peak (264 per warp and plane: 120 for the h planes, 72 for a3, 33 for its
-// staging), issue slots 51%, FMA pipe 45%; the FMAs alone would take 9 ms at
-// J = 9.  22.5 ms at J = 9 and 15 bins; 25.5 ms with the a3 addresses computed
-// anew for every plane, the h plane spread over four threads a column and two
-// block barriers a step.
+// What bounds it (ncu, J = 8, 15 bins): the stencil's chain of shared-memory
+// reads and FMAs with eight warps on an SM; shared-memory wavefronts are at 54%
+// of their peak, the FMA pipe at 49% (alone it would take 9 ms at J = 9), issue
+// slots at 43%.  Few wide threads beat many narrow ones: with one bin a thread
+// (256 threads, 128 registers) the h reads alone were 120 of 264 wavefronts a
+// warp and plane, and the wavefronts at 66%.  J = 9, 15 bins: 20.5 ms; 22.2 ms
+// with one bin a thread; 25.5 ms when also the a3 addresses were computed anew
+// for every plane, the h plane was spread over four threads a column and a step
+// had two block barriers.  J = 8, 2 bins in 8 tiles: 0.71 ms with 256 threads of
+// 2 x 2 columns, 0.80 ms with 512 of 2 x 1.
 template <bool kBM, int NT>
-__global__ void __launch_bounds__(tcc::kThr<NT>, NT == 1 ? 2 : 1)
+__global__ void __launch_bounds__(tcc::kThr<kBM, NT>, NT == 1 ? 2 : 1)
 mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map) {
   static_assert(kBM || NT == 1, "tiles side by side read bin-major fields");
   namespace tc = hermes::tc;
-  constexpr int kThr = tcc::kThr<NT>, NBL = kBinStride / NT;
-  constexpr int CZ = NT == 1 ? 2 : 1, NC = 2 * CZ;  // columns of a thread: 2 (y) x CZ (z)
+  constexpr int kThr = tcc::kThr<kBM, NT>, NBL = kBinStride / NT, NBT = tcc::kNbt<kBM, NT>;
+  constexpr int CZ = 2, NC = 2 * CZ;  // columns of a thread: 2 (y) x CZ (z)
   constexpr int kHS = hf::kHSlot<NT>, kEps = ct::EY * (NT * ct::TZ + 2);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* base = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -1116,13 +1141,15 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
 
   const int J = A.J, L = 1 << J, Lm = L - 1, CX = A.CX;
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int b = tid & 15;  // operand slot: bin (NT = 1) or (tile, bin)
-  // column block of this half-warp: the two half-warps of a warp take
-  // blocks 4 cells apart in z, so their rows of the swizzled G operand fall
-  // in complementary halves of the 128-byte rows (no bank conflict)
-  const int hw = (tid >> 4) & 1, wq = tid >> 5;
-  const int cy = NT == 1 ? 2 * (wq >> 1) : 2 * (wq >> 2);
-  const int cz = NT == 1 ? 4 * hw + 2 * (wq & 1) : 4 * hw + (wq & 3);
+  // Threads: 16 / NBT lanes hold the operand slots (NBT b, .. + NBT - 1; a slot is
+  // a bin, or a tile and a bin), the next bits the 2 x 2 column block.  The
+  // blocks of a half-warp (NBT = 2) or of the two half-warps are 4 cells
+  // apart in z, so their rows of the swizzled G operand fall in complementary
+  // halves of the 128-byte rows (no bank conflict).
+  const int b = tid & (kBinStride / NBT - 1);
+  const int hw = NBT == 2 ? (tid >> 3) & 1 : (tid >> 4) & 1, wq = NBT == 2 ? tid >> 4 : tid >> 5;
+  const int cy = 2 * (wq >> 1);
+  const int cz = 4 * hw + 2 * (wq & 1);
   const int nty = L / ct::TY, ntz = L / (NT * ct::TZ);
   auto stage_eps = [&](float* buf, int xe, int y0, int z0) { ct_stage_eps<NT, kThr>(A.eps1, buf, xe, y0, z0, L, Lm); };
   auto compute_h = [&](const float* e, float* h, const float* w) {
@@ -1154,7 +1181,9 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
   for (int i = tid; i < 2 * kMaxBins * kMaxBins; i += kThr) dacc[i] = 0.0;
   if (kBM)
     for (int i = tid; i < 2 * tcc::kA3Buf; i += kThr)
-      if (i % tcc::kA3Buf / tcc::kA3P % NBL >= A.nb3s) abuf[i] = make_float2(0.f, 0.f);
+      if (NBT == 2 ? 2 * (i % tcc::kA3Buf / tcc::kA3P % 8) + i % tcc::kA3Buf / tcc::kA3P / 8 >= A.nb3s
+                   : i % tcc::kA3Buf / tcc::kA3P % NBL >= A.nb3s)
+        abuf[i] = make_float2(0.f, 0.f);
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
@@ -1190,11 +1219,13 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
     compute_h(epsb, hring + 2 * kHS, gsm);
     if (kOneBar) __syncthreads();
 
-    float2 G[5][NC];
+    float2 G[NBT][5][NC];
 #pragma unroll
-    for (int q = 0; q < 5; ++q)
+    for (int u = 0; u < NBT; ++u)
 #pragma unroll
-      for (int c = 0; c < NC; ++c) G[q][c] = make_float2(0.f, 0.f);
+      for (int q = 0; q < 5; ++q)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) G[u][q][c] = make_float2(0.f, 0.f);
     bool first_mma = true;
 
     // The block barrier at the end of a step makes the staged a3 / eps planes
@@ -1237,45 +1268,50 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
         compute_h(epsb + ((st + 1) & 1) * kEps, hring + ((st + 3) & 3) * kHS, gsm);  // h(xa + 3)
       else
         __syncthreads();
-      auto stencil = [&](auto odd_start) {
-        constexpr int kOdd = decltype(odd_start)::value;
+      {
         const float2* ap = abuf + (st & 1) * tcc::kA3Buf;
         const int ht = NT == 1 ? 0 : (b / NBL) * hf::kHTile;
         constexpr int kRing = kOneBar ? 4 : 3;
         const float* hp0 = hring + (st % kRing) * kHS + ht;
         const float* hp1 = hring + ((st + 1) % kRing) * kHS + ht;
         const float* hp2 = hring + ((st + 2) % kRing) * kHS + ht;
-        float2 T[3][NC];
+        float2 T[NBT][3][NC];
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
+        for (int u = 0; u < NBT; ++u)
 #pragma unroll
-          for (int c = 0; c < NC; ++c) T[d][c] = make_float2(0.f, 0.f);
+          for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) T[u][d][c] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int r = 0; r < 6; ++r) {
-          float2 av[6];
-          if (kBM) {  // two cells per 16-byte load (cz - kOdd and kA3P are even)
-            const float4* row4 = reinterpret_cast<const float4*>(ap + b * tcc::kA3P + (cy + r) * ct::HZ + cz - kOdd);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-              const float4 p = row4[k];
-              av[2 * k] = make_float2(p.x, p.y);
-              av[2 * k + 1] = make_float2(p.z, p.w);
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < 6; ++k) av[k] = ap[((cy + r) * ct::HZ + cz + k) * kBinStride + b];
-          }
           // Rz_{l1z}(row, cz + dz) = sum_{l2z} Gamma[l1z][l2z] a3(row, cz + dz + l1z - l2z)
-          float2 rz[CZ][3];
+          float2 rz[NBT][CZ][3];
 #pragma unroll
-          for (int dz = 0; dz < CZ; ++dz)
+          for (int u = 0; u < NBT; ++u) {
+            float2 av[6];
+            if (kBM) {  // two cells per 16-byte load (cz and kA3P are even)
+              const float4* row4 =
+                  reinterpret_cast<const float4*>(ap + (b + 8 * u) * tcc::kA3P + (cy + r) * ct::HZ + cz);
 #pragma unroll
-            for (int l1z = 0; l1z < 3; ++l1z) {
-              const float g0 = A.gm.g[l1z * 3], g1 = A.gm.g[l1z * 3 + 1], g2 = A.gm.g[l1z * 3 + 2];
-              float2 t = __fmul2_rn(make_float2(g2, g2), av[kOdd + dz + l1z]);
-              t = __ffma2_rn(make_float2(g1, g1), av[kOdd + dz + l1z + 1], t);
-              rz[dz][l1z] = __ffma2_rn(make_float2(g0, g0), av[kOdd + dz + l1z + 2], t);
+              for (int k = 0; k < 3; ++k) {
+                const float4 p = row4[k];
+                av[2 * k] = make_float2(p.x, p.y);
+                av[2 * k + 1] = make_float2(p.z, p.w);
+              }
+            } else {
+#pragma unroll
+              for (int k = 0; k < 6; ++k) av[k] = ap[((cy + r) * ct::HZ + cz + k) * kBinStride + b];
             }
+#pragma unroll
+            for (int dz = 0; dz < CZ; ++dz)
+#pragma unroll
+              for (int l1z = 0; l1z < 3; ++l1z) {
+                const float g0 = A.gm.g[l1z * 3], g1 = A.gm.g[l1z * 3 + 1], g2 = A.gm.g[l1z * 3 + 2];
+                float2 t = __fmul2_rn(make_float2(g2, g2), av[dz + l1z]);
+                t = __ffma2_rn(make_float2(g1, g1), av[dz + l1z + 1], t);
+                rz[u][dz][l1z] = __ffma2_rn(make_float2(g0, g0), av[dz + l1z + 2], t);
+              }
+          }
 #pragma unroll
           for (int dy = 0; dy < 2; ++dy) {
             const int uy = r - 2 - dy;
@@ -1286,33 +1322,31 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
 #pragma unroll
               for (int d = 0; d < 3; ++d) {
                 const float4 h4 = *reinterpret_cast<const float4*>((d == 0 ? hp0 : (d == 1 ? hp1 : hp2)) + hoff);
-                float2 t = T[d][dy * CZ + dz];
-                t = __ffma2_rn(make_float2(h4.x, h4.x), rz[dz][0], t);
-                t = __ffma2_rn(make_float2(h4.y, h4.y), rz[dz][1], t);
-                t = __ffma2_rn(make_float2(h4.z, h4.z), rz[dz][2], t);
-                T[d][dy * CZ + dz] = t;
+#pragma unroll
+                for (int u = 0; u < NBT; ++u) {
+                  float2 t = T[u][d][dy * CZ + dz];
+                  t = __ffma2_rn(make_float2(h4.x, h4.x), rz[u][dz][0], t);
+                  t = __ffma2_rn(make_float2(h4.y, h4.y), rz[u][dz][1], t);
+                  t = __ffma2_rn(make_float2(h4.z, h4.z), rz[u][dz][2], t);
+                  T[u][d][dy * CZ + dz] = t;
+                }
               }
             }
           }
         }
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
+        for (int u = 0; u < NBT; ++u)
 #pragma unroll
-          for (int l1x = 0; l1x < 3; ++l1x) {
-            const float gx = A.gm.g[l1x * 3 + d];
+          for (int d = 0; d < 3; ++d)
 #pragma unroll
-            for (int c = 0; c < NC; ++c)
-              G[d - l1x + 2][c] = d - l1x + 2 == 4 ? __fmul2_rn(make_float2(gx, gx), T[d][c])
-                                                   : __ffma2_rn(make_float2(gx, gx), T[d][c], G[d - l1x + 2][c]);
-          }
-      };
-      if constexpr (CZ == 1) {  // a warp's columns all start at an even or all at an odd z
-        if (cz & 1)
-          stencil(std::integral_constant<int, 1>{});
-        else
-          stencil(std::integral_constant<int, 0>{});
-      } else {
-        stencil(std::integral_constant<int, 0>{});
+            for (int l1x = 0; l1x < 3; ++l1x) {
+              const float gx = A.gm.g[l1x * 3 + d];
+#pragma unroll
+              for (int c = 0; c < NC; ++c)
+                G[u][d - l1x + 2][c] =
+                    d - l1x + 2 == 4 ? __fmul2_rn(make_float2(gx, gx), T[u][d][c])
+                                     : __ffma2_rn(make_float2(gx, gx), T[u][d][c], G[u][d - l1x + 2][c]);
+            }
       }
       // G(xa - 2) and the a2 plane xa - 2 become the operands of this plane's MMA
       const bool full = st >= 4;
@@ -1324,16 +1358,24 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
         }
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-          float2 g = G[0][c];
-          if (A.conj_src) g = make_float2(A.sign * g.x, -A.sign * g.y);
-          tc_put_pair(gbf, (cy + c / CZ) * ct::TZ + cz + c % CZ, b, g.x, g.y);
+          float2 g[NBT];
+#pragma unroll
+          for (int u = 0; u < NBT; ++u) {
+            g[u] = G[u][0][c];
+            if (A.conj_src) g[u] = make_float2(A.sign * g[u].x, -A.sign * g[u].y);
+          }
+          const int cell = (cy + c / CZ) * ct::TZ + cz + c % CZ;
+          if constexpr (NBT == 2)
+            tc_put_two(gbf, cell, b, g[0], g[1]);
+          else
+            tc_put_pair(gbf, cell, b, g[0].x, g[0].y);
         }
         // this thread's operand row (cell) and slots kS q .. kS q + kS - 1; with
         // bin-major planes ([slot][cell] in shared memory) a warp takes 32
         // cells of one q
         constexpr int kS = 1024 / kThr;
         const int cell = kBM ? (tid & 63) : (tid >> 2), q = kBM ? (tid >> 6) : (tid & 3);
-        float v[8];
+        float v[2 * kS];
         if (kBM) {
           const uint32_t par = (st & 1) ? tma_ph1 : tma_ph0;
           if (!tc::mbar_wait(&bars[st & 1], par)) *s_abort = 1;  // a2 plane (TMA)
@@ -1362,29 +1404,29 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
           }
         }
         if (st & 1) tma_ph1 ^= (tma_a2 ? 1u : 0u); else tma_ph0 ^= (tma_a2 ? 1u : 0u);
-        uint32_t hv[4], mv[4], lv[4];
+        uint32_t hv[kS], mv[kS], lv[kS];
 #pragma unroll
         for (int i = 0; i < kS; ++i) split3(v[2 * i], v[2 * i + 1], hv[i], mv[i], lv[i]);
         unsigned char* atom = abf + (cell >> 3) * 1024;
-        if constexpr (kS == 4) {
-          // elements 8q .. 8q+7 of the row: chunk q (hi), 4 + q (mid), q of column 1 (lo)
-          *reinterpret_cast<uint4*>(atom + tc::sw128_offset(cell & 7, q)) = make_uint4(hv[0], hv[1], hv[2], hv[3]);
-          *reinterpret_cast<uint4*>(atom + tc::sw128_offset(cell & 7, 4 + q)) = make_uint4(mv[0], mv[1], mv[2], mv[3]);
-          *reinterpret_cast<uint4*>(atom + tcc::kAtomCol + tc::sw128_offset(cell & 7, q)) =
-              make_uint4(lv[0], lv[1], lv[2], lv[3]);
-        } else {  // elements 4q .. 4q+3: half (q & 1) of the chunks of q / 2
-          const uint32_t half = (q & 1) * 8;
-          *reinterpret_cast<uint2*>(atom + tc::sw128_offset(cell & 7, q >> 1) + half) = make_uint2(hv[0], hv[1]);
-          *reinterpret_cast<uint2*>(atom + tc::sw128_offset(cell & 7, 4 + (q >> 1)) + half) = make_uint2(mv[0], mv[1]);
-          *reinterpret_cast<uint2*>(atom + tcc::kAtomCol + tc::sw128_offset(cell & 7, q >> 1) + half) =
-              make_uint2(lv[0], lv[1]);
+        // elements 8k .. 8k+7 of the row, k = kS q / 4 + j: chunk k (hi), 4 + k (mid), k of column 1 (lo)
+#pragma unroll
+        for (int j = 0; j < kS / 4; ++j) {
+          const int k = kS / 4 * q + j;
+          *reinterpret_cast<uint4*>(atom + tc::sw128_offset(cell & 7, k)) =
+              make_uint4(hv[4 * j], hv[4 * j + 1], hv[4 * j + 2], hv[4 * j + 3]);
+          *reinterpret_cast<uint4*>(atom + tc::sw128_offset(cell & 7, 4 + k)) =
+              make_uint4(mv[4 * j], mv[4 * j + 1], mv[4 * j + 2], mv[4 * j + 3]);
+          *reinterpret_cast<uint4*>(atom + tcc::kAtomCol + tc::sw128_offset(cell & 7, k)) =
+              make_uint4(lv[4 * j], lv[4 * j + 1], lv[4 * j + 2], lv[4 * j + 3]);
         }
         tc::fence_proxy_async_smem();
       }
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+      for (int u = 0; u < NBT; ++u)
 #pragma unroll
-        for (int c = 0; c < NC; ++c) G[q][c] = G[q + 1][c];
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int c = 0; c < NC; ++c) G[u][q][c] = G[u][q + 1][c];
       cp_async_wait<0>();
       __syncthreads();
       if (*s_abort) break;
@@ -1433,8 +1475,8 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
     }
     tc::tc_fence_before();
     __syncthreads();
-    if (kThr == 256 || tid < 256) {
-      const int b2 = tid >> 4, b3 = tid & 15;
+    for (int i = tid; i < kMaxBins * kMaxBins; i += kThr) {
+      const int b2 = i >> 4, b3 = i & 15;
       double sr = 0.0, si = 0.0;
 #pragma unroll
       for (int sp = 0; sp < 3; ++sp) {
@@ -1996,11 +2038,11 @@ enum { kEngineTensor = 0, kEngineSimt = 1, kEngineTensorBinMajor = 2 };
 // Tiles side by side in the tensor-core contraction of nb bins (1, 2, 4 or
 // 8, with 16 / tiles >= nb bin slots each): the count with the least work,
 // rounds of items times the cost of a round.  Two blocks of one tile share an
-// SM, and their round of 132 planes takes 0.42 ms; a block of 2, 4 or 8 tiles
-// has the SM to itself and takes 0.30, 0.32 and 0.40 ms.  At J = 8, 2 bins take
-// 0.80 ms with 8 tiles, 2.93 ms with one.
+// SM, and their round of 132 planes takes 0.38 ms; a block of 2, 4 or 8 tiles
+// has the SM to itself and takes 0.26, 0.29 and 0.36 ms.  At J = 8, 2 bins take
+// 0.71 ms with 8 tiles, 2.67 ms with one.
 static int contract_tiles(int nb, int per_tile, int L, int ctas_per_sm, int nsm) {
-  const double round[4] = {0.21 * ctas_per_sm, 0.30, 0.32, 0.40};
+  const double round[4] = {0.19 * ctas_per_sm, 0.26, 0.29, 0.36};
   int best = 1;
   double cost = 1e30;
   for (int k = 0, t = 1; k < 4 && (t == 1 || (t * nb <= kBinStride && t * ct::TZ <= L)); ++k, t *= 2) {
@@ -2106,7 +2148,8 @@ static int mp_contract_launch(const float* eps1, const void* fields2, int nb2, c
     }
     HERMES_CUDA_TRY(cudaMemsetAsync(w.status, 0, sizeof(int), s));
     void* args[] = {&A, &map};
-    HERMES_CUDA_TRY(cudaLaunchKernel(fn, dim3(nblk), dim3(tiles > 1 ? 512 : ct::kThreads), args, smem, s));
+    HERMES_CUDA_TRY(cudaLaunchKernel(fn, dim3(nblk),
+                                     dim3(engine == kEngineTensorBinMajor && tiles == 1 ? tcc::kThr<true, 1> : ct::kThreads), args, smem, s));
     HERMES_LAUNCH_CHECK("mp_contract_tc_kernel");
   } else {
     mp_contract_kernel<<<nblk, ct::kThreads, ct::kSmem, s>>>(A);
