@@ -19,6 +19,7 @@
 // first pass of its inverse are one pass (kFused): a thread's eight outputs of
 // the forward transform, x[n1 + 64 n2], n2 = 0..7, are its eight inputs of
 // the inverse one.
+#include "fft_device.cuh"
 #include "fft_lines.cuh"
 #include "hermes_common.cuh"
 
@@ -28,37 +29,6 @@ namespace {
 enum { kInverse = 0, kForward = 1, kFused = 2 };
 constexpr int kLen = 512;
 constexpr int kPitch = kLen + 1;  // float2 per column in shared memory (odd: conflict-free columns)
-
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-
-// a[k] <- sum_n a[n] e^{+2 pi i n k / 8}: two 4-point transforms of the
-// even and odd inputs, combined with e^{+i pi k / 4}.
-__device__ __forceinline__ void idft8(float2 (&a)[8]) {
-  constexpr float r = 0.70710678118654752f;  // 1/sqrt(2)
-  const float2 b0 = make_float2(a[0].x + a[4].x, a[0].y + a[4].y), b1 = make_float2(a[0].x - a[4].x, a[0].y - a[4].y);
-  const float2 b2 = make_float2(a[2].x + a[6].x, a[2].y + a[6].y), b3 = make_float2(a[2].x - a[6].x, a[2].y - a[6].y);
-  const float2 b4 = make_float2(a[1].x + a[5].x, a[1].y + a[5].y), b5 = make_float2(a[1].x - a[5].x, a[1].y - a[5].y);
-  const float2 b6 = make_float2(a[3].x + a[7].x, a[3].y + a[7].y), b7 = make_float2(a[3].x - a[7].x, a[3].y - a[7].y);
-  // even part E[k] and odd part O[k], k = 0..3 (i b = (-b.y, b.x))
-  const float2 e0 = make_float2(b0.x + b2.x, b0.y + b2.y), e2 = make_float2(b0.x - b2.x, b0.y - b2.y);
-  const float2 e1 = make_float2(b1.x - b3.y, b1.y + b3.x), e3 = make_float2(b1.x + b3.y, b1.y - b3.x);
-  const float2 o0 = make_float2(b4.x + b6.x, b4.y + b6.y), o2 = make_float2(b4.x - b6.x, b4.y - b6.y);
-  const float2 o1 = make_float2(b5.x - b7.y, b5.y + b7.x), o3 = make_float2(b5.x + b7.y, b5.y - b7.x);
-  // w^k O[k], w = e^{+i pi / 4}
-  const float2 t1 = make_float2((o1.x - o1.y) * r, (o1.x + o1.y) * r);
-  const float2 t2 = make_float2(-o2.y, o2.x);
-  const float2 t3 = make_float2(-(o3.x + o3.y) * r, (o3.x - o3.y) * r);
-  a[0] = make_float2(e0.x + o0.x, e0.y + o0.y);
-  a[4] = make_float2(e0.x - o0.x, e0.y - o0.y);
-  a[1] = make_float2(e1.x + t1.x, e1.y + t1.y);
-  a[5] = make_float2(e1.x - t1.x, e1.y - t1.y);
-  a[2] = make_float2(e2.x + t2.x, e2.y + t2.y);
-  a[6] = make_float2(e2.x - t2.x, e2.y - t2.y);
-  a[3] = make_float2(e3.x + t3.x, e3.y + t3.y);
-  a[7] = make_float2(e3.x - t3.x, e3.y - t3.y);
-}
 
 // 16-byte asynchronous global -> shared copy (L2 only) and its group fences
 __device__ __forceinline__ void cp_async16_cg(void* dst, const void* src) {
@@ -151,22 +121,7 @@ fft512_cols_kernel(float2* __restrict__ data, int nf, int axis, FftWindow win) {
   extern __shared__ __align__(16) float2 sm[];
   float2* tw = sm + 3 * kBuf;
   float* G = reinterpret_cast<float*>(tw + kLen);  // gaussian window factors (kFused)
-  // e^{2 pi i j / 512}: the first octant in float64 (slow on this part: 512
-  // evaluations cost as much as two tiles), the others are its reflections
-  for (int j = threadIdx.x; j <= kLen / 8; j += T) {
-    double sd, cd;
-    sincospi((double)j / 256.0, &sd, &cd);
-    const float sn = (float)sd, cs = (float)cd;
-    const int q = kLen / 4;  // a quarter turn
-    tw[j] = make_float2(cs, sn);
-    tw[q - j] = make_float2(sn, cs);
-    tw[q + j] = make_float2(-sn, cs);
-    tw[2 * q - j] = make_float2(-cs, sn);
-    tw[2 * q + j] = make_float2(-cs, -sn);
-    tw[3 * q - j] = make_float2(-sn, -cs);
-    tw[3 * q + j] = make_float2(sn, -cs);
-    if (j > 0) tw[4 * q - j] = make_float2(cs, -sn);
-  }
+  fill_twiddles<kLen>(tw, T);
   if (kMode == kFused && win.axis_factor)
     for (int j = threadIdx.x; j < kLen; j += T) G[j] = win.axis_factor[j];
   const long long L = kLen, L2 = L * kRow, L3 = L2 * L;
@@ -290,6 +245,76 @@ fft512_cols_kernel(float2* __restrict__ data, int nf, int axis, FftWindow win) {
   cp_async_wait_group<0>();  // no copy outlives the kernel
 }
 
+// The strided pass of L = 128 and 256: tiles of 16 columns as above, one
+// eight-point transform a thread (line_ifft's stages, its buffer per column
+// with an odd pitch), two blocks an SM.
+template <int L>
+__global__ void __launch_bounds__(2 * L, 2)
+fft_cols_kernel(float2* __restrict__ data, int nf, int axis) {
+  constexpr int C = kCols, T = 2 * L, PT = L / 8, R = L / 64, kCol = 9 * PT + 1, kTile = C * kCol;
+  extern __shared__ __align__(16) float2 sm[];
+  float2* tw = sm + 3 * kTile;
+  fill_twiddles<L>(tw, T);
+  const int astride = axis == 1 ? L * L : L, rstride = axis == 1 ? L : L * L;
+  const int ntiles = nf * L * (L / C);
+  auto tile_ptr = [&](int t) {
+    const int zb = t % (L / C), fa = t / (L / C);
+    return data + (long long)(fa / L) * (L * L * L) + (fa % L) * astride + zb * C;
+  };
+  auto prefetch = [&](int t, float2* buf) {
+    if (t < ntiles) {
+      const float2* g = tile_ptr(t);
+#pragma unroll
+      for (int q = 0; q < 8 * L / T; ++q) {
+        const int j = threadIdx.x + T * q, row = j >> 3, part = j & 7;
+        cp_async16_cg(buf + row * C + 2 * part, g + row * rstride + 2 * part);
+      }
+    }
+    cp_async_commit();
+  };
+  auto sync = [] { __syncthreads(); };
+  const int c = threadIdx.x % C, n1 = threadIdx.x / C;
+  int t = blockIdx.x;
+  prefetch(t, sm);
+  prefetch(t + gridDim.x, sm + kTile);
+  for (int k = 0; t < ntiles; t += gridDim.x, ++k) {
+    float2* buf = sm + (k % 3) * kTile;
+    cp_async_wait_group<1>();
+    __syncthreads();
+    float2 v[8];
+#pragma unroll
+    for (int n2 = 0; n2 < 8; ++n2) v[n2] = buf[(n1 + PT * n2) * C + c];
+    prefetch(t + 2 * gridDim.x, sm + ((k + 2) % 3) * kTile);
+    __syncthreads();
+    line_ifft<L>(v, buf + c * kCol, tw, n1, sync);
+    float2* g = tile_ptr(t) + c;
+#pragma unroll
+    for (int i = 0; i < 8 / R; ++i)
+#pragma unroll
+      for (int q = 0; q < R; ++q) g[(n1 + PT * i + 64 * q) * rstride] = v[R * i + q];
+    __syncthreads();  // buffer free: the next iteration prefetches into it
+  }
+  cp_async_wait_group<0>();
+}
+
+template <int L>
+int launch_fft_cols(float2* data, int nf, int axis, cudaStream_t s) {
+  constexpr size_t smem = sizeof(float2) * (3 * (size_t)kCols * (9 * L / 8 + 1) + L);
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  HERMES_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || !attr_set[dev]) {  // once per device, before any stream capture
+    HERMES_CUDA_TRY(cudaFuncSetAttribute(fft_cols_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (dev >= 0 && dev < 64) attr_set[dev] = true;
+  }
+  int nsm = 0;
+  HERMES_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const int ntiles = nf * L * (L / kCols), per_sm = L == 128 ? 4 : 2;
+  fft_cols_kernel<L><<<ntiles < nsm * per_sm ? ntiles : nsm * per_sm, 2 * L, smem, s>>>(data, nf, axis);
+  HERMES_LAUNCH_CHECK("fft_cols_kernel");
+  return HERMES_OK;
+}
+
 template <int kMode, bool kHalf>
 int launch_cols(float2* data, int nf, int axis, const FftWindow& win, cudaStream_t s) {
   constexpr size_t smem = sizeof(float2) * (3 * (size_t)kBuf + kLen) + (kMode == kFused ? sizeof(float) * kLen : 0);
@@ -314,6 +339,13 @@ int launch_cols(float2* data, int nf, int axis, const FftWindow& win, cudaStream
 // axis 0: x, axis 1: y.
 int fft512_strided_inverse(float2* data, int nf, int axis, cudaStream_t s) {
   return launch_cols<kInverse, false>(data, nf, axis, FftWindow{}, s);
+}
+
+int fft_strided_inverse(float2* data, int J, int nf, int axis, cudaStream_t s) {
+  if (J == 9) return fft512_strided_inverse(data, nf, axis, s);
+  if (J == 8) return launch_fft_cols<256>(data, nf, axis, s);
+  if (J == 7) return launch_fft_cols<128>(data, nf, axis, s);
+  return fail(HERMES_ERR_UNSUPPORTED, "fft_strided_inverse: J=%d", J);
 }
 
 int fft512_half_y(float2* data, bool forward, cudaStream_t s) {

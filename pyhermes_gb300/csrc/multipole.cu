@@ -36,14 +36,14 @@
 
 #include <cudaTypedefs.h>
 
+#include "fft_device.cuh"
 #include "hermes_common.cuh"
 #include "tc_common.cuh"
 #include "window_eval.cuh"
 
 namespace hermes {
 int get_plan_c2c_batch(int J, int batch, cufftHandle* out);
-int get_plan_c2c_lines(int J, int fields, cufftHandle* out);
-int fft512_strided_inverse(float2* data, int nf, int axis, cudaStream_t s);
+int fft_strided_inverse(float2* data, int J, int nf, int axis, cudaStream_t s);
 int prepare_window(const hermes_window_t& in, int L, WinDev* out);
 }
 
@@ -111,8 +111,10 @@ __device__ float sph_jl_f32(int l, float xh, float xl) {
   return jc;
 }
 
-// T[n2 * kBinStride + b] = j_l(2 pi sqrt(n2) R_b / L), n2 = 0 .. n2max (rows
-// padded to 16 floats so one image's bins are four float4 loads).
+// T[n2 * ts + b] = j_l(2 pi sqrt(n2) R_b / L), n2 = 0 .. n2max.  Rows of ts = 4, 8
+// or 16 floats for up to that many bins (an image's bins are ts / 4 float4
+// loads): with few bins the table is 4 times smaller and its threads are not
+// idle (2 bins at J = 8: 0.010 ms, 0.046 with rows of 16).
 struct RhoArgs {
   float v[2 * kMaxBins];  // R_b / L as double-float (hi, lo) pairs
 };
@@ -120,11 +122,11 @@ struct RhoArgs {
 // Radii travel as a kernel argument (no host-to-device copy), so the fields
 // call can be captured into a CUDA graph.
 __global__ void mp_jl_table_kernel(float* __restrict__ T, int n2max, RhoArgs rho,
-                                   int nb, int l) {
-  const long long total = (long long)(n2max + 1) * kBinStride;
+                                   int nb, int l, int ts) {
+  const long long total = (long long)(n2max + 1) * ts;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
-    const int n2 = (int)(i / kBinStride), b = (int)(i % kBinStride);
+    const int n2 = (int)(i / ts), b = (int)(i % ts);
     if (b >= nb) {
       T[i] = 0.f;
       continue;
@@ -136,21 +138,21 @@ __global__ void mp_jl_table_kernel(float* __restrict__ T, int n2max, RhoArgs rho
   }
 }
 
-// T[n2 * 16 + b] = U_b(|k|) for isotropic window transfers (sphere, gaussian,
+// T[n2 * ts + b] = U_b(|k|) for isotropic window transfers (sphere, gaussian,
 // shell, thick_shell, gaussian_shell; the analytic monopole profiles of
 // radial_multipole_windows.py:60-128), k = sqrt(n2) / L.  The window
 // descriptors are staged in shared memory.
 struct IsoWins {
   hermes::WinDev w[kMaxBins];
 };
-__global__ void mp_iso_table_kernel(float* __restrict__ T, int n2max, IsoWins wins, int nb) {
+__global__ void mp_iso_table_kernel(float* __restrict__ T, int n2max, IsoWins wins, int nb, int ts) {
   __shared__ hermes::WinDev sw[kMaxBins];
   if (threadIdx.x < kMaxBins) sw[threadIdx.x] = wins.w[threadIdx.x];
   __syncthreads();
-  const long long total = (long long)(n2max + 1) * kBinStride;
+  const long long total = (long long)(n2max + 1) * ts;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
-    const int n2 = (int)(i / kBinStride), b = (int)(i % kBinStride);
+    const int n2 = (int)(i / ts), b = (int)(i % ts);
     float v = 0.f;
     if (b < nb) {
       bool ok;
@@ -161,7 +163,7 @@ __global__ void mp_iso_table_kernel(float* __restrict__ T, int n2max, IsoWins wi
   }
 }
 
-// T[n2 * 16 + b] = U_b(k) from uniform tables over k in [0, kmax_b] (n_b
+// T[n2 * ts + b] = U_b(k) from uniform tables over k in [0, kmax_b] (n_b
 // points; physical k = sqrt(n2) * k_scale), with the local cubic of
 // radial_multipole_windows.py:186-210 (linear in the first and last
 // interval, clamped outside), float64.
@@ -172,7 +174,7 @@ struct TabArgs {
   double k_scale;  // grid_to_physical / L
 };
 __global__ void mp_tab_table_kernel(float* __restrict__ T, int n2max, const double* __restrict__ tables, TabArgs ta,
-                                    int nb) {
+                                    int nb, int ts) {
   __shared__ long long soff[kMaxBins];
   __shared__ int sn[kMaxBins];
   __shared__ double skm[kMaxBins];
@@ -182,10 +184,10 @@ __global__ void mp_tab_table_kernel(float* __restrict__ T, int n2max, const doub
     skm[threadIdx.x] = ta.kmax[threadIdx.x];
   }
   __syncthreads();
-  const long long total = (long long)(n2max + 1) * kBinStride;
+  const long long total = (long long)(n2max + 1) * ts;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
-    const int n2 = (int)(i / kBinStride), b = (int)(i % kBinStride);
+    const int n2 = (int)(i / ts), b = (int)(i % ts);
     double v = 0.0;
     if (b < nb) {
       const double* t = tables + soff[b];
@@ -305,9 +307,9 @@ __device__ __forceinline__ void mp_window_sum(int x, int y, int z, int L, const 
         const float pw = pa[i] * pb[j] * pc[k];
         const float2 yv = kPair ? ylm_pair_at(Y, ic[k], n2) : ylm_at(Y, ia[i], ib[j], ic[k], n2);
         const float2 yw = make_float2(pw * yv.x, pw * yv.y);  // (Re, Im) of P Y, one paired FMA per bin
-        const float4* tr = T4 + (long long)n2 * (kBinStride / 4);
+        const float4* tr = T4 + (long long)n2 * NB4;
         if (kPair) {
-          const float4* trb = T4b + (long long)n2 * (kBinStride / 4);
+          const float4* trb = T4b + (long long)n2 * NB4;
 #pragma unroll
           for (int q = 0; q < NB4; ++q) {
             const float4 ja = __ldg(tr + q), jb = __ldg(trb + q);
@@ -428,6 +430,8 @@ mp_prepass_quad_kernel(const float2* __restrict__ half, int J, const float* __re
   }
 }
 
+__device__ __forceinline__ void mp_edge_line(int bi, int L, int& x, int& y);
+
 // Edge lines, x in {0, L/2} or y in {0, L/2} (4L - 4 lines): one thread per
 // half-spectrum mode, which also writes its inversion when z is not 0 or
 // L/2, evaluating it on the x = 0 and y = 0 lines.
@@ -445,15 +449,7 @@ mp_prepass_edge_kernel(const float2* __restrict__ half, int J, const float* __re
        w += (long long)gridDim.x * blockDim.x) {
     const int z = (int)(w % H), bi = (int)(w / H);
     int x, y;
-    if (bi < 2 * L) {  // x in {0, L/2}, any y
-      x = bi < L ? 0 : L / 2;
-      y = bi & Lm;
-    } else {           // y in {0, L/2}, x not in {0, L/2}
-      const int t = bi - 2 * L;
-      y = t < L - 2 ? 0 : L / 2;
-      x = (t < L - 2 ? t : t - (L - 2)) + 1;
-      if (x >= L / 2) ++x;
-    }
+    mp_edge_line(bi, L, x, y);
     const float2 e = half[((long long)x * L + y) * H + z];
     float2 acc[NB];
     mp_window_sum<NB4, kPair>(x, y, z, L, P, T4, T4b, Y, acc);
@@ -497,6 +493,153 @@ mp_prepass_edge_kernel(const float2* __restrict__ half, int J, const float* __re
         }
       }
     }
+  }
+}
+
+// (x, y) of edge line bi of the 4 L - 4 lines with x or y in {0, L/2}.
+__device__ __forceinline__ void mp_edge_line(int bi, int L, int& x, int& y) {
+  if (bi < 2 * L) {  // x in {0, L/2}, any y
+    x = bi < L ? 0 : L / 2;
+    y = bi & (L - 1);
+  } else {           // y in {0, L/2}, x not in {0, L/2}
+    const int t = bi - 2 * L;
+    y = t < L - 2 ? 0 : L / 2;
+    x = (t < L - 2 ? t : t - (L - 2)) + 1;
+    if (x >= L / 2) ++x;
+  }
+}
+
+// ---- prepass and inverse z transform in one pass ------------------------------
+// mp_prepass_quad_kernel writes the spectra and the z transform reads them back:
+// 32 GB of the 107 GB that the fields of 15 bins moved at J = 9.  Here a block
+// takes the four reflected lines (x, y), (L-x, y), (x, L-y), (L-x, L-y) of an
+// interior (x, y): thread z evaluates the window once (z = 0 .. L/2, all bins)
+// into shared memory, then each line's L / 8 threads form its values in
+// registers (those beyond L/2 are the inversions of line 3 - a), transform them
+// (line_ifft) and write the line, bin after bin.  The values are those of the
+// prepass.  The last warp only evaluates z = L/2.  15 bins at J = 9: 6.7 ms, 9.6 ms
+// in two passes (2.4 ms is the write alone); 2 bins at J = 8: 0.15 ms, 0.20 in two.
+template <int L, int NB4>
+struct LinesSmem {
+  static constexpr int H = L / 2 + 1, NB = 4 * NB4;
+  float2 k[NB][H];          // window of the interior (x, y)
+  float2 e[4][H];           // eps_hat / L^3 of the four lines
+  float2 buf[4][9 * L / 8];
+  float2 tw[L];
+};
+
+template <int L>
+struct LineSync {  // of the L / 8 threads of a line
+  int id;
+  __device__ __forceinline__ void operator()() const {
+    if constexpr (L / 8 > 32)
+      asm volatile("bar.sync %0, %1;\n" ::"r"(id + 1), "n"(L / 8) : "memory");
+    else
+      __syncwarp(L / 8 == 32 ? 0xffffffffu : 0xffffu << (threadIdx.x & 16));
+  }
+};
+
+// resident blocks: registers for the window sums of many bins, warps else
+constexpr int lines_blocks(int L, int nb4, bool pair) {
+  return L == 512 ? (nb4 < 4 ? (pair ? 3 : 4) : (pair ? 2 : 3)) : (L == 256 ? (nb4 == 4 ? 4 : 7) : (nb4 == 4 ? 7 : 10));
+}
+template <int L, int NB4, bool kPair>
+__global__ void __launch_bounds__(L / 2 + 32, lines_blocks(L, NB4, kPair))
+mp_lines_quad_kernel(const float2* __restrict__ half, const float* __restrict__ P, const float4* __restrict__ T4,
+                     const float4* __restrict__ T4b, YlmConst Y, int nb, float2* __restrict__ out, float inv_n) {
+  using S = LinesSmem<L, NB4>;
+  constexpr int H = S::H, NB = S::NB, Q1 = L / 2 - 1, PT = L / 8;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  S& sm = *reinterpret_cast<S*>(smem_raw);
+  const long long N = (long long)L * L * L;
+  const int tid = threadIdx.x;
+  hermes::fill_twiddles<L>(sm.tw, blockDim.x);
+  const int a = tid / PT, t = tid % PT;  // line and place in it (tid < L / 2)
+  const LineSync<L> sync{a};
+  const float lsign = (Y.l & 1) ? -1.f : 1.f, msign = (Y.m & 1) ? -1.f : 1.f;
+  // K of line a is cr (Re K + i sg Im K); line 3 - a has the same sg
+  const float sg = (a == 1 || a == 2) ? -1.f : 1.f;
+  const float cr = (a & 1) ? msign : 1.f, crm = lsign * ((a & 1) ? 1.f : msign);
+  for (int li = blockIdx.x; li < Q1 * Q1; li += gridDim.x) {
+    const int x = 1 + li / Q1, y = 1 + li % Q1;
+    __syncthreads();  // the previous quad's window has been read
+    if (tid < H) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int xq = (q & 1) ? L - x : x, yq = (q & 2) ? L - y : y;
+        const float2 e = half[(xq * L + yq) * (long long)H + tid];
+        sm.e[q][tid] = make_float2(e.x * inv_n, e.y * inv_n);
+      }
+      float2 acc[NB];
+      mp_window_sum<NB4, kPair>(x, y, tid, L, P, T4, T4b, Y, acc);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) sm.k[b][tid] = acc[b];
+    }
+    __syncthreads();
+    if (tid >= L / 2) continue;
+    float2 ev[8];
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      const int z = t + PT * n;
+      if (z <= L / 2) {
+        const float2 e = sm.e[a][z];
+        ev[n] = kPair ? e : make_float2(cr * e.x, cr * e.y);
+      } else {
+        const float2 e = sm.e[3 - a][L - z];
+        ev[n] = kPair ? make_float2(e.x, -e.y) : make_float2(crm * e.x, -(crm * e.y));
+      }
+    }
+    const int xa = (a & 1) ? L - x : x, ya = (a & 2) ? L - y : y;
+    float2* line = out + (long long)(xa * L + ya) * L;
+    for (int b = 0; b < nb; ++b) {
+      float2 v[8];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        const int z = t + PT * n;
+        const float2 k = sm.k[b][z <= L / 2 ? z : L - z];
+        if (kPair) {
+          const float kk = z <= L / 2 ? k.x + k.y : k.x - k.y;
+          v[n] = make_float2(ev[n].x * kk, ev[n].y * kk);
+        } else {
+          const float ki = sg * k.y;
+          v[n] = make_float2(ev[n].x * k.x - ev[n].y * ki, ev[n].x * ki + ev[n].y * k.x);
+        }
+      }
+      hermes::line_ifft<L>(v, sm.buf[a], sm.tw, t, sync);
+      float2* o = line + b * N;
+      constexpr int R = L / 64;
+#pragma unroll
+      for (int i = 0; i < 8 / R; ++i)
+#pragma unroll
+        for (int q = 0; q < R; ++q) o[t + PT * i + 64 * q] = v[R * i + q];
+      sync();  // buf free
+    }
+  }
+}
+
+// The z transform of the edge lines (in place), one line per L / 8 threads.
+template <int L>
+__global__ void __launch_bounds__(256) mp_lines_edge_kernel(float2* __restrict__ out, int nb) {
+  constexpr int PT = L / 8, G = 256 / PT, R = L / 64;
+  __shared__ float2 buf[G][9 * PT];
+  __shared__ float2 tw[L];
+  hermes::fill_twiddles<L>(tw, blockDim.x);
+  __syncthreads();
+  const int g = threadIdx.x / PT, t = threadIdx.x % PT;
+  const LineSync<L> sync{g};
+  for (int i = blockIdx.x * G + g; i < (4 * L - 4) * nb; i += gridDim.x * G) {
+    int x, y;
+    mp_edge_line(i % (4 * L - 4), L, x, y);
+    float2* line = out + (long long)(i / (4 * L - 4)) * L * L * L + (long long)(x * L + y) * L;
+    float2 v[8];
+#pragma unroll
+    for (int n = 0; n < 8; ++n) v[n] = line[t + PT * n];
+    hermes::line_ifft<L>(v, buf[g], tw, t, sync);
+#pragma unroll
+    for (int k = 0; k < 8 / R; ++k)
+#pragma unroll
+      for (int q = 0; q < R; ++q) line[t + PT * k + 64 * q] = v[R * k + q];
+    sync();
   }
 }
 
@@ -1685,6 +1828,9 @@ YlmConst make_ylm_pair(int l) {
 // outnumber the blocks), else min(64, L).
 int default_chunk(int L) { return L >= 256 ? 128 : (L < ct::kMaxCX ? L : ct::kMaxCX); }
 
+// floats per row of the radial tables (the prepass's 4 * NB4)
+int table_stride(int nb) { return nb <= 4 ? 4 : (nb <= 8 ? 8 : kBinStride); }
+
 size_t table_floats(int J) {
   const long long L = 1LL << J;
   return (size_t)(3 * L * L + 1) * kBinStride;
@@ -1784,11 +1930,33 @@ int fields_setup(const void* half_spec, int J, int l, int m, int nb, const doubl
   return HERMES_OK;
 }
 
-// Inverse 3-D FFT of the fields: 0 = cuFFT's 3-D plan; 1 (default) = at
-// J = 9, cuFFT's 1-D z lines (contiguous, near HBM speed) then
-// fft512_strided_inverse over y and x in place of cuFFT's strided passes
-// (15 fields: 19.95 ms per fields call against 25.7 ms).
+// Inverse 3-D FFT of the fields: 0 = cuFFT's 3-D plan; 1 (default) = at J = 7, 8
+// and 9, the z transform in the prepass, then fft_strided_inverse over y and x.
+// 15 fields at J = 9: 17.1 ms per fields call, 19.9 ms with cuFFT's z lines after
+// the prepass, 25.7 ms with its plan; 15 at J = 8 2.2 ms (plan 2.65), 10 at J = 7
+// 0.24 ms (plan 0.28).  Below J = 7 a field fits L2 and launches dominate; at
+// J = 10 the line does not split into 8 * 8 * R.
 std::atomic<int> g_fft_mode{1};
+
+template <int L, int NB4, bool kPair>
+int launch_lines_quad(const float2* half, const float* P, const float4* T4, const float4* T4b, const YlmConst& Y, int nb,
+                      float2* out, float inv_n, int nsm, cudaStream_t s) {
+  const auto fn = mp_lines_quad_kernel<L, NB4, kPair>;
+  constexpr size_t smem = sizeof(LinesSmem<L, NB4>);
+  static std::atomic<int> per_sm[64];
+  int dev = 0;
+  HERMES_CUDA_TRY(cudaGetDevice(&dev));
+  int n = dev >= 0 && dev < 64 ? per_sm[dev].load() : 0;
+  if (n == 0) {  // once per device, before any stream capture
+    HERMES_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HERMES_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, L / 2 + 32, smem));
+    if (n < 1) n = 1;
+    if (dev >= 0 && dev < 64) per_sm[dev].store(n);
+  }
+  fn<<<nsm * n, L / 2 + 32, smem, s>>>(half, P, T4, T4b, Y, nb, out, inv_n);
+  HERMES_LAUNCH_CHECK("mp_lines_quad_kernel");
+  return HERMES_OK;
+}
 
 // pair: the window K_{l,0} + K_{l+1,0} for even l, with the radial tables
 // of l in ctx.T and of l + 1 in ctx.T2 (m is 0).
@@ -1802,11 +1970,20 @@ int fields_run(const FieldsCtx& ctx, const void* half_spec, int J, int l, int m,
   const float4* T4b = reinterpret_cast<const float4*>(ctx.T2);
   const long long we = (long long)(4 * ctx.L - 4) * (ctx.L / 2 + 1);
   const int grid_e = (int)std::min<long long>(grid, (we + 255) / 256);
-#define HERMES_PREPASS(NB4, PAIR)                                                                               \
-  do {                                                                                                          \
-    mp_prepass_quad_kernel<NB4, PAIR><<<grid, 256, 0, s>>>(half, J, ctx.Pf, T4, T4b, Y, nb, ctx.binmajor, inv_n); \
-    mp_prepass_edge_kernel<NB4, PAIR><<<grid_e, 256, 0, s>>>(half, J, ctx.Pf, T4, T4b, Y, nb, ctx.binmajor,      \
-                                                            inv_n);                                            \
+  const bool own = J >= 7 && J <= 9 && g_fft_mode.load() != 0;
+  int rc = HERMES_OK;
+#define HERMES_PREPASS(NB4, PAIR)                                                                                  \
+  do {                                                                                                             \
+    if (own && J == 9)                                                                                             \
+      rc = launch_lines_quad<512, NB4, PAIR>(half, ctx.Pf, T4, T4b, Y, nb, ctx.binmajor, inv_n, ctx.nsm, s);       \
+    else if (own && J == 8)                                                                                        \
+      rc = launch_lines_quad<256, NB4, PAIR>(half, ctx.Pf, T4, T4b, Y, nb, ctx.binmajor, inv_n, ctx.nsm, s);       \
+    else if (own)                                                                                                  \
+      rc = launch_lines_quad<128, NB4, PAIR>(half, ctx.Pf, T4, T4b, Y, nb, ctx.binmajor, inv_n, ctx.nsm, s);       \
+    else                                                                                                           \
+      mp_prepass_quad_kernel<NB4, PAIR><<<grid, 256, 0, s>>>(half, J, ctx.Pf, T4, T4b, Y, nb, ctx.binmajor, inv_n); \
+    mp_prepass_edge_kernel<NB4, PAIR><<<grid_e, 256, 0, s>>>(half, J, ctx.Pf, T4, T4b, Y, nb, ctx.binmajor,         \
+                                                            inv_n);                                               \
   } while (0)
   if (pair) {
     if (nb <= 4) HERMES_PREPASS(1, true);
@@ -1818,22 +1995,24 @@ int fields_run(const FieldsCtx& ctx, const void* half_spec, int J, int l, int m,
     else HERMES_PREPASS(4, false);
   }
 #undef HERMES_PREPASS
-  HERMES_LAUNCH_CHECK("mp_prepass_kernel");
-  const int fft_mode = g_fft_mode.load();
-  const bool own = J == 9 && fft_mode != 0;
-  cufftHandle h;
-  int rc = own ? hermes::get_plan_c2c_lines(J, nb, &h) : hermes::get_plan_c2c_batch(J, nb, &h);
   if (rc) return rc;
-  cufftResult r = cufftSetStream(h, s);
-  if (r != CUFFT_SUCCESS) return fail(HERMES_ERR_CUFFT, "cufftSetStream failed: %d", (int)r);
-  r = cufftExecC2C(h, reinterpret_cast<cufftComplex*>(ctx.binmajor), reinterpret_cast<cufftComplex*>(ctx.binmajor),
-                   CUFFT_INVERSE);
-  if (r != CUFFT_SUCCESS) return fail(HERMES_ERR_CUFFT, "cufftExecC2C failed: %d", (int)r);
-  if (own) {  // z lines by cuFFT above, then the y and x passes
-    rc = hermes::fft512_strided_inverse(ctx.binmajor, nb, 1, s);
+  HERMES_LAUNCH_CHECK("mp_prepass_kernel");
+  if (own) {  // the z transform of the edge lines, then the y and x passes
+    const auto edge = J == 9 ? mp_lines_edge_kernel<512> : (J == 8 ? mp_lines_edge_kernel<256> : mp_lines_edge_kernel<128>);
+    edge<<<ctx.nsm * 4, 256, 0, s>>>(ctx.binmajor, nb);
+    HERMES_LAUNCH_CHECK("mp_lines_edge_kernel");
+    rc = hermes::fft_strided_inverse(ctx.binmajor, J, nb, 1, s);
+    if (!rc) rc = hermes::fft_strided_inverse(ctx.binmajor, J, nb, 0, s);
     if (rc) return rc;
-    rc = hermes::fft512_strided_inverse(ctx.binmajor, nb, 0, s);
+  } else {
+    cufftHandle h;
+    rc = hermes::get_plan_c2c_batch(J, nb, &h);
     if (rc) return rc;
+    cufftResult r = cufftSetStream(h, s);
+    if (r != CUFFT_SUCCESS) return fail(HERMES_ERR_CUFFT, "cufftSetStream failed: %d", (int)r);
+    r = cufftExecC2C(h, reinterpret_cast<cufftComplex*>(ctx.binmajor), reinterpret_cast<cufftComplex*>(ctx.binmajor),
+                     CUFFT_INVERSE);
+    if (r != CUFFT_SUCCESS) return fail(HERMES_ERR_CUFFT, "cufftExecC2C failed: %d", (int)r);
   }
   if (nb > 1 && !ctx.bin_major) {
     long long nblk = ctx.N / kIlCells;
@@ -1861,10 +2040,10 @@ static int fields_radii(const void* half_spec, int J, int l, int m, const double
     hrho.v[2 * b] = (float)v;
     hrho.v[2 * b + 1] = (float)(v - (double)hrho.v[2 * b]);
   }
-  mp_jl_table_kernel<<<ctx.nsm * 8, 256, 0, ctx.s>>>(ctx.T, 3 * ctx.L * ctx.L, hrho, nb, l);
+  mp_jl_table_kernel<<<ctx.nsm * 8, 256, 0, ctx.s>>>(ctx.T, 3 * ctx.L * ctx.L, hrho, nb, l, table_stride(nb));
   HERMES_LAUNCH_CHECK("mp_jl_table_kernel");
   if (pair) {
-    mp_jl_table_kernel<<<ctx.nsm * 8, 256, 0, ctx.s>>>(ctx.T2, 3 * ctx.L * ctx.L, hrho, nb, l + 1);
+    mp_jl_table_kernel<<<ctx.nsm * 8, 256, 0, ctx.s>>>(ctx.T2, 3 * ctx.L * ctx.L, hrho, nb, l + 1, table_stride(nb));
     HERMES_LAUNCH_CHECK("mp_jl_table_kernel");
   }
   return fields_run(ctx, half_spec, J, l, m, nb, pair);
@@ -1917,7 +2096,7 @@ static int fields_window(const void* half_spec, int J, int l, int m, const herme
     rc = hermes::prepare_window(bins[b], ctx.L, &wins.w[b]);
     if (rc) return rc;
   }
-  mp_iso_table_kernel<<<ctx.nsm * 8, 256, 0, ctx.s>>>(ctx.T, 3 * ctx.L * ctx.L, wins, nb);
+  mp_iso_table_kernel<<<ctx.nsm * 8, 256, 0, ctx.s>>>(ctx.T, 3 * ctx.L * ctx.L, wins, nb, table_stride(nb));
   HERMES_LAUNCH_CHECK("mp_iso_table_kernel");
   return fields_run(ctx, half_spec, J, l, m, nb);
 }
@@ -1959,7 +2138,7 @@ static int fields_table(const void* half_spec, int J, int l, int m, const double
     ta.kmax[b] = k_max[b];
   }
   ta.k_scale = grid_to_physical / (double)ctx.L;
-  mp_tab_table_kernel<<<ctx.nsm * 8, 256, 0, ctx.s>>>(ctx.T, 3 * ctx.L * ctx.L, tables, ta, nb);
+  mp_tab_table_kernel<<<ctx.nsm * 8, 256, 0, ctx.s>>>(ctx.T, 3 * ctx.L * ctx.L, tables, ta, nb, table_stride(nb));
   HERMES_LAUNCH_CHECK("mp_tab_table_kernel");
   return fields_run(ctx, half_spec, J, l, m, nb);
 }
