@@ -369,11 +369,7 @@ class Corr_2PCF:
 
     def _field_in_task_normalization(self, field):
         self._density_physical_scale = float(field.scale_factor) ** 3
-        if self.weight_normalization == "unit":
-            return field.with_normalization("unit")
-        if getattr(field, "field_kind", None) != "catalog_field":
-            return field.copy()
-        return field.switch_weight_normalization(self.weight_normalization)
+        return field._in_normalization(self.weight_normalization)
 
     def _required_flags(self):
         flags = {"dd": (True, False), "dr": (True, True), "rd": (True, True), "delta_dd": (True, True),

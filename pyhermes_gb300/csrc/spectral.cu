@@ -824,7 +824,9 @@ int pp_folded(const PPArgs& a, const PPWs& w, const double* phi_power, bool radi
   const long long ncol = fold_columns(L);
   const int fold_grid = (int)std::min<long long>((ncol + 7) / 8, (long long)nsm * 8);
   HERMES_CUDA_TRY(cudaMemsetAsync(w.maxbits, 0, sizeof(unsigned) * NP, s));
-  pp_fold_kernel<NP><<<fold_grid, kHistThreads, 0, s>>>(a, w.fold, w.maxbits);
+  for (int p = 0; p < NP; ++p)
+    pp_fold_kernel<<<fold_grid, kHistThreads, 0, s>>>(a.si[p], a.sj[p], L, a.exclude_k0, w.fold + (size_t)p * ncol * H,
+                                                      w.maxbits + p);
   HERMES_LAUNCH_CHECK("pp_fold_kernel");
   if (radial) {
     const int nh = 3 * L * L + 1;
@@ -918,9 +920,9 @@ extern "C" int hermes_pair_products(const void* const* spectra, int n_spec, cons
   cudaStream_t s = as_stream(stream);
   HERMES_CUDA_TRY(cudaMemcpyAsync(dwin, hw.data(), sizeof(WinDev) * n_bins, cudaMemcpyHostToDevice, s));
   // The folded passes, at any level and bin count: 30 shells x 2 pairs at
-  // J = 9 take 1.89 ms (fold 1.03, histogram 0.67, bins 0.19), 143.3 ms in
-  // the generic kernel; 20 shells at J = 7 0.06 ms, 1.68 ms there; 300 rings
-  // at J = 9 0.69 ms (fold 0.23, A table 0.28, columns 0.18), 1.74 ms over
+  // J = 9 take 0.65 ms (fold 0.22, histogram 0.25, bins 0.19), 143.3 ms in
+  // the generic kernel; 20 shells at J = 7 0.05 ms, 1.68 ms there; 300 rings
+  // at J = 9 0.57 ms (fold 0.11, A table 0.28, columns 0.18), 1.74 ms over
   // the unfolded columns.
   const bool radial = bandwidth == 1 && all_radial(hw, exclude_k0 != 0);
   if (radial || (all_cyl_z(hw) && cylz_smem(a.np, L, n_pairs) <= 200 * 1024)) {

@@ -979,11 +979,7 @@ class Corr_3PCF_Multipole:
 
     def _normalized(self, field):
         self._density_physical_scale = float(field.scale_factor) ** 3
-        if self.weight_normalization == "unit":
-            return field.with_normalization("unit")
-        if getattr(field, "field_kind", None) != "catalog_field":
-            return field.copy()
-        return field.switch_weight_normalization(self.weight_normalization)
+        return field._in_normalization(self.weight_normalization)
 
     def _expanded(self):
         out = list(self.products)

@@ -265,6 +265,17 @@ class SFCField:
         new.format_sfc_params()
         return new
 
+    def _in_normalization(self, mode):
+        """The field in a task's weight normalisation, for the task's reading:
+        it shares this field's coefficients where they need no rescaling."""
+        if mode == "unit":
+            return self.with_normalization("unit")
+        kind = getattr(self, "field_kind", None)
+        if kind != "catalog_field" or normalize_weight_normalization(
+                getattr(self, "weight_normalization", "raw")) == normalize_weight_normalization(mode):
+            return self._same_coefficients()
+        return self.switch_weight_normalization(mode)
+
     def _derived_field_integral(self, field):
         t = field.epsilon_device
         if t is None:
