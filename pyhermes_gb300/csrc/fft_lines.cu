@@ -245,6 +245,84 @@ fft512_cols_kernel(float2* __restrict__ data, int nf, int axis, FftWindow win) {
   cp_async_wait_group<0>();  // no copy outlives the kernel
 }
 
+// ---- z lines of a real field ------------------------------------------------------
+// Two rows of 512 real values are one complex line: z = a + i b, of which
+// A[k] = (Z[k] + conj Z[-k]) / 2 and B[k] = -i (Z[k] - conj Z[-k]) / 2.  64
+// threads a line pair, eight points a thread in registers (line_ifft), rows read
+// and written once in whole 128-byte lines.  Bound by HBM: 211 and 210 us (1.08 GB:
+// 5.1 TB/s) where cuFFT's 1-D real transforms on the same rows took 305 and 308.
+constexpr int kRealGroups = 4, kLinePT = kLen / 8;
+
+struct RealLineSync {
+  int id;
+  __device__ __forceinline__ void operator()() const {
+    asm volatile("bar.sync %0, %1;\n" ::"r"(id + 1), "n"(kLinePT) : "memory");
+  }
+};
+
+// rows [512 * 512][512] -> half spectra [512 * 512][kFft512HalfPitch] (257 values)
+__global__ void __launch_bounds__(kRealGroups* kLinePT) real_to_half_kernel(const float* __restrict__ in,
+                                                                            float2* __restrict__ out) {
+  __shared__ float2 buf[kRealGroups][9 * kLinePT];
+  __shared__ float2 tw[kLen];
+  fill_twiddles<kLen>(tw, blockDim.x);
+  __syncthreads();
+  const int g = threadIdx.x / kLinePT, t = threadIdx.x % kLinePT;
+  const RealLineSync sync{g};
+  for (int p = blockIdx.x * kRealGroups + g; p < kLen * kLen / 2; p += gridDim.x * kRealGroups) {
+    const float* a = in + (long long)p * 2 * kLen;
+    float2 v[8];
+#pragma unroll
+    for (int n = 0; n < 8; ++n) v[n] = make_float2(__ldcs(a + kLen + t + kLinePT * n), __ldcs(a + t + kLinePT * n));  // exchanged
+    line_ifft<kLen>(v, buf[g], tw, t, sync);
+    sync();
+#pragma unroll
+    for (int n = 0; n < 8; ++n) buf[g][t + kLinePT * n] = swapped(v[n]);
+    sync();
+    float2* o = out + (long long)p * 2 * kFft512HalfPitch;
+#pragma unroll
+    for (int n = 0; n < 5; ++n) {
+      const int k = t + kLinePT * n;
+      if (n == 4 && t != 0) break;
+      const float2 z = buf[g][k], m = buf[g][(kLen - k) & (kLen - 1)];
+      o[k] = make_float2(0.5f * (z.x + m.x), 0.5f * (z.y - m.y));
+      o[k + kFft512HalfPitch] = make_float2(0.5f * (z.y + m.y), 0.5f * (m.x - z.x));
+    }
+    sync();  // buf free
+  }
+}
+
+// the inverse, unnormalised; the imaginary parts at k = 0 and 256 count as zero
+__global__ void __launch_bounds__(kRealGroups* kLinePT) half_to_real_kernel(const float2* __restrict__ in,
+                                                                            float* __restrict__ out) {
+  __shared__ float2 buf[kRealGroups][9 * kLinePT];
+  __shared__ float2 tw[kLen];
+  fill_twiddles<kLen>(tw, blockDim.x);
+  __syncthreads();
+  const int g = threadIdx.x / kLinePT, t = threadIdx.x % kLinePT;
+  const RealLineSync sync{g};
+  for (int p = blockIdx.x * kRealGroups + g; p < kLen * kLen / 2; p += gridDim.x * kRealGroups) {
+    const float2* h = in + (long long)p * 2 * kFft512HalfPitch;
+    float2 v[8];
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      const int k = t + kLinePT * n;
+      const bool low = n < 4 || (n == 4 && t == 0);
+      const float2 a = h[low ? k : kLen - k], b = h[(low ? k : kLen - k) + kFft512HalfPitch];
+      v[n] = low ? make_float2(a.x - b.y, a.y + b.x) : make_float2(a.x + b.y, b.x - a.y);
+      if ((n == 0 || n == 4) && t == 0) v[n] = make_float2(a.x, b.x);
+    }
+    line_ifft<kLen>(v, buf[g], tw, t, sync);
+    float* o = out + (long long)p * 2 * kLen;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      o[t + kLinePT * n] = v[n].x;
+      o[kLen + t + kLinePT * n] = v[n].y;
+    }
+    sync();  // buf free
+  }
+}
+
 // The strided pass of L = 128 and 256: tiles of 16 columns as above, one
 // eight-point transform a thread (line_ifft's stages, its buffer per column
 // with an odd pitch), two blocks an SM.
@@ -346,6 +424,30 @@ int fft_strided_inverse(float2* data, int J, int nf, int axis, cudaStream_t s) {
   if (J == 8) return launch_fft_cols<256>(data, nf, axis, s);
   if (J == 7) return launch_fft_cols<128>(data, nf, axis, s);
   return fail(HERMES_ERR_UNSUPPORTED, "fft_strided_inverse: J=%d", J);
+}
+
+static int real_grid(int* blocks) {
+  int dev = 0, nsm = 0;
+  HERMES_CUDA_TRY(cudaGetDevice(&dev));
+  HERMES_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  *blocks = nsm * 8;
+  return HERMES_OK;
+}
+
+int fft512_real_to_half(const float* in, float2* out, cudaStream_t s) {
+  int blocks = 0, rc = real_grid(&blocks);
+  if (rc) return rc;
+  real_to_half_kernel<<<blocks, kRealGroups * kLinePT, 0, s>>>(in, out);
+  HERMES_LAUNCH_CHECK("real_to_half_kernel");
+  return HERMES_OK;
+}
+
+int fft512_half_to_real(const float2* in, float* out, cudaStream_t s) {
+  int blocks = 0, rc = real_grid(&blocks);
+  if (rc) return rc;
+  half_to_real_kernel<<<blocks, kRealGroups * kLinePT, 0, s>>>(in, out);
+  HERMES_LAUNCH_CHECK("half_to_real_kernel");
+  return HERMES_OK;
 }
 
 int fft512_half_y(float2* data, bool forward, cudaStream_t s) {

@@ -1,4 +1,4 @@
-// Strided 512-point FFT passes (fft_lines.cu) of a convolution's half spectrum.
+// 512-point FFT passes (fft_lines.cu) of a convolution's half spectrum.
 #pragma once
 
 #include "hermes_common.cuh"
@@ -20,6 +20,10 @@ struct FftWindow {
   int zero_k0;
 };
 
+// z lines of a real field [512][512][512] to half spectra and back,
+// unnormalised.
+int fft512_real_to_half(const float* in, float2* out, cudaStream_t s);
+int fft512_half_to_real(const float2* in, float* out, cudaStream_t s);
 // y transform, in place, unnormalised.
 int fft512_half_y(float2* data, bool forward, cudaStream_t s);
 // Forward x transform, the window, inverse x transform, in place.

@@ -25,7 +25,7 @@
 namespace hermes {
 
 // ---- cuFFT plan cache ----------------------------------------------------
-enum PlanKind { kR2C = 0, kC2R = 1, kC2C = 2, kR2CLines = 3, kC2RLines = 4 };
+enum PlanKind { kR2C = 0, kC2R = 1, kC2C = 2 };
 
 static std::mutex g_plan_mu;
 static std::map<std::tuple<int, int, int, int>, cufftHandle> g_plans;
@@ -42,16 +42,6 @@ int get_plan(int J, PlanKind kind, int batch, cufftHandle* out) {
   }
   cufftHandle h;
   const int L = 1 << J;
-  if (kind == kR2CLines || kind == kC2RLines) {  // the L^2 real z lines against rows of `batch` complex values
-    int n1[1] = {L}, real[1] = {L}, cplx[1] = {batch};
-    const bool fwd = kind == kR2CLines;
-    cufftResult r = cufftPlanMany(&h, 1, n1, fwd ? real : cplx, 1, fwd ? L : batch, fwd ? cplx : real, 1, fwd ? batch : L,
-                                  fwd ? CUFFT_R2C : CUFFT_C2R, L * L);
-    if (r != CUFFT_SUCCESS) return fail(HERMES_ERR_CUFFT, "cufftPlanMany(real lines, J=%d, pitch=%d) failed: %d", J, batch, (int)r);
-    g_plans[key] = h;
-    *out = h;
-    return HERMES_OK;
-  }
   int n[3] = {L, L, L};
   cufftType t = kind == kR2C ? CUFFT_R2C : (kind == kC2R ? CUFFT_C2R : CUFFT_C2C);
   long long dist_in = kind == kC2R ? (long long)L * L * (L / 2 + 1) : (long long)L * L * L;
@@ -386,20 +376,6 @@ int check_power(int J, int bw) {
 
 using namespace hermes;
 
-// The z lines of a real 512^3 field against rows of kFft512HalfPitch complex
-// values (cuFFT's contiguous 1-D transforms), either way.
-static int real_lines(const float* field, float2* spec, float* out, cudaStream_t s) {
-  cufftHandle h;
-  int rc = get_plan(9, field ? kR2CLines : kC2RLines, kFft512HalfPitch, &h);
-  if (rc) return rc;
-  HERMES_CUFFT_TRY(cufftSetStream(h, s));
-  if (field)
-    HERMES_CUFFT_TRY(cufftExecR2C(h, const_cast<cufftReal*>(field), reinterpret_cast<cufftComplex*>(spec)));
-  else
-    HERMES_CUFFT_TRY(cufftExecC2R(h, reinterpret_cast<cufftComplex*>(spec), out));
-  return HERMES_OK;
-}
-
 extern "C" int hermes_fft_r2c(const float* field, void* spec, int J, void* stream) {
   if (J < 2 || J > 10) return fail(HERMES_ERR_INVALID, "fft: J=%d outside [2,10]", J);
   cufftHandle h;
@@ -506,11 +482,11 @@ extern "C" int hermes_window_apply(const float* eps, float* out, int J, const he
   if (!fused) return hermes_fft_c2r(ws.spec, out, J, stream);
   // J = 9: z lines, y, then x, the window and x back in one pass, y, z lines
   const FftWindow fw = {kind == kFoldAxes ? ws.tab : nullptr, ws.folded, w.scale, factor, w.zero_k0};
-  rc = real_lines(eps, ws.spec, nullptr, s);
+  rc = fft512_real_to_half(eps, ws.spec, s);
   if (!rc) rc = fft512_half_y(ws.spec, true, s);
   if (!rc) rc = fft512_half_x_window_x(ws.spec, fw, s);
   if (!rc) rc = fft512_half_y(ws.spec, false, s);
-  return rc ? rc : real_lines(nullptr, ws.spec, out, s);
+  return rc ? rc : fft512_half_to_real(ws.spec, out, s);
 }
 
 extern "C" int hermes_window_materialize(const hermes_window_t* win, const double* phi_power, int bandwidth,
