@@ -1970,7 +1970,10 @@ int fields_run(const FieldsCtx& ctx, const void* half_spec, int J, int l, int m,
   const float4* T4b = reinterpret_cast<const float4*>(ctx.T2);
   const long long we = (long long)(4 * ctx.L - 4) * (ctx.L / 2 + 1);
   const int grid_e = (int)std::min<long long>(grid, (we + 255) / 256);
-  const bool own = J >= 7 && J <= 9 && g_fft_mode.load() != 0;
+  // the strided passes copy 16 bytes at a time; fields the caller keeps at an
+  // odd complex value take cuFFT's plan
+  const bool aligned = (reinterpret_cast<uintptr_t>(ctx.binmajor) & 15u) == 0;
+  const bool own = J >= 7 && J <= 9 && aligned && g_fft_mode.load() != 0;
   int rc = HERMES_OK;
 #define HERMES_PREPASS(NB4, PAIR)                                                                                  \
   do {                                                                                                             \

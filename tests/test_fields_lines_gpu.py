@@ -55,3 +55,18 @@ def test_lines_with_analytic_bins():
     finally:
         _lib.load().hermes_multipole_set_fft(1)
     assert (got - ref).abs().max() <= 2e-6 * ref.abs().max()
+
+
+@pytest.mark.parametrize("J,nb", [(7, 1), (7, 3), (8, 2)])
+def test_fields_at_an_odd_complex_value(J, nb):
+    """Fields 8 but not 16 bytes aligned: accepted, on the plan's route."""
+    L = 1 << J
+    g = torch.Generator(device="cuda").manual_seed(J)
+    spec = rfft_field(torch.randn((L,) * 3, generator=g, device="cuda"))
+    P = phi_power_device(PHI, L, 1, 1024, "cuda")
+    radii = [5.0 + 3 * i for i in range(nb)]
+    ref = mp.multipole_fields(spec, J, 2, 1, radii, P, bin_major=True).view(-1)
+    out = torch.empty(nb * L ** 3 + 2, dtype=torch.complex64, device="cuda")[1:-1]
+    assert out.data_ptr() % 16 == 8
+    mp.multipole_fields(spec, J, 2, 1, radii, P, out=out, bin_major=True)
+    assert (out - ref).abs().max() <= 2e-6 * ref.abs().max()
