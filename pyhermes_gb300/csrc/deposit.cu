@@ -67,6 +67,7 @@ struct DepStatus {
   double scale_d;               // fixed-point scale (power of two)
   double inv_d;                 // 1 / scale_d
   float scale_f, inv_f;         // the same as float
+  float qmax;                   // max |w| max |phi|^3 scale_d, rounded up
 };
 
 __device__ __forceinline__ float warp_max(float v) {
@@ -254,6 +255,8 @@ __global__ void dep_scan_chunks_kernel(unsigned* chunk_sums, int nchunks, DepSta
     st->inv_d = 1.0 / sc;
     st->scale_f = (float)sc;
     st->inv_f = (float)(1.0 / sc);
+    const double pm = (double)__uint_as_float(st->phimax_bits);
+    st->qmax = __double2float_ru((double)__uint_as_float(st->wmax_bits) * pm * pm * pm * sc);
   }
   for (int i = threadIdx.x; i < n_phi; i += blockDim.x) phi_f[i] = __double2float_rn(phi[i]);
   __shared__ unsigned total;
@@ -369,16 +372,131 @@ __device__ __forceinline__ void split_q(float v, float two_sb, float inv_two_sb,
   }
 }
 
-// The split point sb of the two-word accumulation for a tile reached by T
-// records (0: int64 atomics), see dep_accum_kernel.
-__device__ __forceinline__ int split_bits(unsigned total, const DepStatus* __restrict__ st) {
+// How a tile reached by T records accumulates (dep_add_records): kWide 64-bit
+// atomics; kSplit and kMagic two 32-bit words split at bit sb.  sb of kMagic is the
+// largest for which LO cannot wrap; its hi parts have to fit the float32 integers
+// of kRound, and the sum of a cell's hi parts 31 bits.  qmax bounds |q| but for the
+// roundings of its product (the factors 1.001 and, in kSplit, 2).
+enum { kWide = 0, kSplit = 1, kMagic = 2 };
+struct TileSum {
+  int how, sb;
+};
+
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((127 + e) << 23); }
+
+__device__ __forceinline__ TileSum tile_sum(unsigned total, const DepStatus* __restrict__ st) {
+  const float qmax = st->qmax, T = (float)total * 1.001f;
+  const unsigned long long room = total ? 0xFFFFFFFFull / (3ull * total) : 0ull;
+  const int sbm = room ? min(21, 31 - __clz((int)(unsigned)min(room, 0x7FFFFFFFull))) : 0;
+  if (sbm >= 8 && st->scale_f >= 0x1p-80f && st->scale_f <= 0x1p80f) {
+    const float h = 1.001f * qmax * pow2f(-sbm) + 2.0f;
+    if (h < 4194304.0f && T * h < 2147483648.0f) return {kMagic, sbm};
+  }
   const int clog = total > 1u ? 32 - __clz((int)(total - 1u)) : 0;  // ceil(log2 T)
   const int cand = 32 - clog;
-  if (cand < 8 || cand > 31) return 0;
-  const double pm = (double)__uint_as_float(st->phimax_bits);
-  const double qmax = (double)__uint_as_float(st->wmax_bits) * pm * pm * pm * st->scale_d;
-  // factor 2 margin for the float32 rounding of each product
-  return (double)total * (2.0 * ldexp(qmax, -cand) + 1.0) < 2147483648.0 ? cand : 0;
+  if (cand < 8 || cand > 31) return {kWide, 0};
+  return T * (2.0f * qmax * pow2f(-cand) + 1.0f) < 2147483648.0f ? TileSum{kSplit, cand} : TileSum{kWide, 0};
+}
+
+// 1.5 2^23: adding it rounds a float32 |x| < 2^22 to an integer, which its low bits then hold
+constexpr float kRound = 12582912.0f;
+
+// Adds a tile's records to its accumulators: 27 contributions q = round(w phi phi
+// phi scale), halves away from zero, per record, of which those in the tile count.
+//
+// A 64-bit shared-memory atomic add costs about four 32-bit ones, so where the
+// tile's sums allow it each int64 q = hi 2^sb + lo goes into two 32-bit words per
+// cell, LO (unsigned) and HI (two's complement; wrap-around addition is
+// associative), and the total HI 2^sb + LO is the int64 of kWide bit for bit.  With
+// T records reaching the tile no cell gets more than T contributions.
+//
+// kSplit takes 0 <= lo < 2^sb from the integer words of q (split_q): three
+// conversions and a rounding on the quarter-rate pipe, about 26 instructions a term.
+// kMagic splits in float32 additions whose roundings are the integers wanted, about
+// 14 a term and no conversion.  With x = v scale: hi = rn(x 2^-sb) from the low bits
+// of x 2^-sb + kRound; r = x - hi 2^sb is exact (|r| <= 2^(sb-1), a multiple of
+// x's last place); M = 2^22 + 2^sb has a last place of 1/2, so M + 1/2 + r
+// rounded down (x >= 0) or M + r rounded up (x < 0), with the half bit dropped,
+// is M + lo with ties away from zero as in kWide.  The low mantissa bits are
+// 2 (lo + 2^sb): LO takes them as they are, HI takes hi - 1 for the 2^sb, and the
+// cell's total is HI 2^sb + LO / 2.  It needs hi in float32's integers: from about
+// 5e5 particles on (qmax is 2^62 / n); below, kSplit.  4e6 clustered particles on
+// 512^3: 320 us against 427 us with kSplit alone (256 threads, 5 blocks an SM; 128
+// or 192 threads and 6 blocks 330 and 327, 4 blocks 352).
+template <int S, int kHow>
+__device__ __forceinline__ void dep_add_records(const DepRec* __restrict__ sorted, const unsigned* r_start,
+                                                const unsigned* r_pref, const unsigned* r_home, int nr,
+                                                const float* __restrict__ phif, const DepGeom& g, float scale_f, int sb,
+                                                int x0, int y0, int z0, long long* acc, int ncell, unsigned* cnt,
+                                                bool counts) {
+  const int Lm = g.L - 1, tzl = g.tz_log2, tyzl = g.ty_log2 + g.tz_log2;
+  const unsigned total = r_pref[nr];
+  unsigned* acc_lo = reinterpret_cast<unsigned*>(acc);
+  int* acc_hi = reinterpret_cast<int*>(acc) + ncell;
+  const float two_sb = kHow == kWide ? 0.f : pow2f(sb), inv_two_sb = kHow == kWide ? 0.f : pow2f(-sb);
+  const float to_hi = inv_two_sb * scale_f, from_hi = kHow == kMagic ? two_sb / scale_f : 0.f;
+  const float m_up = 4194304.0f + two_sb, m_down = m_up + 0.5f;
+  for (unsigned k = threadIdx.x; k < total; k += blockDim.x) {
+    int lo = 0, hi = nr - 1;  // largest r with r_pref[r] <= k
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (r_pref[mid] <= k) lo = mid; else hi = mid - 1;
+    }
+    const int r = lo;
+    const DepRec rec = sorted[r_start[r] + (k - r_pref[r])];
+    const int cx = rec.cell >> 20, cy = (rec.cell >> 10) & 1023, cz = rec.cell & 1023;
+    const int fx = rec.frac >> 20, fy = (rec.frac >> 10) & 1023, fz = rec.frac & 1023;
+    int lx[S], ly[S], lz[S];
+    float px[S], py[S], pz[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      lx[s] = (cx - s - x0) & Lm;
+      ly[s] = (cy - s - y0) & Lm;
+      lz[s] = (cz - s - z0) & Lm;
+      px[s] = rec.w * __ldg(&phif[fx + g.res * s]);
+      py[s] = __ldg(&phif[fy + g.res * s]);
+      pz[s] = __ldg(&phif[fz + g.res * s]);
+    }
+    // every lane runs all S^3 terms and predicates the adds on the term's
+    // cell lying in this tile (no divergent skips between the lanes'
+    // particles)
+#pragma unroll
+    for (int a = 0; a < S; ++a) {
+      const bool va = lx[a] < g.tx;
+#pragma unroll
+      for (int b = 0; b < S; ++b) {
+        const bool vb = va && ly[b] < g.ty;
+        const float pxy = px[a] * py[b];
+        const int row = (lx[a] << tyzl) + (ly[b] << tzl);
+#pragma unroll
+        for (int c = 0; c < S; ++c) {
+          const bool v = vb && lz[c] < g.tz;
+          const int cell = row + lz[c];
+          const float p = pxy * pz[c];
+          if (kHow == kMagic) {
+            const float t = __fmaf_rn(p, to_hi, kRound);
+            const float rest = __fmaf_rn(-__fsub_rn(t, kRound), from_hi, p);
+            const float u = p < 0.f ? __fmaf_ru(rest, scale_f, m_up) : __fmaf_rd(rest, scale_f, m_down);
+            if (v) {
+              atomicAdd(&acc_lo[cell], __float_as_uint(u) & 0x7FFFFEu);
+              atomicAdd(&acc_hi[cell], __float_as_int(t) - (__float_as_int(kRound) + 1));
+            }
+          } else if (kHow == kSplit) {
+            int qh;
+            unsigned ql;
+            split_q(p * scale_f, two_sb, inv_two_sb, 1u << sb, qh, ql);
+            if (v && ql != 0u) atomicAdd(&acc_lo[cell], ql);
+            if (v && qh != 0) atomicAdd(&acc_hi[cell], qh);
+          } else {
+            const long long q = f32_to_ll_rn(p * scale_f);
+            if (v && q != 0)
+              atomicAdd(reinterpret_cast<unsigned long long*>(&acc[cell]), static_cast<unsigned long long>(q));
+          }
+        }
+      }
+    }
+    if (counts && r_home[r]) atomicAdd(&cnt[((cx - x0) << tyzl) + ((cy - y0) << tzl) + (cz - z0)], 1u);
+  }
 }
 
 template <int S, bool kF64Out>
@@ -392,7 +510,8 @@ dep_accum_kernel(const DepRec* __restrict__ sorted, const unsigned* __restrict__
   long long* acc = reinterpret_cast<long long*>(smem);
   unsigned* cnt = reinterpret_cast<unsigned*>(acc + ncell);
   __shared__ unsigned r_start[64], r_pref[65], r_home[64];
-  __shared__ int n_ranges, s_sb;
+  __shared__ int n_ranges;
+  __shared__ TileSum s_sum;
 
   const int tile = blockIdx.x;
   const int hz = tile % g.ntz, hy = (tile / g.ntz) % g.nty, hx = tile / (g.ntz * g.nty);
@@ -455,7 +574,7 @@ dep_accum_kernel(const DepRec* __restrict__ sorted, const unsigned* __restrict__
       const int nr = __popc(v0) + __popc(v1);
       r_pref[nr] = inc;
       n_ranges = nr;
-      s_sb = split_bits(inc, st);
+      s_sum = tile_sum(inc, st);
     }
   }
   __syncthreads();
@@ -477,118 +596,15 @@ dep_accum_kernel(const DepRec* __restrict__ sorted, const unsigned* __restrict__
     return;
   }
 
-  const float scale_f = st->scale_f;
-  const int Lm = g.L - 1;
-  // Split accumulation.  A 64-bit shared-memory atomic add costs about four
-  // 32-bit ones on this part, so when the tile's sums allow it each int64
-  // contribution q = hi * 2^sb + lo (0 <= lo < 2^sb, hi = q >> sb) goes into
-  // two 32-bit words per cell: LO += lo (unsigned) and HI += hi (two's
-  // complement).  With T records reaching the tile no cell gets more than T
-  // contributions, so LO is exact when T * (2^sb - 1) < 2^32, and HI's final
-  // value is exact (wrap-around addition is associative) when the true sum
-  // of the hi parts fits in 31 bits: |sum hi| <= T * (qmax / 2^sb + 1), with
-  // qmax = max|w| * max|phi|^3 * scale the largest |q|.  The cell total
-  // HI * 2^sb + LO is then the same int64 as the plain path's, bit for bit.
-  // Otherwise (dense tiles) sb = 0 and the tile uses int64 atomics.  The
-  // same bound gives |q| / 2^sb < 2^31 for every contribution, which
-  // split_q needs.
-  const int sb = s_sb;  // chosen once per tile by the range-table warp (float64 is slow on this part)
-  if (sb > 0) {
-    unsigned* acc_lo = reinterpret_cast<unsigned*>(acc);
-    int* acc_hi = reinterpret_cast<int*>(acc) + ncell;
-    const float two_sb = ldexpf(1.0f, sb), inv_two_sb = ldexpf(1.0f, -sb);
-    const unsigned lo_one = 1u << sb;
-    for (unsigned k = threadIdx.x; k < total; k += blockDim.x) {
-      int lo = 0, hi = nr - 1;  // largest r with r_pref[r] <= k
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (r_pref[mid] <= k) lo = mid; else hi = mid - 1;
-      }
-      const int r = lo;
-      const DepRec rec = sorted[r_start[r] + (k - r_pref[r])];
-      const int cx = rec.cell >> 20, cy = (rec.cell >> 10) & 1023, cz = rec.cell & 1023;
-      const int fx = rec.frac >> 20, fy = (rec.frac >> 10) & 1023, fz = rec.frac & 1023;
-      int lx[S], ly[S], lz[S];
-      float px[S], py[S], pz[S];
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        lx[s] = (cx - s - x0) & Lm;
-        ly[s] = (cy - s - y0) & Lm;
-        lz[s] = (cz - s - z0) & Lm;
-        px[s] = rec.w * __ldg(&phif[fx + g.res * s]);
-        py[s] = __ldg(&phif[fy + g.res * s]);
-        pz[s] = __ldg(&phif[fz + g.res * s]);
-      }
-      // every lane runs all S^3 terms and predicates the adds on the term's
-      // cell lying in this tile (no divergent skips between the lanes'
-      // particles)
-#pragma unroll
-      for (int a = 0; a < S; ++a) {
-        const bool va = lx[a] < g.tx;
-#pragma unroll
-        for (int b = 0; b < S; ++b) {
-          const bool vb = va && ly[b] < g.ty;
-          const float pxy = px[a] * py[b];
-          const int row = (lx[a] << tyzl) + (ly[b] << tzl);
-#pragma unroll
-          for (int c = 0; c < S; ++c) {
-            const bool v = vb && lz[c] < g.tz;
-            int qh;
-            unsigned ql;
-            split_q(pxy * pz[c] * scale_f, two_sb, inv_two_sb, lo_one, qh, ql);
-            const int cell = row + lz[c];
-            if (v && ql != 0u) atomicAdd(&acc_lo[cell], ql);
-            if (v && qh != 0) atomicAdd(&acc_hi[cell], qh);
-          }
-        }
-      }
-      if (counts_out && r_home[r]) {
-        atomicAdd(&cnt[((cx - x0) << tyzl) + ((cy - y0) << tzl) + (cz - z0)], 1u);
-      }
-    }
-  } else
-  for (unsigned k = threadIdx.x; k < total; k += blockDim.x) {
-    int lo = 0, hi = nr - 1;  // largest r with r_pref[r] <= k
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (r_pref[mid] <= k) lo = mid; else hi = mid - 1;
-    }
-    const int r = lo;
-    const DepRec rec = sorted[r_start[r] + (k - r_pref[r])];
-    const int cx = rec.cell >> 20, cy = (rec.cell >> 10) & 1023, cz = rec.cell & 1023;
-    const int fx = rec.frac >> 20, fy = (rec.frac >> 10) & 1023, fz = rec.frac & 1023;
-    int lx[S], ly[S], lz[S];
-    float px[S], py[S], pz[S];
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-      lx[s] = (cx - s - x0) & Lm;
-      ly[s] = (cy - s - y0) & Lm;
-      lz[s] = (cz - s - z0) & Lm;
-      px[s] = rec.w * __ldg(&phif[fx + g.res * s]);
-      py[s] = __ldg(&phif[fy + g.res * s]);
-      pz[s] = __ldg(&phif[fz + g.res * s]);
-    }
-#pragma unroll
-    for (int a = 0; a < S; ++a) {
-      const bool va = lx[a] < g.tx;
-#pragma unroll
-      for (int b = 0; b < S; ++b) {
-        const bool vb = va && ly[b] < g.ty;
-        const float pxy = px[a] * py[b];
-        const int row = (lx[a] << tyzl) + (ly[b] << tzl);
-#pragma unroll
-        for (int c = 0; c < S; ++c) {
-          const bool v = vb && lz[c] < g.tz;
-          const long long q = f32_to_ll_rn(pxy * pz[c] * scale_f);
-          if (v && q != 0)
-            atomicAdd(reinterpret_cast<unsigned long long*>(&acc[row + lz[c]]), static_cast<unsigned long long>(q));
-        }
-      }
-    }
-    if (counts_out && r_home[r]) {
-      atomicAdd(&cnt[((cx - x0) << tyzl) + ((cy - y0) << tzl) + (cz - z0)], 1u);
-    }
-  }
+  const TileSum sum = s_sum;
+  const int sb = sum.how == kWide ? 0 : sum.sb, half = sum.how == kMagic ? 1 : 0;
+#define HERMES_ADD_RECORDS(HOW)                                                                                     \
+  dep_add_records<S, HOW>(sorted, r_start, r_pref, r_home, nr, phif, g, st->scale_f, sb, x0, y0, z0, acc, ncell, cnt, \
+                          counts_out != nullptr)
+  if (sum.how == kMagic) HERMES_ADD_RECORDS(kMagic);
+  else if (sum.how == kSplit) HERMES_ADD_RECORDS(kSplit);
+  else HERMES_ADD_RECORDS(kWide);
+#undef HERMES_ADD_RECORDS
   __syncthreads();
 
   const float inv_f = st->inv_f;
@@ -597,7 +613,8 @@ dep_accum_kernel(const DepRec* __restrict__ sorted, const unsigned* __restrict__
     const int lz_ = i & (g.tz - 1), ly_ = (i >> tzl) & (g.ty - 1), lx_ = i >> tyzl;
     const size_t gi = ((size_t)(x0 + lx_) * g.L + (y0 + ly_)) * g.L + (z0 + lz_);
     if (!kF64Out && sb > 0) {  // float32 field from the two words, no 64-bit arithmetic
-      const uint4 l4 = *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned*>(acc) + i);
+      uint4 l4 = *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned*>(acc) + i);
+      l4 = make_uint4(l4.x >> half, l4.y >> half, l4.z >> half, l4.w >> half);
       const int4 h4 = *reinterpret_cast<const int4*>(reinterpret_cast<const int*>(acc) + ncell + i);
       *reinterpret_cast<float4*>(out32 + gi) =
           make_float4(split_to_f32(h4.x, l4.x, sb) * inv_f, split_to_f32(h4.y, l4.y, sb) * inv_f,
@@ -606,8 +623,9 @@ dep_accum_kernel(const DepRec* __restrict__ sorted, const unsigned* __restrict__
       continue;
     }
     longlong2 a01, a23;
-    if (sb > 0) {  // cell total = HI * 2^sb + LO
-      const uint4 l4 = *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned*>(acc) + i);
+    if (sb > 0) {  // cell total = HI * 2^sb + LO (kMagic: LO / 2)
+      uint4 l4 = *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned*>(acc) + i);
+      l4 = make_uint4(l4.x >> half, l4.y >> half, l4.z >> half, l4.w >> half);
       const int4 h4 = *reinterpret_cast<const int4*>(reinterpret_cast<const int*>(acc) + ncell + i);
       const long long m = 1LL << sb;
       a01 = make_longlong2((long long)h4.x * m + l4.x, (long long)h4.y * m + l4.y);
