@@ -4,12 +4,13 @@
 // for one GB300.  The reference walks particles sequentially and does 27
 // float64 read-modify-writes per particle into the grid.  Here:
 //
-//   K0 dep_max_kernel     max|w| and max|phi| (order-independent bound)
 //   K1 dep_bin_kernel     per particle: float64 cell/frac (bit-identical to the
 //                         reference's floor/astype(int32)), packed 16-byte
 //                         record, histogram over (home tile, region) buckets
-//   K2 dep_scan_*         exclusive scan of the bucket histogram
-//   K3 dep_scatter_kernel counting-sort scatter (warp-aggregated slots)
+//                         (the record keeps its slot in its bucket), max|w|
+//   K2 dep_scan_*         exclusive scan of the bucket histogram; max|phi| and
+//                         the fixed-point scale
+//   K3 dep_scatter_kernel counting-sort scatter
 //   K4 dep_accum_kernel   one CTA per output tile: gathers the records of its
 //                         own tile and of the <=7 upper-neighbour tiles whose
 //                         support reaches it, accumulates each particle's
@@ -48,7 +49,7 @@ struct __align__(16) DepRec {
   uint32_t cell;  // cx << 20 | cy << 10 | cz
   uint32_t frac;  // fx << 20 | fy << 10 | fz
   float w;
-  uint32_t key;   // home_tile * 8 + region, or kRejected
+  uint32_t slot;  // place in its bucket (dep_key), or kRejected
 };
 
 struct DepGeom {
@@ -73,27 +74,6 @@ struct DepStatus {
 __device__ __forceinline__ float warp_max(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
-}
-
-__global__ void dep_max_kernel(const double* __restrict__ w, int64_t n,
-                               const double* __restrict__ phi, int n_phi,
-                               DepStatus* st) {
-  float m = 0.f, pm = 0.f;
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    double v = fabs(w[i]);
-    if (isfinite(v)) m = fmaxf(m, __double2float_ru(v));
-  }
-  if (blockIdx.x == 0) {
-    for (int i = threadIdx.x; i < n_phi; i += blockDim.x)
-      pm = fmaxf(pm, __double2float_ru(fabs(phi[i])));
-  }
-  m = warp_max(m);
-  pm = warp_max(pm);
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax(&st->wmax_bits, __float_as_uint(m));
-    atomicMax(&st->phimax_bits, __float_as_uint(pm));
-  }
 }
 
 // float64 cell / fraction index of one coordinate, exactly as the reference:
@@ -129,8 +109,9 @@ __device__ __forceinline__ bool dep_axis_fast(double x, const DepGeom& g, int& c
   return true;
 }
 
+// The bucket of a cell: home_tile * 8 + region.
 __device__ __forceinline__ unsigned dep_key(int cx, int cy, int cz, const DepGeom& g) {
-  int hx = cx / g.tx, hy = cy / g.ty, hz = cz / g.tz;
+  const int hx = cx >> g.tx_log2, hy = cy >> g.ty_log2, hz = cz >> g.tz_log2;
   unsigned region = 0;
   if (g.ntx > 1 && (cx - hx * g.tx) < g.S - 1) region |= 1u;
   if (g.nty > 1 && (cy - hy * g.ty) < g.S - 1) region |= 2u;
@@ -152,36 +133,44 @@ __device__ __forceinline__ unsigned warp_agg_slot(unsigned* ctr, unsigned key) {
   return base + rank;
 }
 
+// One pass over the particles for the records, the histogram and max|w| (a pass of
+// its own for the maximum cost 20 us at 4e6 particles).  A slot comes from the
+// histogram's own atomics, so the scatter needs none.  Whole deposit, before and
+// after: 2e6 particles on 128^3 406 -> 361 us, 2e5 on 256^3 101 -> 86, 3e4 on 64^3
+// 68 -> 58, 1e6 on 512^3 342 -> 325; 4e6 on 512^3 equal (the atomics' returns and
+// the scatter's reads of 1 MB of offsets cost what the pass saves).  Two or four
+// particles a thread in flight measured the same.
 __global__ void dep_bin_kernel(const double* __restrict__ pos, const double* __restrict__ w,
                                int64_t n, DepGeom g, DepRec* __restrict__ rec,
                                unsigned* __restrict__ counts, DepStatus* st) {
+  float wmax = 0.f;
   int64_t warp_stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += warp_stride) {
     int64_t i = base + threadIdx.x;
     unsigned key = kRejected;
+    DepRec r = {0, 0, 0.f, kRejected};
     if (i < n) {
       double x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
       double wi = w[i];
+      if (isfinite(wi)) wmax = fmaxf(wmax, __double2float_ru(fabs(wi)));
       int cx, cy, cz, fx, fy, fz;
       bool ok = isfinite(x) && isfinite(y) && isfinite(z) && isfinite(wi) &&
                 dep_axis_fast(x, g, cx, fx) && dep_axis_fast(y, g, cy, fy) && dep_axis_fast(z, g, cz, fz);
-      DepRec r;
       if (ok) {
         key = dep_key(cx, cy, cz, g);
         r.cell = ((unsigned)cx << 20) | ((unsigned)cy << 10) | (unsigned)cz;
         r.frac = ((unsigned)fx << 20) | ((unsigned)fy << 10) | (unsigned)fz;
         r.w = (float)wi;
       } else {
-        r.cell = 0;
-        r.frac = 0;
-        r.w = 0.f;
         atomicAdd(&st->rejected, 1ULL);
       }
-      r.key = key;
-      rec[i] = r;
     }
-    warp_agg_slot(counts, key);
+    const unsigned slot = warp_agg_slot(counts, key);
+    if (key != kRejected) r.slot = slot;
+    if (i < n) rec[i] = r;
   }
+  wmax = warp_max(wmax);
+  if ((threadIdx.x & 31) == 0 && wmax > 0.f) atomicMax(&st->wmax_bits, __float_as_uint(wmax));
 }
 
 // Scan phase 1: per-chunk sums.
@@ -244,12 +233,24 @@ __device__ __forceinline__ double dep_fixed_scale(const DepStatus* st, int64_t n
 }
 
 // Scan phase 2: exclusive scan of chunk sums (single block, serial over
-// groups of 1024).  Also fixes the fixed-point scale and the float32 copy of
+// groups of 1024).  Also fixes max|phi|, the fixed-point scale and the float32 copy of
 // phi used by the accumulation.
 __global__ void dep_scan_chunks_kernel(unsigned* chunk_sums, int nchunks, DepStatus* st, int64_t n,
                                        const double* __restrict__ phi, int n_phi,
                                        float* __restrict__ phi_f) {
+  __shared__ unsigned s_pmax;
+  if (threadIdx.x == 0) s_pmax = 0u;
+  __syncthreads();
+  float pmax = 0.f;
+  for (int i = threadIdx.x; i < n_phi; i += blockDim.x) {
+    phi_f[i] = __double2float_rn(phi[i]);
+    pmax = fmaxf(pmax, __double2float_ru(fabs(phi[i])));
+  }
+  pmax = warp_max(pmax);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_pmax, __float_as_uint(pmax));
+  __syncthreads();
   if (threadIdx.x == 0) {
+    st->phimax_bits = s_pmax;
     const double sc = dep_fixed_scale(st, n);
     st->scale_d = sc;
     st->inv_d = 1.0 / sc;
@@ -258,7 +259,6 @@ __global__ void dep_scan_chunks_kernel(unsigned* chunk_sums, int nchunks, DepSta
     const double pm = (double)__uint_as_float(st->phimax_bits);
     st->qmax = __double2float_ru((double)__uint_as_float(st->wmax_bits) * pm * pm * pm * sc);
   }
-  for (int i = threadIdx.x; i < n_phi; i += blockDim.x) phi_f[i] = __double2float_rn(phi[i]);
   __shared__ unsigned total;
   unsigned carry = 0;
   for (int beg = 0; beg < nchunks; beg += 1024) {
@@ -271,12 +271,11 @@ __global__ void dep_scan_chunks_kernel(unsigned* chunk_sums, int nchunks, DepSta
   }
 }
 
-// Scan phase 3: rescan each chunk with its prefix; writes offsets and the
-// scatter cursor, and offsets[nb] = grand total.
+// Scan phase 3: rescan each chunk with its prefix; writes offsets, and
+// offsets[nb] = grand total.
 __global__ void dep_scan_apply_kernel(const unsigned* __restrict__ counts, int nb,
                                       const unsigned* __restrict__ chunk_prefix,
-                                      unsigned* __restrict__ offsets,
-                                      unsigned* __restrict__ cursor) {
+                                      unsigned* __restrict__ offsets) {
   __shared__ unsigned total;
   int beg = blockIdx.x * kScanChunk + threadIdx.x * 4;
   unsigned v[4];
@@ -287,29 +286,20 @@ __global__ void dep_scan_apply_kernel(const unsigned* __restrict__ counts, int n
   }
   unsigned ex = block_excl_scan_1024(s, &total) + chunk_prefix[blockIdx.x];
   for (int k = 0; k < 4; ++k) {
-    if (beg + k < nb) {
-      offsets[beg + k] = ex;
-      cursor[beg + k] = ex;
-    }
+    if (beg + k < nb) offsets[beg + k] = ex;
     ex += v[k];
   }
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 1023) offsets[nb] = ex;
 }
 
-__global__ void dep_scatter_kernel(const DepRec* __restrict__ rec, int64_t n,
-                                   unsigned* __restrict__ cursor,
+__global__ void dep_scatter_kernel(const DepRec* __restrict__ rec, int64_t n, DepGeom g,
+                                   const unsigned* __restrict__ offsets,
                                    DepRec* __restrict__ sorted) {
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-    int64_t i = base + threadIdx.x;
-    DepRec r;
-    unsigned key = kRejected;
-    if (i < n) {
-      r = rec[i];
-      key = r.key;
-    }
-    unsigned slot = warp_agg_slot(cursor, key);
-    if (key != kRejected) sorted[slot] = r;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const DepRec r = rec[i];
+    if (r.slot == kRejected) continue;
+    sorted[offsets[dep_key(r.cell >> 20, (r.cell >> 10) & 1023, r.cell & 1023, g)] + r.slot] = r;
   }
 }
 
@@ -700,7 +690,6 @@ int dep_plan(int64_t n, int J, int S, int res, DepPlan* p, int tile) {
   c.take<DepStatus>(1);
   c.take<unsigned>(p->nbuckets);      // counts
   c.take<unsigned>(p->nbuckets + 1);  // offsets
-  c.take<unsigned>(p->nbuckets);      // cursor
   c.take<unsigned>(p->nchunks);       // chunk sums
   c.take<float>(kMaxSupport * 1024);  // float32 phi
   c.take<DepRec>((size_t)(n > 0 ? n : 1));  // unsorted records
@@ -760,7 +749,6 @@ struct DepBuffers {
   DepStatus* st;
   unsigned* counts;
   unsigned* offsets;
-  unsigned* cursor;
   unsigned* chunk_sums;
   float* phif;
   DepRec* rec;
@@ -781,7 +769,6 @@ int dep_prepare(int64_t n, int J, double box, int n_phi, int phi_res, const doub
   b->st = c.take<DepStatus>(1);
   b->counts = c.take<unsigned>(p->nbuckets);
   b->offsets = c.take<unsigned>(p->nbuckets + 1);
-  b->cursor = c.take<unsigned>(p->nbuckets);
   b->chunk_sums = c.take<unsigned>(p->nchunks);
   b->phif = c.take<float>(kMaxSupport * 1024);
   b->rec = c.take<DepRec>((size_t)(n > 0 ? n : 1));
@@ -805,8 +792,6 @@ int deposit_sort(const double* pos, const double* w, int64_t n, int J, double bo
   const int64_t want = (n + 255) / 256;
   const int grid_p = (int)(want < 1 ? 1 : (want < (int64_t)nsm * 8 ? want : (int64_t)nsm * 8));
 
-  dep_max_kernel<<<grid_p, 256, 0, s>>>(w, n, phi, n_phi, b.st);
-  HERMES_LAUNCH_CHECK("dep_max_kernel");
   if (n > 0) {
     dep_bin_kernel<<<grid_p, 256, 0, s>>>(pos, w, n, p.g, b.rec, b.counts, b.st);
     HERMES_LAUNCH_CHECK("dep_bin_kernel");
@@ -815,10 +800,10 @@ int deposit_sort(const double* pos, const double* w, int64_t n, int J, double bo
   HERMES_LAUNCH_CHECK("dep_scan_sums_kernel");
   dep_scan_chunks_kernel<<<1, 1024, 0, s>>>(b.chunk_sums, p.nchunks, b.st, n, phi, n_phi, b.phif);
   HERMES_LAUNCH_CHECK("dep_scan_chunks_kernel");
-  dep_scan_apply_kernel<<<p.nchunks, 1024, 0, s>>>(b.counts, p.nbuckets, b.chunk_sums, b.offsets, b.cursor);
+  dep_scan_apply_kernel<<<p.nchunks, 1024, 0, s>>>(b.counts, p.nbuckets, b.chunk_sums, b.offsets);
   HERMES_LAUNCH_CHECK("dep_scan_apply_kernel");
   if (n > 0) {
-    dep_scatter_kernel<<<grid_p, 256, 0, s>>>(b.rec, n, b.cursor, b.sorted);
+    dep_scatter_kernel<<<grid_p, 256, 0, s>>>(b.rec, n, p.g, b.offsets, b.sorted);
     HERMES_LAUNCH_CHECK("dep_scatter_kernel");
   }
   return HERMES_OK;
