@@ -374,7 +374,7 @@ def deposit_bench(dev, lib, kernels, phi, flush, steps):
     ach = alg / (acc_ms / 1e3) / 1e9
     return {"metric": "deposit Mparticles/s (4M lognormal points, J=9, float32 field)",
             "value": DEP_N / (step_ms / 1e3) / 1e6, "unit": "Mparticles/s",
-            "ms_per_step": step_ms, "launches_per_step": 7,
+            "ms_per_step": step_ms, "launches_per_step": 6,
             "tile": "x".join(map(str, tile)), "tile_ms_per_deposit": tile_ms,
             "default_tile": {"tile": "8x16x32", "ms_per_step": default_step, "accumulate_ms": default_acc,
                              "value": DEP_N / (default_step / 1e3) / 1e6},
@@ -498,13 +498,13 @@ def c2_bench(dev, phi, steps):
             "window_roofline": {"bound": "hbm", "achieved": win_bytes / t_win / 1e9, "peak": hbm, "peak_kind": kind,
                                 "unit": "GB/s", "frac": win_bytes / t_win / 1e9 / hbm,
                                 "algorithmic_bytes": win_bytes,
-                                "note": "cuFFT R2C + on-the-fly window multiply + cuFFT C2R"},
+                                "note": "z lines, y, x with the window and x back in one pass, y, z lines"},
             "twopcf_roofline": {"bound": "hbm", "achieved": tp_bytes / t_2pcf / 1e9, "peak": hbm,
                                 "peak_kind": kind, "unit": "GB/s", "frac": tp_bytes / t_2pcf / 1e9 / hbm,
                                 "algorithmic_bytes": tp_bytes,
                                 "traffic": profile_traffic("pair_products_cylz_kernel"),
-                                "note": "one forward rFFT and one pass over the half spectrum for all 300 bins "
-                                        "(separable ring windows, column kernel); issue-bound"}}
+                                "note": "one forward rFFT, one fold of the half spectrum and one pass over the folded "
+                                        "columns for all 300 bins (separable ring windows)"}}
 
 
 def mc_bench(dev, phi_np, steps):
@@ -817,11 +817,11 @@ def run_gb300(args, ws, rank, local):
     value = t_total / (args.steps * ws)
     zeta = np.asarray(res.zeta_l)
 
-    # our kernels per step: 2 deposits x 7; per product, per single (l, m) term 8 (fields: power,
-    # j_l table, interior and edge prepass, the y and x FFT passes after cuFFT's z lines; contract:
-    # tensor-core contraction, reduce) and per degree pair 9 (a second j_l table); the mixing solve
+    # our kernels per step: 2 deposits x 6; per product, per single (l, m) term 9 (fields: power,
+    # j_l table, interior lines, edge prepass, edge lines, the y and x FFT passes; contract:
+    # tensor-core contraction, reduce) and per degree pair 10 (a second j_l table); the mixing solve
     n_pairs = len(mp.degree_pairs([(l, m) for l in range(MP_LMAX + 1) for m in range(l + 1)]))
-    kernel_launches = args.steps * (14 + 2 * ((N_LM - 2 * n_pairs) * 8 + n_pairs * 9) + 1)
+    kernel_launches = args.steps * (12 + 2 * ((N_LM - 2 * n_pairs) * 9 + n_pairs * 10) + 1)
 
     # end to end: catalogues in pinned host memory, copies inside the timed region
     h = [torch.as_tensor(a).pin_memory() for a in (dpos_np, dw_np, rpos_np, rw_np)]
@@ -934,9 +934,9 @@ def run_gb300(args, ws, rank, local):
                      "stencil_fp32": {"flops": stencil_flops, "achieved_tflops": stencil_flops / t_con["tensor"] / 1e12,
                                       "nominal_peak_tflops": 80.6,
                                       "frac": stencil_flops / t_con["tensor"] / 1e12 / 80.6}},
-        "fields_roofline": {"kernels": "mp_jl_table + mp_prepass_quad/edge + inverse FFT of 15 fields (cuFFT 1-D z "
-                                       "lines, fft512_cols_kernel over y and x; bin-major output, read as is by the "
-                                       "tensor-core contraction)",
+        "fields_roofline": {"kernels": "mp_jl_table + mp_lines_quad/edge (prepass with the z transform) + "
+                                       "fft512_cols_kernel over y and x, 15 fields; bin-major output, read as is by "
+                                       "the tensor-core contraction",
                             "bound": "hbm", "ms_per_lm": t_fld["bin_major"] * 1e3, "algorithmic_bytes": fld_bytes,
                             "achieved": fld_bytes / t_fld["bin_major"] / 1e9, "peak": hbm, "peak_kind": kind,
                             "unit": "GB/s", "frac": fld_bytes / t_fld["bin_major"] / 1e9 / hbm,

@@ -360,9 +360,9 @@ int hermes_multipole_contract_pair_bm_async(const float* eps1, const void* field
  * _stream_convolution_fields, utils/corr3pcf_multipoles.py:267-321).
  * hermes_multipole_set_fft: 0 = cuFFT's batched 3-D plan; 1 (default) = at
  * J = 7, 8 and 9, the z lines transformed as they are made, followed by strided
- * passes over y and x (hermes_fft512_strided_inverse at J = 9; other J keep the
- * 3-D plan).  Returns the previous mode,
- * HERMES_ERR_INVALID outside [0, 1].  Process-wide.
+ * passes over y and x (hermes_fft512_strided_inverse at J = 9); other J, and
+ * fields that are not 16-byte aligned, keep the 3-D plan.  Returns the previous
+ * mode, HERMES_ERR_INVALID outside [0, 1].  Process-wide.
  * hermes_fft512_strided_inverse: in-place unnormalised inverse 512-point
  * FFTs (e^{+2 pi i n k / 512}, as CUFFT_INVERSE) along axis 0 (x, element
  * stride 512^2) or 1 (y, stride 512) of nfields (1..64) complex64 fields

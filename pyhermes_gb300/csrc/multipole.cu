@@ -10,18 +10,20 @@
 // Here, per (l, m), for all radial bins at once:
 //   mp_jl_table_kernel   j_l(2 pi sqrt(n2) R_b / L) tabulated over the integer
 //                        |k|^2 grid (float32, double-float phase)
-//   mp_prepass_*_kernel  eps_hat(k) K_lm^b(k) / L^3 for every bin b, Y_lm
-//                        shared by the bins, written as a batch of spectra;
-//                        one window evaluation serves k, its x- and
-//                        y-reflections and their inversions
-//   cuFFT (batched C2C)  -> a_lm^b(x) for every bin, one contiguous field per
-//                        bin (cuFFT is far slower on strided batches)
-//   mp_interleave_kernel bin-major -> bin-interleaved [cell][16], so one
-//                        cell's bins are one 128-byte row for the contraction
-//   mp_contract_kernel   S[b2,b3] = sum_y a2^{b2}(y) G^{b3}(y) with
+//   mp_lines_*_kernel    J = 7, 8, 9: eps_hat(k) K_lm^b(k) / L^3 for every bin b,
+//                        Y_lm shared by the bins; one window evaluation serves
+//                        k, its x- and y-reflections and their inversions; the
+//                        z transform of the lines before they are written
+//   fft_cols kernels     the y and x transforms, in place -> a_lm^b(x)
+//   mp_prepass_*_kernel  other J: the spectra alone, transformed by cuFFT's
+//                        batched 3-D plan (far slower on strided batches)
+//   mp_contract_tc_kernel S[b2,b3] = sum_y a2^{b2}(y) G^{b3}(y) with
 //                        G(y) = sum_{l1,l2} Gamma3 eps1(y+l1) a3(y+l1-l2), an
-//                        x-marching separable pair stencil (see the kernel)
-//   mp_reduce_kernel     float64 cross-block reduction
+//                        x-marching separable pair stencil, the bin x bin
+//                        product on the tensor cores (see the kernel)
+//   mp_reduce_*_kernel   float64 cross-block reduction
+//   mp_interleave_kernel, mp_contract_kernel  the bin-interleaved layout
+//                        [cell][16] and the all-FP32 engine on it
 // The identity S = sum_y a2(y) G3(y) is the reference sum with y = x - l1.
 // mp_plain_kernel is the reference-form contraction of one (a2, a3) pair
 // (the per-sample path the batched engine is measured against).
@@ -1235,7 +1237,7 @@ struct A3Copy {
   }
 };
 
-// kBM: fields in the bin-major layout [bin][cell] that cuFFT writes (a2 by a
+// kBM: fields in the bin-major layout [bin][cell] of the transforms (a2 by a
 // 4-D TMA map over (z, y, x, bin), a3 staged per bin); otherwise the
 // bin-interleaved [cell][16] layout or a single [cell] field.
 //
@@ -1839,7 +1841,7 @@ size_t table_floats(int J) {
 }  // namespace
 
 // Workspace: j_l table, partial sums and, for nb > 1, the bin-major fields
-// (nb * L^3 complex64) that cuFFT transforms before they are interleaved.
+// (nb * L^3 complex64) that are transformed before they are interleaved.
 namespace {
 // The one workspace layout of the fields and contraction calls.
 struct MpWs {
@@ -1903,7 +1905,7 @@ struct FieldsCtx {
   bool bin_major;
 };
 
-// bin_major: the caller's fields_out holds the batch as cuFFT leaves it,
+// bin_major: the caller's fields_out holds the batch as the transforms leave it,
 // [nb][L^3] (no interleave, and the workspace needs no bin-major copy).
 int fields_setup(const void* half_spec, int J, int l, int m, int nb, const double* phi_power, void* fields_out,
                  void* workspace, size_t workspace_bytes, void* stream, FieldsCtx* ctx, bool bin_major = false) {

@@ -1,13 +1,15 @@
-// Spectral window passes around cuFFT: `field @ window`, kernel
+// Spectral window passes around the FFTs: `field @ window`, kernel
 // materialisation, and multi-bin pair products by Parseval.
 //
 // Reference path (pyhermes/utils/convolution.py, io/window.py,
 // theory/corr2pcf.py:366-372): materialise a float64 kernel array of
 // L^2 (L/2+1) values per window (8 images x W(k) per mode), then
 // irfftn(rfftn(eps) * K), then mean(conv * eps2) -- two FFTs and a kernel
-// build per bin.  Here the kernel is evaluated on the fly in the pass that
+// build per bin.  Here a window whose 8 images fold to a table by symmetry is
+// applied from that table, any other is evaluated on the fly in the pass that
 // touches the spectrum, and the 2PCF products of every bin are one pass over
-// the half spectra:  sum_x (f1 * K)(x) f2(x) / L^3 = sum_k F1 K conj(F2) / L^6.
+// the half spectra (radial bins: over their histogram by |k|^2):
+// sum_x (f1 * K)(x) f2(x) / L^3 = sum_k F1 K conj(F2) / L^6.
 #include <cufft.h>
 
 #include <algorithm>
