@@ -168,7 +168,12 @@ typedef struct hermes_window {
 
 /* Forward / inverse 3D FFTs in float32 (the reference's scipy.fft rfftn,
  * irfftn, fftn, ifftn in utils/convolution.py:284-295).  Unnormalised like
- * cuFFT (the inverse passes below fold in 1/L^3).  C2R overwrites `spec`. */
+ * cuFFT (the inverse passes below fold in 1/L^3).  C2R overwrites `spec`.
+ * hermes_fft_r2c_ws: the same transform with a workspace of
+ * hermes_fft_r2c_workspace_size bytes (0 but for J = 9), which the library's own
+ * passes use at J = 9 (about 0.6 GB). */
+int hermes_fft_r2c_workspace_size(int J, size_t* bytes);
+int hermes_fft_r2c_ws(const float* field, void* spec, int J, void* workspace, size_t workspace_bytes, void* stream);
 int hermes_fft_r2c(const float* field, void* spec /* float2 [L,L,L/2+1] */,
                    int J, void* stream);
 int hermes_fft_c2r(void* spec, float* field, int J, void* stream);

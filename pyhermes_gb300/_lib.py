@@ -37,6 +37,8 @@ SIGNATURES = {
     "hermes_field_sum": (_c_int, [_p, _c_i64, _p, _p, _c_sz, _p]),
     "hermes_field_shift": (_c_int, [_p, _c_i64, _dbl, _p, _p]),
     "hermes_fft_r2c": (_c_int, [_p, _p, _c_int, _p]),
+    "hermes_fft_r2c_workspace_size": (_c_int, [_c_int, ctypes.POINTER(ctypes.c_size_t)]),
+    "hermes_fft_r2c_ws": (_c_int, [_p, _p, _c_int, _p, ctypes.c_size_t, _p]),
     "hermes_fft_c2r": (_c_int, [_p, _p, _c_int, _p]),
     "hermes_window_workspace_size": (_c_int, [_c_int, ctypes.POINTER(_c_sz)]),
     "hermes_window_apply": (_c_int, [_p, _p, _c_int, _p, _p, _c_int, _p, _c_sz, _p]),

@@ -26,7 +26,7 @@
 namespace hermes {
 namespace {
 
-enum { kInverse = 0, kForward = 1, kFused = 2 };
+enum { kInverse = 0, kForward = 1, kFused = 2, kCompact = 3 };
 constexpr int kLen = 512;
 constexpr int kPitch = kLen + 1;  // float2 per column in shared memory (odd: conflict-free columns)
 
@@ -112,10 +112,12 @@ __device__ __forceinline__ void fft512_registers(float2 (&v)[kR][8], float2* buf
 }
 
 // kHalf: half spectra of 257 columns with rows of kHalfPitch values, else full
-// fields of 512 columns.
+// fields of 512 columns.  kCompact: the forward x pass from such rows to `out`,
+// [512][512][257]; its 128-byte rows start on any 8 bytes, which the stores do
+// not mind (0.236 ms; cuFFT's compact passes 0.255 ms each).
 template <int kMode, bool kHalf>
 __global__ void __launch_bounds__(kThreads, 1)
-fft512_cols_kernel(float2* __restrict__ data, int nf, int axis, FftWindow win) {
+fft512_cols_kernel(float2* __restrict__ data, int nf, int axis, FftWindow win, float2* __restrict__ out) {
   constexpr int C = kCols, T = kThreads, R = kR;
   constexpr int kRow = kHalf ? kFft512HalfPitch : kLen;
   extern __shared__ __align__(16) float2 sm[];
@@ -218,9 +220,18 @@ fft512_cols_kernel(float2* __restrict__ data, int nf, int axis, FftWindow win) {
     __syncthreads();  // buffer free: the next iteration prefetches into it
     float2* g = tile_ptr(t);
     [[maybe_unused]] const long long cs = kHalf && t >= nfull ? astride : 1;
+    if constexpr (kMode == kCompact) {
+      int a, z;
+      long long unused;
+      half_tile(t, a, z, unused);
+      g = out + (long long)a * (kLen / 2 + 1) + z;
+    }
+    constexpr long long kOutRow = (long long)kLen * (kLen / 2 + 1);
     auto store = [&](int r, int q1) {
       const int i = threadIdx.x + T * r, c = i % C, k0 = i / C;
-      g[(long long)(k0 + 64 * q1) * rstride + (kHalf ? c * cs : c)] = kMode == kForward ? swapped(v[r][q1]) : v[r][q1];
+      if constexpr (kMode == kCompact)
+        g[(k0 + 64 * q1) * kOutRow + (cs == 1 ? c : c * (kLen / 2 + 1))] = swapped(v[r][q1]);
+      else g[(long long)(k0 + 64 * q1) * rstride + (kHalf ? c * cs : c)] = kMode == kForward ? swapped(v[r][q1]) : v[r][q1];
     };
     // The order of the row stores decides the x pass (rows 2 MB apart): both
     // transforms' rows of one q1 together 5.1 ms for 15 fields, one
@@ -394,7 +405,7 @@ int launch_fft_cols(float2* data, int nf, int axis, cudaStream_t s) {
 }
 
 template <int kMode, bool kHalf>
-int launch_cols(float2* data, int nf, int axis, const FftWindow& win, cudaStream_t s) {
+int launch_cols(float2* data, int nf, int axis, const FftWindow& win, cudaStream_t s, float2* out = nullptr) {
   constexpr size_t smem = sizeof(float2) * (3 * (size_t)kBuf + kLen) + (kMode == kFused ? sizeof(float) * kLen : 0);
   static bool attr_set[64] = {false};
   int dev = 0;
@@ -407,7 +418,7 @@ int launch_cols(float2* data, int nf, int axis, const FftWindow& win, cudaStream
   int nsm = 0;
   HERMES_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   // one block per SM: every shape has more tiles (8224 at least) than SMs
-  fft512_cols_kernel<kMode, kHalf><<<nsm, kThreads, smem, s>>>(data, nf, axis, win);
+  fft512_cols_kernel<kMode, kHalf><<<nsm, kThreads, smem, s>>>(data, nf, axis, win, out);
   HERMES_LAUNCH_CHECK("fft512_cols_kernel");
   return HERMES_OK;
 }
@@ -453,6 +464,10 @@ int fft512_half_to_real(const float2* in, float* out, cudaStream_t s) {
 int fft512_half_y(float2* data, bool forward, cudaStream_t s) {
   return forward ? launch_cols<kForward, true>(data, 1, 1, FftWindow{}, s)
                  : launch_cols<kInverse, true>(data, 1, 1, FftWindow{}, s);
+}
+
+int fft512_half_x_compact(float2* data, float2* out, cudaStream_t s) {
+  return launch_cols<kCompact, true>(data, 1, 0, FftWindow{}, s, out);
 }
 
 int fft512_half_x_window_x(float2* data, const FftWindow& win, cudaStream_t s) {

@@ -26,6 +26,8 @@ int fft512_real_to_half(const float* in, float2* out, cudaStream_t s);
 int fft512_half_to_real(const float2* in, float* out, cudaStream_t s);
 // y transform, in place, unnormalised.
 int fft512_half_y(float2* data, bool forward, cudaStream_t s);
+// Forward x transform into compact rows, out[512][512][257]; data is left as it is.
+int fft512_half_x_compact(float2* data, float2* out, cudaStream_t s);
 // Forward x transform, the window, inverse x transform, in place.
 int fft512_half_x_window_x(float2* data, const FftWindow& win, cudaStream_t s);
 

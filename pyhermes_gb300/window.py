@@ -613,7 +613,12 @@ def rfft_field(eps):
     L = eps.shape[0]
     J = L.bit_length() - 1
     spec = torch.empty((L, L, L // 2 + 1), dtype=torch.complex64, device=eps.device)
-    _lib.check(_lib.load().hermes_fft_r2c(_ptr(eps), _ptr(spec), J, _stream_ptr(eps.device)), "hermes_fft_r2c")
+    lib = _lib.load()
+    need = ctypes.c_size_t(0)
+    _lib.check(lib.hermes_fft_r2c_workspace_size(J, ctypes.byref(need)), "hermes_fft_r2c_workspace_size")
+    ws = torch.empty(need.value, dtype=torch.uint8, device=eps.device)
+    _lib.check(lib.hermes_fft_r2c_ws(_ptr(eps), _ptr(spec), J, _ptr(ws), need.value, _stream_ptr(eps.device)),
+               "hermes_fft_r2c_ws")
     return spec
 
 

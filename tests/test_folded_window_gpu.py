@@ -8,6 +8,8 @@ another grouping, so each mode differs by at most about 10 roundings of
 2^-24 = 6e-7 of it, and the fields by 1e-6 in the 2-norm.  A float32
 transform of 512^3 values is off by a few 1e-7 in the 2-norm (log2 N roundings
 adding at random): 1e-6."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -59,3 +61,20 @@ def test_real_transforms_at_512():
     back = torch.empty_like(f)
     _lib.check(_lib.load().hermes_fft_c2r(_ptr(s), _ptr(back), 9, _stream_ptr(f.device)), "hermes_fft_c2r")
     assert (back / 512 ** 3 - f).double().norm() <= 1e-6 * f.double().norm()
+
+
+@pytest.mark.parametrize("J,shift", [(6, 0), (9, 0), (9, 8)])
+def test_transform_with_a_workspace(J, shift):
+    """Own passes (aligned workspace at J = 9) and the plan agree; a workspace
+    that is too small is refused."""
+    L, lib = 1 << J, _lib.load()
+    f = torch.randn((L,) * 3, generator=torch.Generator(device="cuda").manual_seed(J), device="cuda")
+    need = ctypes.c_size_t()
+    _lib.check(lib.hermes_fft_r2c_workspace_size(J, ctypes.byref(need)), "size")
+    ws = torch.empty(need.value + 16, dtype=torch.uint8, device="cuda")[shift:]
+    got, ref = (torch.empty((L, L, L // 2 + 1), dtype=torch.complex64, device="cuda") for _ in range(2))
+    _lib.check(lib.hermes_fft_r2c_ws(_ptr(f), _ptr(got), J, _ptr(ws), need.value, _stream_ptr(f.device)), "ws")
+    _lib.check(lib.hermes_fft_r2c(_ptr(f), _ptr(ref), J, _stream_ptr(f.device)), "plan")
+    assert (got - ref).to(torch.complex128).norm() <= 2e-6 * ref.to(torch.complex128).norm()
+    if need.value:
+        assert lib.hermes_fft_r2c_ws(_ptr(f), _ptr(got), J, _ptr(ws), need.value - 1, _stream_ptr(f.device)) != 0
