@@ -120,10 +120,11 @@ pp_hist_kernel(const float* __restrict__ T, int L, const double* __restrict__ pd
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (kHistThreads / 32);
   int shift[NP];
+  bool finite[NP];  // a pair that is not finite is left out: its bins report NaN
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
     const unsigned mb = maxbits[p];
-    if (mb >= 0x7F800000u) return;  // not finite: the bins report NaN
+    finite[p] = mb < 0x7F800000u;
     shift[p] = hist_shift(mb);
   }
   for (int c = blockIdx.x * (kHistThreads / 32) + (threadIdx.x >> 5); c < ncol; c += nw) {
@@ -143,6 +144,7 @@ pp_hist_kernel(const float* __restrict__ T, int L, const double* __restrict__ pd
       const float p1 = P[z], p2 = P[L - z];
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
+        if (!finite[p]) continue;
         const float* Tp = T + (size_t)p * ncol * H;
         float t = Tp[(size_t)c * H + z];
         if (y != z) t += Tp[(size_t)(cx + z) * H + y];
