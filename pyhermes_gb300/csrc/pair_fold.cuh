@@ -19,7 +19,13 @@
 // more, onto x >= y >= z) and pp_radial_bins_kernel evaluates each bin's window
 // once per n2, 3 L^2 + 1 values, instead of 8 times per mode.  The histogram
 // is in 64-bit fixed point (exponent from the largest |T|), so its sums are
-// exact and do not depend on the order of the atomics.
+// exact and do not depend on the order of the atomics.  It has two levels: a
+// contribution that is a whole number of quanta, 2^-46 of the largest |T|, goes
+// to the first, any other to the second, whose quanta are 2^-26 of those.  All 24
+// bits of a float32 contribution therefore count down to 2^-48 of the largest |T|
+// (one level lost them from 2^-18 on, and a mode below 2^-43 altogether: a window
+// that does not weigh the large modes, over a mean or a steep spectrum, then
+// had no more than its strongest few bits).
 #pragma once
 
 #include "pair_products.cuh"
@@ -27,7 +33,12 @@
 namespace hermes {
 
 constexpr int kHistThreads = 256;
-constexpr int kHistBits = 42;       // max |T| < 2^42 quanta: 2^20 additions cannot overflow
+// max |T| < 2^46 quanta.  pp_hist_kernel adds sums of up to three T, and an n2
+// has at most 3234 images (L = 1024): below 2^60.  Values below 2^24 quanta, of the
+// second level's below 2^50, stay below 2^62 there.
+constexpr int kHistBits = 46;
+constexpr int kFineBits = 26;
+constexpr int kLevels = 2;
 constexpr int kRadialPerBlock = 4096;
 constexpr int kRadialBins = 4;      // bins per block of pp_radial_bins_kernel
 
@@ -86,26 +97,25 @@ pp_fold_kernel(const float2* __restrict__ si, const float2* __restrict__ sj, int
 }
 
 // Exponent shift of the fixed point: quanta = v * 2^shift, |v| <= the largest |T|.
-__device__ __forceinline__ int hist_shift(unsigned maxbits) { return kHistBits + 126 - (int)(maxbits >> 23); }
+__device__ __forceinline__ int hist_shift(unsigned maxbits) { return kHistBits + 126 - max((int)(maxbits >> 23), 1); }
 
-// v * 2^shift rounded to the nearest integer (ties away from zero), with
-// integer operations only; |v| 2^shift < 2^62.
-__device__ __forceinline__ long long f32_shifted_ll(float v, int shift) {
+// hist[level][n2] += v in the level's quanta (exact in the first level; in the
+// second rounded to the nearest integer, ties away from zero), with integer
+// operations only.
+__device__ __forceinline__ void hist_add(unsigned long long* __restrict__ hist, int nh, int n2, float v, int shift) {
   const int b = __float_as_int(v);
   const int e = (b >> 23) & 0xFF;
-  if (e == 0) return 0;  // zero or subnormal
-  const long long m = (long long)((b & 0x7FFFFF) | 0x800000);
-  const int up = e + shift - 150;
-  long long q;
-  if (up >= 0) {
-    q = m << up;
-  } else {
-    q = up <= -25 ? 0 : ((m + (1LL << (-up - 1))) >> -up);
+  const long long m = e ? (b & 0x7FFFFF) | 0x800000 : b & 0x7FFFFF;  // v = m 2^(max(e, 1) - 150)
+  int up = max(e, 1) + shift - 150;
+  if (up < 0) {
+    up += kFineBits;
+    hist += nh;
   }
-  return b < 0 ? -q : q;
+  const long long q = up >= 0 ? m << up : (up <= -25 ? 0 : ((m + (1LL << (-up - 1))) >> -up));
+  if (q) atomicAdd(hist + n2, (unsigned long long)(b < 0 ? -q : q));
 }
 
-// hist[p][n2] += P(a) P(b) P(c) T over the images (a, b, c) of every mode with
+// hist[p][level][n2] += P(a) P(b) P(c) T over the images (a, b, c) of every mode with
 // x >= y >= z, T the sum over the places that z can take among the three (each
 // once); one warp per column (x, y), lanes along z.  J = 9: 0.12 ms a
 // pair, 0.33 folded over x and y alone.
@@ -149,12 +159,11 @@ pp_hist_kernel(const float* __restrict__ T, int L, const double* __restrict__ pd
         float t = Tp[(size_t)c * H + z];
         if (y != z) t += Tp[(size_t)(cx + z) * H + y];
         if (x != y) t += Tp[(size_t)(cy + z) * H + x];
-        unsigned long long* h = hist + (size_t)p * nh;
+        unsigned long long* h = hist + (size_t)p * kLevels * nh;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const long long q1 = f32_shifted_ll(w[i] * p1 * t, shift[p]), q2 = f32_shifted_ll(w[i] * p2 * t, shift[p]);
-          if (q1) atomicAdd(h + s[i] + z2, (unsigned long long)q1);
-          if (q2) atomicAdd(h + s[i] + m2, (unsigned long long)q2);
+          hist_add(h, nh, s[i] + z2, w[i] * p1 * t, shift[p]);
+          hist_add(h, nh, s[i] + m2, w[i] * p2 * t, shift[p]);
         }
       }
     }
@@ -188,9 +197,10 @@ pp_radial_bins_kernel(const WinDev* __restrict__ wins, int n_bins, int L, const 
     bool any = false;
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-      const long long q = (long long)hist[(size_t)p * nh + n2];
-      any = any || q != 0;
-      h[p] = (double)q;
+      const unsigned long long* hp = hist + (size_t)p * kLevels * nh + n2;
+      const long long q = (long long)hp[0], f = (long long)hp[nh];
+      any = any || (q | f) != 0;
+      h[p] = fma((double)f, 1.0 / (1 << kFineBits), (double)q);
     }
     if (!any) continue;
 #pragma unroll

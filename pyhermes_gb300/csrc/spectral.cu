@@ -792,7 +792,7 @@ struct PPWs {
   unsigned* maxbits;         // [n_pairs]
   union {                    // one of the two folded passes runs
     float* atab;             // A table of cylindrical bins [folded columns][nbp]
-    unsigned long long* hist;  // histogram over n2 [n_pairs][3 L^2 + 1]
+    unsigned long long* hist;  // histogram over n2 [n_pairs][kLevels][3 L^2 + 1]
   };
   size_t used;
 };
@@ -810,7 +810,7 @@ PPWs pp_carve(void* ws, size_t cap, int J, int n_bins, int n_pairs) {
   w.maxbits = c.take<unsigned>((size_t)n_pairs);
   w.fold = c.take<float>(n_pairs * ncol * H);
   const size_t shared = std::max(ncol * (size_t)cylz_nbp(n_bins) * sizeof(float),
-                                 n_pairs * (3 * (size_t)L * L + 1) * sizeof(unsigned long long));
+                                 n_pairs * kLevels * (3 * (size_t)L * L + 1) * sizeof(unsigned long long));
   w.hist = reinterpret_cast<unsigned long long*>(c.take<char>(shared));
   w.used = c.used;
   return w;
@@ -835,7 +835,7 @@ int pp_folded(const PPArgs& a, const PPWs& w, const double* phi_power, bool radi
   if (radial) {
     const int nh = 3 * L * L + 1;
     const size_t psm = sizeof(float) * (size_t)(L + 1);
-    HERMES_CUDA_TRY(cudaMemsetAsync(w.hist, 0, sizeof(unsigned long long) * NP * (size_t)nh, s));
+    HERMES_CUDA_TRY(cudaMemsetAsync(w.hist, 0, sizeof(unsigned long long) * NP * kLevels * (size_t)nh, s));
     pp_hist_kernel<NP><<<fold_grid, kHistThreads, psm, s>>>(w.fold, L, phi_power, w.maxbits, w.hist, nh);
     HERMES_LAUNCH_CHECK("pp_hist_kernel");
     *nblk = (nh + kRadialPerBlock - 1) / kRadialPerBlock;
