@@ -11,15 +11,10 @@
 namespace {
 
 using hermes::fail;
+using hermes::two_sum;
 
 constexpr int kThreads = 256;
 constexpr int kMaxBlocks = 2048;
-
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-  s = __fadd_rn(a, b);
-  const float bb = __fsub_rn(s, a);
-  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-}
 
 // float64 sum of a block (fixed order).
 __device__ __forceinline__ double block_sum(double v) {

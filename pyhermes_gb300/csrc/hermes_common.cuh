@@ -49,6 +49,15 @@ struct Carver {
   } while (0)
 
 // ---- device helpers --------------------------------------------------------
+namespace hermes {
+// s = a + b rounded and its rounding error e, a + b = s + e (Knuth's two-sum).
+__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
+  s = __fadd_rn(a, b);
+  const float bb = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+}
+}  // namespace hermes
+
 __device__ __forceinline__ int wrap_mod(int v, int L) {  // L is a power of two
   return v & (L - 1);
 }

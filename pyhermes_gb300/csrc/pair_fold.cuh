@@ -57,6 +57,8 @@ __device__ __forceinline__ void fold_xy(int c, int& x, int& y) {
 
 // T[column][z] of the folded columns of one pair (si, sj), one warp per
 // column; the largest |T| (as float bits; a NaN has the largest) in maxbits.
+// The up to eight products are added with their rounding errors kept (the pass is
+// bound by its reads), so that T is rounded once however they cancel.
 // One launch per pair: 0.11 ms for an auto pair at J = 9 (0.54 GB, 4.9 TB/s);
 // two pairs of different spectra in one launch took 0.57 ms.
 __global__ void __launch_bounds__(kHistThreads)
@@ -75,7 +77,7 @@ pp_fold_kernel(const float2* __restrict__ si, const float2* __restrict__ sj, int
     // rows (x, y), (-x, y), (x, -y), (-x, -y), then the same with x and y exchanged
     const int xs[2] = {x, (L - x) & Lm}, ys[2] = {y, (L - y) & Lm};
     for (int z = lane; z < H; z += 32) {
-      float t = 0.f;
+      float t = 0.f, lost = 0.f;
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
         const int i = r & 1, j = (r >> 1) & 1, s = r >> 2;
@@ -84,10 +86,12 @@ pp_fold_kernel(const float2* __restrict__ si, const float2* __restrict__ sj, int
         const long long m = row * H + z;
         const float2 u = si[m];
         const float2 v = same ? u : sj[m];
-        t += u.x * v.x + u.y * v.y;
+        float e;
+        two_sum(t, u.x * v.x + u.y * v.y, t, e);
+        lost += e;
       }
       const float wgt = (z == 0 || 2 * z == L) ? 1.f : 2.f;
-      const float v = (exclude_k0 && c == 0 && z == 0) ? 0.f : wgt * t;
+      const float v = (exclude_k0 && c == 0 && z == 0) ? 0.f : wgt * (isfinite(t) ? t + lost : t);
       T[(size_t)c * H + z] = v;
       mx = max(mx, __float_as_uint(fabsf(v)));
     }
@@ -131,11 +135,13 @@ pp_hist_kernel(const float* __restrict__ T, int L, const double* __restrict__ pd
   const int nw = gridDim.x * (kHistThreads / 32);
   int shift[NP];
   bool finite[NP];  // a pair that is not finite is left out: its bins report NaN
+  float unit[NP];   // 1/4 where three T could overflow
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
     const unsigned mb = maxbits[p];
     finite[p] = mb < 0x7F800000u;
-    shift[p] = hist_shift(mb);
+    shift[p] = hist_shift(mb) + (mb >= 0x7E000000u ? 2 : 0);
+    unit[p] = mb >= 0x7E000000u ? 0.25f : 1.f;
   }
   for (int c = blockIdx.x * (kHistThreads / 32) + (threadIdx.x >> 5); c < ncol; c += nw) {
     int x, y;
@@ -156,9 +162,10 @@ pp_hist_kernel(const float* __restrict__ T, int L, const double* __restrict__ pd
       for (int p = 0; p < NP; ++p) {
         if (!finite[p]) continue;
         const float* Tp = T + (size_t)p * ncol * H;
-        float t = Tp[(size_t)c * H + z];
-        if (y != z) t += Tp[(size_t)(cx + z) * H + y];
-        if (x != y) t += Tp[(size_t)(cy + z) * H + x];
+        float t, e1, e2;
+        two_sum(unit[p] * Tp[(size_t)c * H + z], y != z ? unit[p] * Tp[(size_t)(cx + z) * H + y] : 0.f, t, e1);
+        two_sum(t, x != y ? unit[p] * Tp[(size_t)(cy + z) * H + x] : 0.f, t, e2);
+        t += e1 + e2;
         unsigned long long* h = hist + (size_t)p * kLevels * nh;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
