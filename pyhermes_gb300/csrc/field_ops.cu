@@ -3,9 +3,9 @@
 // the field minus a mean density.  Both are bound by HBM.  Written with
 // float64 arithmetic they are bound by the float64 pipe (two lanes per SM
 // and clock): a cast-and-sum takes 0.77 ms and a cast, subtract and cast back
-// 1.3 ms for 512^3 cells.  Here the additions are float32 pairs (Knuth's
-// two-sum keeps the rounding error of every addition), and float64 enters
-// once per 16 values: the sum takes 0.093 ms (5.8 TB/s).
+// 1.3 ms for 512^3 cells.  Here the additions are float32 ones that keep their
+// rounding errors (Knuth's two-sum), and float64 enters once per 32 values: the
+// sum takes 0.094 ms (5.7 TB/s), 0.118 ms with float64 once per 16.
 #include "hermes_common.cuh"
 
 namespace {
@@ -28,6 +28,16 @@ __device__ __forceinline__ double block_sum(double v) {
   return s;
 }
 
+// s + c + d += x: s the float32 sum, c the sum of its rounding errors, d the sum of
+// c's.  Up to 32 values then enter float64 with more digits than it has.  An
+// infinity or a NaN in s makes d a NaN.
+__device__ __forceinline__ void add3(float x, float& s, float& c, float& d) {
+  float e;
+  two_sum(s, x, s, e);
+  two_sum(c, e, c, e);
+  d += e;
+}
+
 // partial[block] = sum of x over the block's grid-stride share; kVec: x is
 // 16-byte aligned and read as float4 (the n % 4 last values by block 0).
 template <bool kVec>
@@ -38,30 +48,32 @@ __global__ void __launch_bounds__(kThreads) field_sum_kernel(const float* __rest
   if (kVec) {
     const float4* x4 = reinterpret_cast<const float4*>(x);
     const int64_t n4 = n >> 2;
-    int64_t i = t0;
-    for (; i + 3 * stride < n4; i += 4 * stride) {
-      float4 v[4];
+    for (int64_t i = t0; i < n4;) {
+      const int64_t first = i;
+      float s = 0.f, c = 0.f, d = 0.f;
+      auto add = [&](const float4& v) {
+        add3(v.x, s, c, d);
+        add3(v.y, s, c, d);
+        add3(v.z, s, c, d);
+        add3(v.w, s, c, d);
+      };
+      for (int g = 0; g < 2 && i + 3 * stride < n4; ++g, i += 4 * stride) {
+        float4 v[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) v[k] = __ldcs(x4 + i + k * stride);
-      float s = v[0].x, c = 0.f, e;
+        for (int k = 0; k < 4; ++k) v[k] = __ldcs(x4 + i + k * stride);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (k > 0) {
-          two_sum(s, v[k].x, s, e);
-          c += e;
-        }
-        two_sum(s, v[k].y, s, e);
-        c += e;
-        two_sum(s, v[k].z, s, e);
-        c += e;
-        two_sum(s, v[k].w, s, e);
-        c += e;
+        for (int k = 0; k < 4; ++k) add(v[k]);
       }
-      acc += (double)s + (double)c;
-    }
-    for (; i < n4; i += stride) {
-      const float4 v = x4[i];
-      acc += ((double)v.x + (double)v.y) + ((double)v.z + (double)v.w);
+      if (i == first)  // the last one to three
+        for (; i < n4; i += stride) add(x4[i]);
+      if (isfinite(d)) {
+        acc += (double)s + ((double)c + (double)d);
+      } else {  // an infinity, a NaN or a float32 overflow of s: as float64 gives it
+        for (int64_t j = first; j < i; j += stride) {
+          const float4 v = x4[j];
+          acc += ((double)v.x + (double)v.y) + ((double)v.z + (double)v.w);
+        }
+      }
     }
     if (blockIdx.x == 0 && threadIdx.x < (n & 3)) acc += (double)x[(n4 << 2) + threadIdx.x];
   } else {
