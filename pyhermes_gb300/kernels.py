@@ -48,8 +48,8 @@ def field_sum(t):
 
 
 def field_shift(t, r):
-    """t - r rounded once to float32, r a Python float: hermes_field_shift for
-    a contiguous float32 CUDA tensor, else torch."""
+    """(t.double() - r).to(float32), r a Python float: hermes_field_shift (the
+    same bits) for a contiguous float32 CUDA tensor, else torch."""
     if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
         return (t.double() - r).to(torch.float32)
     out = torch.empty_like(t)
