@@ -154,7 +154,7 @@ class BatchPipeline:
                 specs, dcs = [], []
                 for t in tasks:
                     t.prepare_input_fields()
-                    d = t.data[1].epsilon_device.to(torch.float32).contiguous()
+                    d = t.data[1]._coefficients().to(torch.float32).contiguous()
                     specs.append(rfft_field(d))
                     dcs.append(float(d.double().sum().item()))
                 if windows is None:

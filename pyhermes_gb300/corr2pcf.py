@@ -382,9 +382,7 @@ class Corr_2PCF:
 
     def _apply_window(self, field, win):
         if win is None:
-            out = field.copy()
-            out.format_sfc_params()
-            return out
+            return field._snapshot()
         w = win if isinstance(win, WindowFunc) else WindowFunc(win, field.sfc_info, threads=self.threads,
                                                                 device=self.device)
         return field @ w
@@ -394,7 +392,7 @@ class Corr_2PCF:
         field = self._resolve_field(value, what)
         base = self._field_in_task_normalization(field)
         if win is None and base is not field:
-            return base  # already a copy of the input
+            return base  # rescaled: the task's own
         return self._apply_window(base, win)
 
     def prepare_input_fields(self):
@@ -408,7 +406,7 @@ class Corr_2PCF:
             win = getattr(self, f"window{i}")
             if needs_data:
                 if i == 2 and plain and isinstance(self.sfc_field1, SFCField) and self.sfc_field2 is self.sfc_field1:
-                    self.data[i] = self.data[1]._same_coefficients()
+                    self.data[i] = self.data[1]._snapshot()
                 else:
                     self.data[i] = self._vertex_field(getattr(self, f"sfc_field{i}"), win, f"field vertex {i}")
             if needs_random:
@@ -425,7 +423,7 @@ class Corr_2PCF:
                         raise ValueError("random='uniform' requires a SFCField field with a defined field_integral.")
                     self.rand[i] = field_mean_density(ref)
                 elif i == 2 and plain and isinstance(r, SFCField) and r is self.random1:
-                    self.rand[i] = self.rand[1]._same_coefficients()
+                    self.rand[i] = self.rand[1]._snapshot()
                 else:
                     self.rand[i] = self._vertex_field(r, win, f"random vertex {i}")
         self._fields_prepared = True
@@ -498,7 +496,7 @@ class Corr_2PCF:
         def shared(group):
             # both vertices hold the same coefficient tensor
             a, b = group.get(1), group.get(2)
-            return isinstance(a, SFCField) and isinstance(b, SFCField) and a.epsilon_device is b.epsilon_device
+            return isinstance(a, SFCField) and isinstance(b, SFCField) and a._coefficients() is b._coefficients()
 
         same = {"D": shared(self.data), "R": shared(self.rand)}
         same["d"] = same["D"] and same["R"]
@@ -531,10 +529,10 @@ class Corr_2PCF:
                 if spec_key not in field_keys:
                     side = int(spec_key[1])
                     if spec_key[0] == "d":  # delta against a random field: transform D - R itself
-                        fld_t = field_difference(self.data[side].epsilon_device, self.rand[side].epsilon_device)
+                        fld_t = field_difference(self.data[side]._coefficients(), self.rand[side]._coefficients())
                     else:
                         fld = self.data[side] if spec_key[0] == "D" else self.rand[side]
-                        fld_t = fld.epsilon_device.to(torch.float32).contiguous()
+                        fld_t = fld._coefficients().to(torch.float32).contiguous()
                     field_keys[spec_key] = len(spectra)
                     spectra.append(rfft_field(fld_t))
                     reals.append(fld_t)

@@ -262,7 +262,7 @@ def convolve_complex_full(field, window):
     complex64 [L, L, L] device tensor (utils/convolution.py:291-295), from
     the multipole field kernels."""
     l, m, b = complex_full_window_bin(window)
-    spec = rfft_field(field.epsilon_device.to(torch.float32).contiguous())
+    spec = rfft_field(field._coefficients().to(torch.float32).contiguous())
     a = multipole_fields_bins(spec, window.J, l, m, [b], window.box_size, window.phi_power())
     return a.view(window.L, window.L, window.L)
 
@@ -995,6 +995,8 @@ class Corr_3PCF_Multipole:
         needs_random = any(p in exp for p in ("rrr_l", "delta_ddd_l", "zeta_l"))
         self.data, self.rand = {}, {}
         ref = self._normalized(self._resolve(self.sfc_field1, "field vertex 1"))
+        if ref is self.sfc_field1:  # the task's fields are its own
+            ref = ref._snapshot()
         self.reference = ref
         self.rho = ref.field_mean_density(value_unit="grid")
         # per-vertex density of the normalised field before its window
@@ -1009,10 +1011,12 @@ class Corr_3PCF_Multipole:
                          None)
                 base = ref if i == 1 else normalized[j] if j else \
                     self._normalized(self._resolve(value, f"field vertex {i}"))
+                w = getattr(self, f"window{i}")
+                if base is value and not w:
+                    base = base._snapshot()
                 normalized[i] = base
                 self.rho_vertices[i - 1] = base.field_mean_density(value_unit="grid")
-                w = getattr(self, f"window{i}")
-                self.data[i] = base @ WindowFunc(w, base.sfc_info, device=self.device) if w else base._same_coefficients()
+                self.data[i] = base @ WindowFunc(w, base.sfc_info, device=self.device) if w else base._snapshot()
             if needs_random:
                 r = getattr(self, f"random{i}")
                 if r is None or r == "":
@@ -1025,10 +1029,11 @@ class Corr_3PCF_Multipole:
                     j = next((j for j in range(1, i) if not w and not getattr(self, f"window{j}")
                               and isinstance(r, SFCField) and getattr(self, f"random{j}") is r), None)
                     if j:
-                        self.rand[i] = self.rand[j]._same_coefficients()
+                        self.rand[i] = self.rand[j]._snapshot()
                         continue
                     base = self._normalized(self._resolve(r, f"random vertex {i}"))
-                    self.rand[i] = base @ WindowFunc(w, base.sfc_info, device=self.device) if w else base
+                    self.rand[i] = base @ WindowFunc(w, base.sfc_info, device=self.device) if w else \
+                        base._snapshot() if base is r else base
         self.radial_profile_diagnostics = self._radial_profile_diagnostics()
         self._fields_prepared = True
 
@@ -1056,17 +1061,17 @@ class Corr_3PCF_Multipole:
 
     def _eps(self, product, i):
         if product == "ddd_l":
-            return self.data[i].epsilon_device.to(torch.float32)
+            return self.data[i]._coefficients().to(torch.float32)
         if product == "delta_ddd_l":
             r = self.rand[i]
-            d = self.data[i].epsilon_device
+            d = self.data[i]._coefficients()
             if isinstance(r, float):
                 return field_shift(d, r)
-            return field_difference(d, r.epsilon_device)
+            return field_difference(d, r._coefficients())
         r = self.rand[i]
         if isinstance(r, float):
             return torch.full((self.reference.L,) * 3, r, dtype=torch.float32, device=self.device)
-        return r.epsilon_device.to(torch.float32)
+        return r._coefficients().to(torch.float32)
 
     def _same_vertex(self, product, i, j):
         """Whether vertices i and j have the same field in a product."""
@@ -1074,7 +1079,7 @@ class Corr_3PCF_Multipole:
             a, b = group.get(i), group.get(j)
             if isinstance(a, float) or isinstance(b, float):
                 return isinstance(a, float) and isinstance(b, float) and a == b
-            return a is not None and b is not None and a.epsilon_device is b.epsilon_device
+            return a is not None and b is not None and a._coefficients() is b._coefficients()
 
         return (product == "rrr_l" or same(self.data)) and (product == "ddd_l" or same(self.rand))
 

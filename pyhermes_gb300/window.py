@@ -582,7 +582,7 @@ def convolve_field(field, window):
     """SFCField @ WindowFunc (io/sfc_field.py:93-150) on the GPU."""
     if not isinstance(window, WindowFunc):
         raise TypeError(f"Convolution requires a WindowFunc on the right-hand side; got {type(window)}.")
-    eps = field.epsilon_device
+    eps = field._coefficients()
     if eps is None or eps.ndim != 3:
         raise ValueError("Convolution expects a 3D field.")
     if eps.shape[0] != window.L:
