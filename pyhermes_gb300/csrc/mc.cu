@@ -388,9 +388,24 @@ mc_sample_kernel(const float* __restrict__ eps1, const float* __restrict__ eps2,
   }
 }
 
-// dst[mc_cell<true>(x, y, z)] = src[mc_cell<false>(x, y, z)]: one thread per
-// destination element, so the writes are contiguous; a warp's 32 reads are
-// 4 bricks = 8 rows of 2 cells.
+// dst[mc_cell<true>(x, y, z)] = src[mc_cell<false>(x, y, z)], one thread per
+// brick: the four 8-byte reads of a warp are 256 contiguous bytes each, its
+// 32-byte writes 1 KB.  src 8-byte and dst 32-byte aligned.
+__global__ void __launch_bounds__(256) mc_bricks_kernel(const float* __restrict__ src, int J, float* __restrict__ dst) {
+  const int h = J - 1;
+  const unsigned n = 1u << (3 * h), hm = (1u << h) - 1;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const unsigned x = i >> (2 * h), y = (i >> h) & hm, z = i & hm;
+    const float2* row = reinterpret_cast<const float2*>(src) + ((((size_t)(2 * x) << J) + 2 * y) << h) + z;
+    const size_t dy = (size_t)1 << h, dx = dy << J;
+    const float2 a = __ldcs(row), b = __ldcs(row + dy), c = __ldcs(row + dx), d = __ldcs(row + dx + dy);
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + ((size_t)i << 3)), "f"(a.x), "f"(a.y),
+                 "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y), "f"(d.x), "f"(d.y)
+                 : "memory");
+  }
+}
+
+// The same at any alignment, one thread per cell.
 __global__ void mc_to_bricks_kernel(const float* __restrict__ src, int J, float* __restrict__ dst) {
   const size_t n = (size_t)1 << (3 * J);
   const int h = J - 1;
@@ -574,7 +589,8 @@ extern "C" int hermes_field_to_bricks(const float* field, int J, float* bricks, 
   if (!field || !bricks) return fail(HERMES_ERR_INVALID, "field_to_bricks: NULL argument");
   if (J < 2 || J > 10) return fail(HERMES_ERR_INVALID, "field_to_bricks: J=%d outside [2,10]", J);
   if (field == bricks) return fail(HERMES_ERR_INVALID, "field_to_bricks: the copy cannot be in place");
-  mc_to_bricks_kernel<<<mc_grid(), 256, 0, hermes::as_stream(stream)>>>(field, J, bricks);
+  const auto kernel = aligned(8, field) && aligned(32, bricks) ? mc_bricks_kernel : mc_to_bricks_kernel;
+  kernel<<<mc_grid(), 256, 0, hermes::as_stream(stream)>>>(field, J, bricks);
   HERMES_LAUNCH_CHECK("mc_to_bricks_kernel");
   return HERMES_OK;
 }
