@@ -16,6 +16,8 @@ import copy
 import ctypes
 import inspect
 import os
+import threading
+from collections import OrderedDict
 
 import numpy as np
 import torch
@@ -200,23 +202,37 @@ def custom_window_kernel(func, args, L, bandwidth, power, mode, rows=8):
 
 _POWER_CACHE = {}
 _POWER_KEEP = 64
+_POWER_HOST = OrderedDict()  # the tables on the host, the least recently used first
+_POWER_HOST_KEEP = 256
+_POWER_LOCK = threading.Lock()
 
 
 def phi_power_device(phi_array, L, bandwidth, phi_resolution, device):
     """|phi_hat|^2 at n/L, n = 0..L*bw, as a float64 device tensor.  Kept by
     the samples' values (every copy of a field carries its own phi array; the
-    direct transform takes 22 ms on the host at L = 512), for the first
-    _POWER_KEEP combinations: entries are never replaced, so a tensor that
-    another stream still reads is not freed."""
+    direct transform takes 22 ms on the host at L = 512): the first
+    _POWER_KEEP combinations on the device, never replaced, so that a tensor
+    that another stream still reads is not freed, and the last
+    _POWER_HOST_KEEP in use on the host, from which any other is uploaded."""
     device = torch.device(device)
     if device.type == "cuda" and device.index is None:
         device = torch.device("cuda", torch.cuda.current_device())
     phi = np.ascontiguousarray(phi_array, dtype=np.float64)
-    key = (phi.tobytes(), int(L), int(bandwidth), int(phi_resolution), str(device))
-    t = _POWER_CACHE.get(key)
-    if t is None:
+    table = (phi.tobytes(), int(L), int(bandwidth), int(phi_resolution))
+    key = table + (str(device),)
+    with _POWER_LOCK:
+        t, p = _POWER_CACHE.get(key), _POWER_HOST.get(table)
+        if p is not None:
+            _POWER_HOST.move_to_end(table)
+    if t is not None:
+        return t
+    if p is None:
         p = fourier_power_spectrum(phi, bandwidth, L * bandwidth, phi_resolution)
-        t = torch.as_tensor(p, dtype=torch.float64, device=device)
+    t = torch.tensor(p, dtype=torch.float64, device=device)
+    with _POWER_LOCK:
+        _POWER_HOST[table] = p
+        while len(_POWER_HOST) > _POWER_HOST_KEEP:
+            _POWER_HOST.popitem(last=False)
         if len(_POWER_CACHE) < _POWER_KEEP:
             _POWER_CACHE[key] = t
     return t
