@@ -590,9 +590,10 @@ class MultipoleEngine:
             # one BinSpec per distinct radius (a grid of samples repeats each many times)
             if isinstance(v, BinSpec):
                 return v
-            if v not in made:
-                made[v] = as_bin(v)
-            return made[v]
+            r = float(v)
+            if r not in made:
+                made[r] = as_bin(r)
+            return made[r]
 
         pairs = [(bin_of(a), bin_of(b)) for a, b in pairs]
 
