@@ -632,7 +632,11 @@ def rfft_field(eps):
     lib = _lib.load()
     need = ctypes.c_size_t(0)
     _lib.check(lib.hermes_fft_r2c_workspace_size(J, ctypes.byref(need)), "hermes_fft_r2c_workspace_size")
-    ws = torch.empty(need.value, dtype=torch.uint8, device=eps.device)
+    try:
+        ws = torch.empty(need.value, dtype=torch.uint8, device=eps.device)
+    except torch.OutOfMemoryError:  # no room for the own passes: the plan, which needs none
+        _lib.check(lib.hermes_fft_r2c(_ptr(eps), _ptr(spec), J, _stream_ptr(eps.device)), "hermes_fft_r2c")
+        return spec
     _lib.check(lib.hermes_fft_r2c_ws(_ptr(eps), _ptr(spec), J, _ptr(ws), need.value, _stream_ptr(eps.device)),
                "hermes_fft_r2c_ws")
     return spec
