@@ -468,8 +468,9 @@ class Corr_2PCF:
 
     @staticmethod
     def _dc(field):
-        """float64 sum of a field (its k = 0 Fourier coefficient)."""
-        return float(field_sum(field.epsilon_device))
+        """float64 sum of a field (its k = 0 Fourier coefficient), of the real
+        part of a complex one."""
+        return float(field_sum(field.epsilon_device).real)
 
     def run(self, save_result=True, overwrite=False):
         t0 = time.perf_counter()
