@@ -1274,7 +1274,7 @@ mp_contract_tc_kernel(ContractArgs A, const __grid_constant__ CUtensorMap a2map)
   float* araw = reinterpret_cast<float*>(gbf + tcc::kOpBytes);    // [2][64 cells][32] TMA a2 planes
   float2* abuf = reinterpret_cast<float2*>(reinterpret_cast<unsigned char*>(araw) + 2 * tcc::kRawBytes);
   double* dacc = reinterpret_cast<double*>(abuf + 2 * tcc::kA3Buf);  // [16][16][2]
-  float* hring = reinterpret_cast<float*>(dacc + 2 * kMaxBins * kMaxBins);  // [3][kHPlane]
+  float* hring = reinterpret_cast<float*>(dacc + 2 * kMaxBins * kMaxBins);  // [kRing<NT>][kHSlot<NT>]
   constexpr bool kOneBar = kBM && tcc::kRing<NT> == 4;
   float* epsb = hring + tcc::kRing<NT> * kHS;
   uint64_t* bars = reinterpret_cast<uint64_t*>(epsb + 2 * kEps);  // a2 planes [2], mma
@@ -2275,7 +2275,9 @@ static int mp_contract_launch(const float* eps1, const void* fields2, int nb2, c
   const int n_items1 = (L / chunk_x) * (L / ct::TY) * (L / ct::TZ);
   int tiles = engine == kEngineTensorBinMajor ? contract_tiles(std::max(nb2, nb3), n_items1, L, ctas_per_sm, nsm) : 1;
   const int nbl = kBinStride / tiles;
-  if (tiles > 1 && (size_t)(2 * nbl * nbl) * n_items1 > w.n_item_values) tiles = 1;  // a short chunk_x: more items
+  // the workspace holds the tiles' S at the default chunk; a shorter chunk_x has
+  // more tiles, and where they do not fit (5 to 8 bins) they run one at a time
+  if (tiles > 1 && (size_t)(2 * nbl * nbl) * n_items1 > w.n_item_values) tiles = 1;
   const void* fn = engine == kEngineSimt     ? (const void*)mp_contract_kernel
                    : engine == kEngineTensor ? (const void*)mp_contract_tc_kernel<false, 1>
                    : tiles == 1              ? (const void*)mp_contract_tc_kernel<true, 1>

@@ -59,7 +59,7 @@ __device__ __forceinline__ void fold_xy(int c, int& x, int& y) {
 // column; the largest |T| (as float bits; a NaN has the largest) in maxbits.
 // The up to eight products are added with their rounding errors kept (the pass is
 // bound by its reads), so that T is rounded once however they cancel.
-// One launch per pair: 0.11 ms for an auto pair at J = 9 (0.54 GB, 4.9 TB/s);
+// One launch per pair: 0.098 ms for an auto pair at J = 9 (0.54 GB, 5.5 TB/s);
 // two pairs of different spectra in one launch took 0.57 ms.
 __global__ void __launch_bounds__(kHistThreads)
 pp_fold_kernel(const float2* __restrict__ si, const float2* __restrict__ sj, int L, int exclude_k0, float* __restrict__ T,
@@ -121,8 +121,8 @@ __device__ __forceinline__ void hist_add(unsigned long long* __restrict__ hist, 
 
 // hist[p][level][n2] += P(a) P(b) P(c) T over the images (a, b, c) of every mode with
 // x >= y >= z, T the sum over the places that z can take among the three (each
-// once); one warp per column (x, y), lanes along z.  J = 9: 0.12 ms a
-// pair, 0.33 folded over x and y alone.
+// once, their rounding errors kept); one warp per column (x, y), lanes along z.
+// J = 9: 0.13 ms a pair (0.12 with one level), 0.33 folded over x and y alone.
 template <int NP>
 __global__ void __launch_bounds__(kHistThreads)
 pp_hist_kernel(const float* __restrict__ T, int L, const double* __restrict__ pd, const unsigned* __restrict__ maxbits,

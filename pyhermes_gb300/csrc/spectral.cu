@@ -924,9 +924,9 @@ extern "C" int hermes_pair_products(const void* const* spectra, int n_spec, cons
   cudaStream_t s = as_stream(stream);
   HERMES_CUDA_TRY(cudaMemcpyAsync(dwin, hw.data(), sizeof(WinDev) * n_bins, cudaMemcpyHostToDevice, s));
   // The folded passes, at any level and bin count: 30 shells x 2 pairs at
-  // J = 9 take 0.65 ms (fold 0.22, histogram 0.25, bins 0.19), 143.3 ms in
+  // J = 9 take 0.70 ms (fold 0.20, histogram 0.26, bins 0.24), 143.3 ms in
   // the generic kernel; 20 shells at J = 7 0.05 ms, 1.68 ms there; 300 rings
-  // at J = 9 0.57 ms (fold 0.11, A table 0.28, columns 0.18), 1.74 ms over
+  // at J = 9 0.56 ms (fold 0.10, A table 0.28, columns 0.17), 1.74 ms over
   // the unfolded columns.
   const bool radial = bandwidth == 1 && all_radial(hw, exclude_k0 != 0);
   if (radial || (all_cyl_z(hw) && cylz_smem(a.np, L, n_pairs) <= 200 * 1024)) {
