@@ -4,9 +4,9 @@
 // float64 arithmetic they are bound by the float64 pipe (two lanes per SM
 // and clock): a cast-and-sum takes 0.77 ms and a cast, subtract and cast back
 // 1.3 ms for 512^3 cells.  Here the additions are float32 ones that keep their
-// rounding errors (Knuth's two-sum), and float64 enters once per 32 values: the
-// sum takes 0.094 ms (5.7 TB/s), 0.118 ms with float64 once per 16; the shift, with
-// the bits of float64, 0.170 ms (6.3 TB/s).
+// rounding errors (Knuth's two-sum), and float64 enters once per 64 values: the
+// sum takes 0.091 ms (5.9 TB/s), 0.094 and 0.118 ms with float64 once per 32 and
+// 16; the shift, with the bits of float64, 0.170 ms (6.3 TB/s).
 #include <cmath>
 
 #include "hermes_common.cuh"
@@ -32,7 +32,7 @@ __device__ __forceinline__ double block_sum(double v) {
 }
 
 // s + c + d += x: s the float32 sum, c the sum of its rounding errors, d the sum of
-// c's.  Up to 32 values then enter float64 with more digits than it has.  An
+// c's.  Up to 64 values then enter float64 with more digits than it has.  An
 // infinity or a NaN in s makes d a NaN.
 __device__ __forceinline__ void add3(float x, float& s, float& c, float& d) {
   float e;
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kThreads) field_sum_kernel(const float* __rest
         add3(v.z, s, c, d);
         add3(v.w, s, c, d);
       };
-      for (int g = 0; g < 2 && i + 3 * stride < n4; ++g, i += 4 * stride) {
+      for (int g = 0; g < 4 && i + 3 * stride < n4; ++g, i += 4 * stride) {
         float4 v[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) v[k] = __ldcs(x4 + i + k * stride);
