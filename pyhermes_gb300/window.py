@@ -220,12 +220,13 @@ def phi_power_device(phi_array, L, bandwidth, phi_resolution, device):
     phi = np.ascontiguousarray(phi_array, dtype=np.float64)
     table = (phi.tobytes(), int(L), int(bandwidth), int(phi_resolution))
     key = table + (str(device),)
-    with _POWER_LOCK:
-        t, p = _POWER_CACHE.get(key), _POWER_HOST.get(table)
-        if p is not None:
-            _POWER_HOST.move_to_end(table)
+    t = _POWER_CACHE.get(key)
     if t is not None:
         return t
+    with _POWER_LOCK:
+        p = _POWER_HOST.get(table)
+        if p is not None:
+            _POWER_HOST.move_to_end(table)
     if p is None:
         p = fourier_power_spectrum(phi, bandwidth, L * bandwidth, phi_resolution)
     t = torch.tensor(p, dtype=torch.float64, device=device)
