@@ -121,8 +121,8 @@ def choose_bricks(fields, J, n, single=False):
 def _gathered(fields, J, bricks, n, single=False):
     """(fields in the layout that a Monte Carlo call reads, whether that is
     the brick layout)."""
-    if bricks is True:
-        bricks = choose_bricks(fields, J, n, single)
+    if not isinstance(bricks, (tuple, list)):
+        bricks = choose_bricks(fields, J, n, single) if bricks else False
     return (fields, False) if bricks is False else (bricks, True)
 
 

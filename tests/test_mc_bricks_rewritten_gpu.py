@@ -64,8 +64,8 @@ def test_rule_for_the_copies():
     assert mc3pcf.choose_bricks([None, f[0], f[0]], J, L ** 3 // 128)[0] is None
     for n in (line // 3 - 1, line // 3 + 1):
         c = torch.rand((n, 3), generator=g, device="cuda", dtype=torch.float64) * L
-        got = [mc3pcf.triplet_sum(*f, J, c, off, phi, samples=True, bricks=b) for b in (True, False)]
-        assert got[0][0] == got[1][0] and torch.equal(got[0][1], got[1][1])
+        got = [mc3pcf.triplet_sum(*f, J, c, off, phi, samples=True, bricks=b) for b in (True, False, 1, 0, None)]
+        assert all(t == got[0][0] and torch.equal(v, got[0][1]) for t, v in got[1:])
         for bad in (f[0].double(), f[0].transpose(0, 1), f[0][1:]):
             with pytest.raises(ValueError):
                 mc3pcf.triplet_sum(f[0], f[1], bad, J, c, off, phi)
