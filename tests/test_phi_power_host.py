@@ -17,6 +17,8 @@ def test_more_combinations_than_are_kept_on_the_device(monkeypatch):
         return fourier_power_spectrum(phi, k_max, k_count, res)
 
     monkeypatch.setattr(window, "fourier_power_spectrum", counted)
+    monkeypatch.setattr(window, "_POWER_CACHE", {})
+    monkeypatch.setattr(window, "_POWER_HOST", type(window._POWER_HOST)())
     n = window._POWER_KEEP + 40
     phis = [PHI * (1.0 + 1e-3 * k) for k in range(n)]
     for p in phis:
